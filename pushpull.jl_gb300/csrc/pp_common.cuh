@@ -145,10 +145,12 @@ __device__ __forceinline__ float spline_weights(float x, float* w, float* dw, fl
     } else if constexpr (DP == 4) {             // s = t - 1 in (0, 1]
         const float s = __fsub_rn(x, fo + 1.0f);
         const float a = 1.0f - s;
+        // w[2] as the complement of the others: with both central weights from the
+        // rounded 2/3 the four sum to 1 + 4.2e-8, a bias of 1.3e-7 over three axes
         w[0] = a * a * a * (1.0f / 6.0f);
         w[1] = (2.0f / 3.0f) - s * s * (1.0f - 0.5f * s);
-        w[2] = (2.0f / 3.0f) - a * a * (1.0f - 0.5f * a);
         w[3] = s * s * s * (1.0f / 6.0f);
+        w[2] = (1.0f - w[1]) - (w[0] + w[3]);
         if constexpr (ORD >= 1) {
             dw[0] = -0.5f * a * a;
             dw[1] = s * (1.5f * s - 2.0f);
@@ -166,9 +168,14 @@ __device__ __forceinline__ float spline_weights(float x, float* w, float* dw, fl
         const float a = 0.5f - s, b = 0.5f + s, p = 1.0f + s, q = 1.0f - s;
         w[0] = a * a * a * a * (1.0f / 24.0f);
         w[4] = b * b * b * b * (1.0f / 24.0f);
-        w[2] = (115.0f / 192.0f) + s * s * (s * s * 0.25f - 0.625f);
-        w[1] = (55.0f / 96.0f) + p * ((5.0f / 24.0f) + p * (-1.25f + p * ((5.0f / 6.0f) - p * (1.0f / 6.0f))));
-        w[3] = (55.0f / 96.0f) + q * ((5.0f / 24.0f) + q * (-1.25f + q * ((5.0f / 6.0f) - q * (1.0f / 6.0f))));
+        // even and odd parts in s of the outer central weights; w[2] as the
+        // complement of the others, so that the five sum to one
+        const float s2 = s * s;
+        const float u = (19.0f / 96.0f) + s2 * (0.25f - s2 * (1.0f / 6.0f));
+        const float v = s * ((11.0f / 24.0f) - s2 * (1.0f / 6.0f));
+        w[1] = u - v;
+        w[3] = u + v;
+        w[2] = (1.0f - 2.0f * u) - (w[0] + w[4]);
         if constexpr (ORD >= 1) {
             dw[0] = -a * a * a * (1.0f / 6.0f);
             dw[4] = b * b * b * (1.0f / 6.0f);
