@@ -94,6 +94,8 @@ TileCfg g_tiles[6][5];   // ops: pull, pull_grad, pull_hess, push, push_grad, fu
 bool g_tiles_init = false;
 int g_path = PP_PATH_AUTO;
 
+bool is_push_default(const TileCfg& t) { return t.lx == 3 && t.ly == 3 && t.lz == 3 && t.cap == 16384; }
+
 // The tile code (lx, ly, lz) = (3, 3, 4) selects the warp-specialised pull
 // kernels (pp_ws.cuh, 8 x 8 x 30 tiles); every other shape the
 // block-synchronous ones.
@@ -101,8 +103,9 @@ bool is_ws_tile(const TileCfg& t) { return t.lx == 3 && t.ly == 3 && t.lz == 4 &
 
 void init_tiles_locked() {
     if (g_tiles_init) return;
-    // 8x8x8 tiles; the push family keeps two words per accumulator element; the
-    // fused step's 2560-float budget at degree 2 leaves room for three CTAs per SM.
+    // 8x8x8 tiles; the fused step's 2560-float budget at degree 2 leaves room for
+    // three CTAs per SM.  For push and push_grad at degrees 2..4 the entry stands
+    // for push_default_tile's choice by size.
     // Degrees 0 and 1 (one or two taps per axis) default to the per-voxel
     // kernels (cap 0; the pull family at degree 1 is set below): with so few
     // taps, gathering through L2 is faster than a block-synchronous staging of
@@ -127,6 +130,11 @@ TileCfg tile_for(int op_index, int deg) {
     std::lock_guard<std::mutex> lk(g_cfg_mu);
     init_tiles_locked();
     return g_tiles[op_index][deg < 0 ? 0 : (deg > 4 ? 4 : deg)];
+}
+
+TileCfg push_tile_for(int op, const LaunchArgs& a) {
+    const TileCfg t = tile_for(3 + op, a.g.dp[0] - 1);
+    return is_push_default(t) ? push_default_tile(op, a) : t;
 }
 
 int current_path() {
@@ -248,9 +256,9 @@ static int run_push(int op, float* out, const float* phi, const float* in, const
         if (e != cudaSuccess) return cuda_fail(e, "zero output");
     }
     if (g.n1 == 0) return PP_OK;
-    const TileCfg t = tile_for(3 + op, deg[0]);
+    const TileCfg t = push_tile_for(op, a);
     cudaError_t e;
-    if (current_path() != PP_PATH_DIRECT && tiled_supported(a, t))
+    if (current_path() != PP_PATH_DIRECT && push_supported(a, t))
         e = launch_push_tiled(op, a, t, (cudaStream_t)stream);
     else
         e = launch_push_direct(op, a, (cudaStream_t)stream);
@@ -448,7 +456,7 @@ int pp_autotune(int op, float* out, const float* phi, const float* in, const pp_
     };
     const int tiles[][3] = {{3, 3, 3}, {4, 3, 2}, {4, 2, 3}, {5, 2, 2}, {3, 4, 2}, {3, 3, 2}, {4, 2, 2}, {3, 3, 4}};
     const int caps_pull[] = {6144, 8192, 12288};
-    const int caps_push[] = {12288, 16384, 20480};
+    const int caps_push[] = {7936, 9984, 16384};
     const TileCfg saved = tile_for(op, deg[0]);
     const int saved_path = current_path();
     cudaEvent_t e0, e1;

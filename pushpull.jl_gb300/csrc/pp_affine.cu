@@ -82,6 +82,7 @@ cudaError_t launch_affine_it(bool push, const LaunchArgs& a, const AffineMap& A,
 
 int fail_status(int code, const char* fmt, ...);
 TileCfg tile_for(int op_index, int deg);
+TileCfg push_tile_for(int op, const LaunchArgs& a);
 int current_path();
 int prepare_args(LaunchArgs& a, float* out, const float* phi, const float* in, const pp_usize d0[3],
                  const pp_usize d1[3], int nc, int nb, const int* bnd, int nbnd, const int deg[3], int ext);
@@ -110,8 +111,8 @@ int run_affine(bool push, float* out, const float* in, const float* Aff, const p
         if (!push) {
             if (tile_for(0, deg[0]).cap > 0 && ws_supported(a)) e = launch_ws_pull_affine(a, A, s);
         } else {
-            const TileCfg t = tile_for(3, deg[0]);
-            if (t.cap > 0 && tiled_supported(a, t)) e = launch_push_tiled_affine(a, t, A, s);
+            const TileCfg t = push_tile_for(kPush, a);
+            if (t.cap > 0 && push_supported(a, t)) e = launch_push_tiled_affine(a, t, A, s);
         }
         if (e == cudaErrorNotSupported) (void)cudaGetLastError();
         else if (e != cudaSuccess) return fail_status(PP_ERR_CUDA, "affine launch: %s", cudaGetErrorString(e));

@@ -57,9 +57,9 @@ __device__ __forceinline__ void red_shared_f32(unsigned a, float v) {
 
 // The validity test (VOXOK) of a 0-based position.
 __device__ __forceinline__ bool position_valid(float x0, float x1, float x2, const Geometry& g) {
-    if (!(finitef(x0) && finitef(x1) && finitef(x2))) return false;
-    if (g.ext) return true;
-    return x0 >= -0.01f && x0 <= g.hi[0] && x1 >= -0.01f && x1 <= g.hi[1] && x2 >= -0.01f && x2 <= g.hi[2];
+    const bool fin = finitef(x0) & finitef(x1) & finitef(x2);
+    if (g.ext) return fin;
+    return fin & (x0 >= -0.01f) & (x0 <= g.hi[0]) & (x1 >= -0.01f) & (x1 <= g.hi[1]) & (x2 >= -0.01f) & (x2 <= g.hi[2]);
 }
 
 // x = phi - 1 and the validity test, exactly as the reference evaluates them.

@@ -23,12 +23,13 @@ unsigned status_ws_grad_dot(bool reset);
 unsigned status_ws_hess_dot(bool reset);
 unsigned status_push_affine(bool reset);
 
-bool tiled_supported(const LaunchArgs& a, const TileCfg& t) {
+namespace {
+bool grid_supported(const LaunchArgs& a, const TileCfg& t, int max_vox) {
     const Geometry& g = a.g;
     const int vox = 1 << (t.lx + t.ly + t.lz);
     if (!(g.dp[0] == g.dp[1] && g.dp[1] == g.dp[2])) return false;
-    // whole tiles of 256 or 512 voxels: every thread owns one voxel slot per V
-    if (!(vox == kThreads || vox == 2 * kThreads) || t.cap < 64 || (t.cap & 3) || t.cap > 24 * 1024) return false;
+    // whole tiles of a multiple of the CTA's threads
+    if (vox < kThreads || vox > max_vox || t.cap < 64 || (t.cap & 3) || t.cap > 24 * 1024) return false;
     // a tile must be mostly inside the sample grid: degenerate grids (e.g. a
     // flat list of n1 samples) are better served by the per-voxel kernels
     for (int k = 0; k < 3; ++k) {
@@ -39,6 +40,25 @@ bool tiled_supported(const LaunchArgs& a, const TileCfg& t) {
     const long long nty = (g.d1[1] + (1 << t.ly) - 1) >> t.ly;
     const long long ntz = (g.d1[2] + (1 << t.lz) - 1) >> t.lz;
     return ntx * nty * ntz * g.nb < 0x7fffffffLL;
+}
+}  // namespace
+
+bool tiled_supported(const LaunchArgs& a, const TileCfg& t) { return grid_supported(a, t, 2 * kThreads); }
+bool push_supported(const LaunchArgs& a, const TileCfg& t) { return grid_supported(a, t, 8 * kThreads); }
+
+// The default push tiles are the largest of 16x8x8, 16x8x4 and 8x8x4 voxels that
+// still give every SM a few tiles: with fewer than about three 16x8x8 tiles (two
+// 16x8x4 tiles) per SM the smaller ones win because more CTAs take part.  Cubic
+// push, GB300, device us with 16x8x8 / 16x8x4 / 8x8x4 tiles: 32^3 22 / 18 / 15,
+// 48^3 22 / 20 / 18, 64^3 27 / 22 / 25, 80^3 31 / 33 / 35, 128^3 80 / 92 / 107;
+// at 192^3 16x8x8 takes 226, 8x8x8 255, 16x8x4 263, 32x4x8 244, 32x8x4 242.
+TileCfg push_default_tile(int op, const LaunchArgs& a) {
+    const int cap = op == kPush ? 9984 : 7936;   // words: four CTAs per SM with one ring slot
+    const long long y = (a.g.d1[1] + 7) >> 3, b = a.g.nb;
+    const long long x16 = (a.g.d1[0] + 15) >> 4;
+    if (x16 * y * ((a.g.d1[2] + 7) >> 3) * b >= 3LL * sm_count()) return TileCfg{4, 3, 3, cap};
+    if (x16 * y * ((a.g.d1[2] + 3) >> 2) * b >= 2LL * sm_count()) return TileCfg{4, 3, 2, cap};
+    return TileCfg{3, 3, 2, cap};
 }
 
 cudaError_t launch_pull_tiled(int op, const LaunchArgs& a, const TileCfg& t, cudaStream_t s) {

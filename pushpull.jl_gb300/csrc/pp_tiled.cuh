@@ -5,7 +5,7 @@
 
 namespace pp {
 
-// Tile of sample voxels handled by one CTA: 2^lx x 2^ly x 2^lz (32..512 voxels),
+// Tile of sample voxels handled by one CTA: 2^lx x 2^ly x 2^lz (32..512 voxels, push up to 2048),
 // and the shared-memory budget of its footprint box, in floats (multiple of 4).
 struct TileCfg {
     int lx, ly, lz;
@@ -13,6 +13,10 @@ struct TileCfg {
 };
 
 bool tiled_supported(const LaunchArgs& a, const TileCfg& t);
+// the same for the push family, whose tiles hold up to 2048 voxels
+bool push_supported(const LaunchArgs& a, const TileCfg& t);
+// the push tile for a launch when the registry holds its default entry (16x8x8)
+TileCfg push_default_tile(int op, const LaunchArgs& a);
 // warp-specialised pull family (8 x 8 x 30 tiles, pp_ws.cuh): geometry test and
 // launch (cudaErrorNotSupported for ops or layouts it does not take)
 bool ws_supported(const LaunchArgs& a);
@@ -35,6 +39,7 @@ struct TileGrid {
     int cap;            // box budget in floats
     int pmod;           // box row pitch P is chosen with P % 32 == pmod
     int img_tma;        // pull: interior boxes may be loaded with one TMA copy (image tensor map valid)
+    int nv, stages;     // push: voxels per tile, ring slots
 };
 
 // Fused forward + adjoint step over tiles: grid size for a launch, and the

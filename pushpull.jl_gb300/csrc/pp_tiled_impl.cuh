@@ -138,7 +138,6 @@ struct Box {
     int tma;        // 1: the box is a fixed window loaded by one TMA copy; 2: the same, with mirrored margins to complete
     float S;        // block sum of the caller's per-thread value (push: bound on sum |contribution|)
     int E;          // scale exponent of the fixed-point accumulator for S (see scale_exponent)
-    int wsc;        // push: 1 = scatter one voxel per warp instruction (contracted tile)
 };
 
 __device__ __forceinline__ int clamp_tap(long long o) {
@@ -161,52 +160,12 @@ __device__ __forceinline__ int scale_exponent(float S) {
     return (E < -80 || E > 100) ? INT_MIN : E;
 }
 
-// ---- pitches for the warp-cooperative scatter -------------------------------
-// One voxel per warp instruction, one tap per lane: lane l of pass p takes tap
-// t = 32 p + l, (i, j, k) = t in radix DP, at box element base + i + P j + Q k.
-// The taps of one voxel never share an element, and for (P mod 32, Q mod 32)
-// pairs whose bit is set below (bit Q of entry P, one row per DP = 3, 4, 5) the
-// 32 lanes of every pass also fall in 32 distinct shared-memory banks, so each
-// reduction is a single wavefront whatever the deformation does.
-__device__ const unsigned kScatterQMask[3][32] = {
-    {0x00000000u, 0x00000000u, 0x00000000u, 0x00e00e00u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00200800u,
-     0x00000000u, 0x20000008u, 0x20000008u, 0x22044088u, 0x00000000u, 0x00000000u, 0x00200800u, 0x00000000u,
-     0x00000000u, 0x00000000u, 0x00200800u, 0x00000000u, 0x00000000u, 0x22044088u, 0x20000008u, 0x20000008u,
-     0x00000000u, 0x00200800u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00e00e00u, 0x00000000u, 0x00000000u},
-    {0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00010000u, 0x00000000u, 0x00000000u, 0x00000000u,
-     0x10101010u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00010000u, 0x00000000u, 0x00000000u, 0x00000000u,
-     0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00010000u, 0x00000000u, 0x00000000u, 0x00000000u,
-     0x10101010u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00010000u, 0x00000000u, 0x00000000u, 0x00000000u},
-    {0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x02000000u, 0x00000000u, 0x00000000u,
-     0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u,
-     0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u,
-     0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u, 0x00000000u},
-};
-
-// Smallest row pitch P >= the row's 4-element groups (the flush reads whole
-// groups of 4) and plane pitch Q >= P * e1 of a conflict-free pair.
-template <int DP>
-__device__ __forceinline__ void scatter_pitch(long long e0, long long e1, long long& P, long long& Q) {
-    const unsigned* mask = kScatterQMask[DP - 3];
-    P = (e0 + 3) & ~3LL;
-    while (mask[P & 31] == 0u) ++P;
-    const unsigned m = mask[P & 31];
-    Q = P * e1;
-    while (!((m >> (Q & 31)) & 1u)) ++Q;
-}
-
 // Block-wide reduction of the first-tap bounds into the footprint box.
 // `words` = shared-memory words needed per box element (1 for pull, 2 for push).
 // Also sums `ssum` over the block into box.S (fixed order) and sets box.E.
-// WSCATTER (push): a tile whose box has fewer elements than the tile has
-// voxels (a contracting deformation, many voxels per element) gets the
-// warp-cooperative scatter when its accumulator and the voxel records
-// (rec_floats, kept at the top of the budget) fit: box.wsc = 1 and the
-// conflict-free pitches of scatter_pitch.
-template <int DP, bool WSCATTER = false>
+template <int DP>
 __device__ __forceinline__ void reduce_box(int (&mn)[3], int (&mx)[3], const TileGrid& t, const Geometry& g,
-                                           int words, Box& box, int (&red)[8][7], float ssum = 0.f,
-                                           int nv_tile = 0, int rec_floats = 0) {
+                                           int words, Box& box, int (&red)[8][7], float ssum = 0.f) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -243,7 +202,6 @@ __device__ __forceinline__ void reduce_box(int (&mn)[3], int (&mx)[3], const Til
         if (lo[0] > hi[0]) {
             box.mode = 0;
             box.tma = 0;
-            box.wsc = 0;
         } else {
             const int xo = lo[0] & ~3;
             long long e[3];
@@ -257,22 +215,13 @@ __device__ __forceinline__ void reduce_box(int (&mn)[3], int (&mx)[3], const Til
             // P % 32 == pmod and Q % 32 == 0 keep the warp's rows and planes in
             // disjoint banks; when that padding would not fit, pack tightly.
             long long P = 0, Q = 0;
-            box.wsc = 0;
-            if constexpr (WSCATTER) {
-                if (e[0] * e[1] * e[2] < nv_tile) {
-                    scatter_pitch<DP>(e[0], e[1], P, Q);
-                    if (Q * e[2] * words + rec_floats <= t.cap) box.wsc = 1;
-                }
-            }
-            if (!box.wsc) {
-                P = (e[0] + 3) & ~3LL;
-                long long Pp = P + (((t.pmod - (int)(P & 31)) + 32) & 31);
-                Q = (Pp * e[1] + 31) & ~31LL;
-                if (Q * e[2] * words <= t.cap) {
-                    P = Pp;
-                } else {
-                    Q = (P * e[1] + 3) & ~3LL;
-                }
+            P = (e[0] + 3) & ~3LL;
+            long long Pp = P + (((t.pmod - (int)(P & 31)) + 32) & 31);
+            Q = (Pp * e[1] + 31) & ~31LL;
+            if (Q * e[2] * words <= t.cap) {
+                P = Pp;
+            } else {
+                Q = (P * e[1] + 3) & ~3LL;
             }
             long long size = Q * e[2];
             const bool fits = e[0] <= 4096 && e[1] <= 4096 && e[2] <= 4096 && size * words <= t.cap;
@@ -315,6 +264,7 @@ __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) 
 
 // Rows of the box are distributed over warps; within a warp a group of `lpr`
 // lanes (a power of two) shares a row.
+template <int NT = kThreads>
 struct RowWalk {
     int lg, sub, e0;   // lanes per row = 1 << lg
     int ry, rz;        // this lane group's current row
@@ -328,7 +278,7 @@ struct RowWalk {
         e0 = lane & ((1 << lg) - 1);
         ey = ey_;
         const int first = (threadIdx.x >> 5) * (32 >> lg) + sub;
-        const int step = (kThreads / 32) * (32 >> lg);
+        const int step = (NT / 32) * (32 >> lg);
         rz = first / ey;
         ry = first - rz * ey;
         sz = step / ey;
@@ -349,7 +299,7 @@ struct RowWalk {
 template <typename IT, class FN>
 __device__ __forceinline__ void walk_box(const Box& box, const Geometry& g, int b0, int b1, int b2, FN fn) {
     const int ex = box.ext[0], ey = box.ext[1], ez = box.ext[2];
-    RowWalk rw(ex, ey);
+    RowWalk<> rw(ex, ey);
     const IT sy = (IT)g.d0[0];
     const IT sz = (IT)(g.d0[0] * g.d0[1]);
     const bool xin = box.interior & 1, yin = box.interior & 2, zin = box.interior & 4;
@@ -385,7 +335,7 @@ __device__ __forceinline__ void stage_box(const Box& box, const Geometry& g, int
     if (box.interior == 7 && (g.d0[0] & 3) == 0 && (reinterpret_cast<uintptr_t>(f0) & 15) == 0) {
         const int ey = box.ext[1], ez = box.ext[2];
         const int n4 = (box.ext[0] + 3) >> 2;
-        RowWalk rw(n4, ey);
+        RowWalk<> rw(n4, ey);
         const IT sy = (IT)g.d0[0];
         const IT sz = (IT)(g.d0[0] * g.d0[1]);
         for (; rw.rz < ez; rw.next()) {
@@ -416,16 +366,16 @@ __device__ __forceinline__ void stage_box(const Box& box, const Geometry& g, int
 // is out of range (S = 0, non-finite, or extreme) the tile uses float atomics.
 constexpr float kMagic = 12582912.0f;     // 1.5 * 2^23: float -> nearest int for |y| <= 2^22
 constexpr int kMagicBits = 0x4B400000;
+constexpr float kLoScale = 1048576.0f;    // push tiles of up to 2048 voxels: 2^20 lower quanta per upper one
 
 __device__ __forceinline__ float pow2f(int k) { return __int_as_float((127 + k) << 23); }   // -126 <= k <= 127
 
 struct FixedScale {
-    float inv_q1, q1, inv_q2, q2;
-    __device__ __forceinline__ void set(int E) {
+    float inv_q1, q1, q2;
+    __device__ __forceinline__ void set(int E, int bits = 43) {
         inv_q1 = pow2f(22 - E);
         q1 = pow2f(E - 22);
-        inv_q2 = pow2f(43 - E);
-        q2 = pow2f(E - 43);
+        q2 = pow2f(E - bits);
     }
 };
 
@@ -442,7 +392,7 @@ __device__ __forceinline__ void flush_box(const Box& box, const Geometry& g, int
     if ((box.interior & 1) && (g.d0[0] & 3) == 0 && (reinterpret_cast<uintptr_t>(f0) & 15) == 0) {
         const int ey = box.ext[1], ez = box.ext[2];
         const int n4 = (box.ext[0] + 3) >> 2;        // rows start at xo (16-byte aligned); whole groups
-        RowWalk rw(n4, ey);
+        RowWalk<> rw(n4, ey);
         const IT sy = (IT)g.d0[0];
         const IT sz = (IT)(g.d0[0] * g.d0[1]);
         for (; rw.rz < ez; rw.next()) {
@@ -493,7 +443,7 @@ __device__ __forceinline__ void flush_fixed(const Box& box, const Geometry& g, i
     }
     const int ey = box.ext[1], ez = box.ext[2];
     const int n4 = (box.ext[0] + 3) >> 2;
-    RowWalk rw(n4, ey);
+    RowWalk<> rw(n4, ey);
     if (rw.e0 >= n4) return;   // lanes per row >= n4: at most one group of each row per thread
     const IT sy = (IT)g.d0[0];
     const IT sz = (IT)(g.d0[0] * g.d0[1]);
@@ -1223,363 +1173,14 @@ __device__ __forceinline__ void push_scatter(const WT& wx, const WT& wy, const W
     }
 }
 
-// Push ops and degrees that scatter one voxel per warp instruction: push and
-// push_grad at DP = 3 and 4 (a degree-4 box would need pitches of 37 elements or
-// more).
-template <int DP, int OP>
-__host__ __device__ constexpr bool warp_scatter() {
-    return DP == 3 || DP == 4;
-}
-
-// float4 record arrays per voxel of the warp-cooperative scatter: push keeps
-// x, y (times the scaled value) and z weights; push_grad keeps v0 dw_x, v1 w_x,
-// v2 w_x (values scaled), then w_y, dw_y, w_z, dw_z.
-template <int OP>
-__host__ __device__ constexpr int scatter_records() {
-    return OP == kPushGrad ? 7 : 3;
-}
-
-// Warp-cooperative scatter of a tile's recorded voxels into the fixed-point
-// (or, when !fixed, float) accumulator: warp w takes voxels w, w + 8, ...; lane
-// l of pass p adds tap t = 32 p + l of that voxel.  With the box pitches chosen
-// by scatter_pitch the 32 reductions of a pass hit 32 distinct elements in 32
-// distinct banks.
-// Shared-memory reductions for the warp-cooperative scatter: no compiler memory
-// barrier, so the record loads of the next voxels can be issued ahead of them
-// (the records and the accumulator are disjoint; the phases are separated by
-// __syncthreads).
+// Shared-memory reductions without a compiler memory barrier, so that loads of
+// the next voxels can be issued ahead of them (what they read and the
+// accumulator are disjoint; the phases are separated by __syncthreads).
 __device__ __forceinline__ void red_s32_nb(unsigned a, int v) {
     asm volatile("red.shared.add.s32 [%0], %1;" ::"r"(a), "r"(v));
 }
 __device__ __forceinline__ void red_f32_nb(unsigned a, float v) {
     asm volatile("red.shared.add.f32 [%0], %1;" ::"r"(a), "f"(v));
-}
-
-template <int DP, int OP, int DPP, int NV>
-__device__ __forceinline__ void warp_scatter_tile(const float* rec, const int* rb, int P, int Q, unsigned acc_base,
-                                                  unsigned lo_off, bool fixed) {
-    constexpr int T = DP * DP * DP;
-    constexpr int PASSES = (T + 31) / 32;
-    constexpr int NW = kThreads / 32;
-    constexpr int U = OP == kPushGrad ? 1 : 2;   // voxels per warp iteration (registers)
-    static_assert(NV % (U * NW) == 0, "whole warp iterations");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int ti[PASSES], tj[PASSES], tk[PASSES], off[PASSES];
-#pragma unroll
-    for (int p = 0; p < PASSES; ++p) {
-        const int tt = p * 32 + lane < T ? p * 32 + lane : 0;
-        ti[p] = tt % DP;
-        tj[p] = (tt / DP) % DP;
-        tk[p] = tt / (DP * DP);
-        off[p] = ti[p] + P * tj[p] + Q * tk[p];
-    }
-    // U voxels per iteration: all record loads first, then the reductions
-    for (int s0 = warp; s0 < NV; s0 += U * NW) {
-        int bv[U];
-        float y[U][PASSES];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int sidx = s0 + u * NW;
-            bv[u] = rb[sidx];
-            const float* R = rec + sidx * DPP;   // record array r of this voxel at R + r * DPP * NV
-            constexpr int RS = DPP * NV;
-            if constexpr (OP == kPushGrad) {
-                // v0 dwx wy wz + v1 wx dwy wz + v2 wx wy dwz = wz (wy A + dwy B) + dwz (wy C)
-#pragma unroll
-                for (int p = 0; p < PASSES; ++p) {
-                    const float A = R[ti[p]], B = R[RS + ti[p]], C = R[2 * RS + ti[p]];
-                    const float Y = R[3 * RS + tj[p]], DY = R[4 * RS + tj[p]];
-                    const float Z = R[5 * RS + tk[p]], DZ = R[6 * RS + tk[p]];
-                    y[u][p] = fmaf(Z, fmaf(Y, A, DY * B), DZ * (Y * C));
-                }
-            } else {
-#pragma unroll
-                for (int p = 0; p < PASSES; ++p) y[u][p] = (R[ti[p]] * R[RS + tj[p]]) * R[2 * RS + tk[p]];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (bv[u] < 0) continue;   // warp-uniform: every lane read the same record
-#pragma unroll
-            for (int p = 0; p < PASSES; ++p) {
-                if (p * 32 + lane >= T) continue;
-                const unsigned a = acc_base + 4u * (unsigned)(bv[u] + off[p]);
-                if (fixed) {
-                    // y in q1 units, |y| <= 2^22: hi = round(y), lo = round((y - hi) * 2^21)
-                    const float t1 = __fadd_rn(y[u][p], kMagic);
-                    const float r = __fsub_rn(y[u][p], __fsub_rn(t1, kMagic));
-                    red_s32_nb(a, __float_as_int(t1) - kMagicBits);
-                    red_s32_nb(a + lo_off, __float_as_int(__fmaf_rn(r, 2097152.0f, kMagic)) - kMagicBits);
-                } else {
-                    red_f32_nb(a, y[u][p]);
-                }
-            }
-        }
-    }
-}
-
-// Persistent push family.  The ring holds each tile's deformation and its
-// channel-0 values kStages tiles ahead; the tile scatters into the shared
-// accumulator and flushes it with global reductions.  The flush clears every
-// element it reads, so the accumulator is zero again for the next tile.
-// AFF: the affine push -- positions A * (i, j, k, 1) from `aff`, no deformation.
-template <int DP, int OP, int V, typename IT, bool TMA, bool AFF = false>
-__global__ void __launch_bounds__(kThreads, 2) k_push_tiled(const __grid_constant__ LaunchArgs a,
-                                                            const __grid_constant__ TileGrid t,
-                                                            const __grid_constant__ CUtensorMap phimap,
-                                                            const __grid_constant__ CUtensorMap valmap,
-                                                            const __grid_constant__ AffineMap aff) {
-    extern __shared__ __align__(128) float4 smem4[];
-    constexpr int ORD = OP == kPushGrad ? 1 : 0;
-    constexpr int NCOMP = OP == kPushGrad ? 3 : 1;
-    constexpr int NV = kThreads * V;
-    // contracted tiles of push and push_grad at degrees 2 and 3 scatter one voxel
-    // per warp instruction (see kScatterQMask); other tiles and degrees one voxel
-    // per thread
-    constexpr bool WSC = warp_scatter<DP, OP>();
-    constexpr int DPP = 4;   // record stride per axis (DP <= 4 under WSC)
-    __shared__ int red[8][7];
-    __shared__ float sred[8];
-    __shared__ Box box;
-    __shared__ int s_abort;
-    const Geometry& g = a.g;
-    const long long n1 = g.n1;
-    const int G = gridDim.x;
-    const int T0 = blockIdx.x;
-    if (T0 >= t.ntiles) return;
-    const int ntl = (t.ntiles - T0 + G - 1) / G;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const ThreadVox<V> tv(t, g);
-
-    float* sm = reinterpret_cast<float*>(smem4);
-    Ring ring;
-    ring.base = sm;
-    ring.slot_floats = (3 + NCOMP) * NV;
-    float* accf = sm + kStages * (3 + NCOMP) * NV;
-    ring.bars = smem_addr(accf + t.cap);
-    // voxel records of the warp-cooperative scatter (contracted tiles only), at
-    // the top of the accumulator budget: the float4 arrays of scatter_records,
-    // then the box-relative first tap (-1: skip)
-    constexpr int NREC = scatter_records<OP>();
-    constexpr int kRec = (NREC * DPP + 1) * NV;
-    float* rx = accf + (WSC ? t.cap - kRec : 0);
-    int* rb = reinterpret_cast<int*>(rx + NREC * DPP * NV);
-    for (int i = threadIdx.x; i < (t.cap >> 2); i += kThreads)
-        reinterpret_cast<float4*>(accf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (threadIdx.x == 0) {
-        s_abort = 0;
-        if (TMA) {
-            for (int k = 0; k < kStages; ++k) mbar_init(ring.bars + 8u * k, 1);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-    }
-    __syncthreads();
-    for (int j = 0; j < kStages && j < ntl; ++j)
-        ring_fill<V, NCOMP, TMA, IT, AFF>(ring, j, T0 + j * G, a, t, tv, phimap, valmap, a.in);
-    if (!TMA) __syncthreads();
-
-    const unsigned acc_base = smem_addr(accf);
-    for (int j = 0; j < ntl; ++j) {
-        const TileOrigin o = tile_origin(t, T0 + j * G);
-        const float* slot = ring.base + (j % kStages) * ring.slot_floats;
-        if (!ring_wait<TMA>(ring, j)) s_abort = 1;
-        const TilePos<NV, AFF> pos{slot, &aff, t.lx, t.ly};
-        // deformation validity, first-tap bounds and the channel-0 scale bound
-        int mn[3], mx[3];
-        tile_bounds_pos<DP, V, IT>(g, o, tv, pos, mn, mx);
-        float bound0 = 0.f;
-#pragma unroll
-        for (int q = 0; q < V; ++q) {
-            const int lin = threadIdx.x + q * kThreads;
-            float x0, x1, x2;
-            if (tv.template index<IT>(o, q) < 0 ||
-                !pos(g, o, lin, x0, x1, x2))
-                continue;
-            bool fin = true;
-            float s1 = 0.f;
-#pragma unroll
-            for (int p = 0; p < NCOMP; ++p) {
-                const float v = slot[(3 + p) * NV + lin];
-                fin = fin && finitef(v);
-                s1 += fabsf(v);
-            }
-            if (fin) bound0 += OP == kPushGrad ? 2.f * s1 : s1;
-        }
-        reduce_box<DP, WSC>(mn, mx, t, g, 2, box, red, bound0, NV, WSC ? kRec : 0);
-        if (s_abort) break;
-        if (box.mode == 2) {
-#pragma unroll
-            for (int q = 0; q < V; ++q) {
-                const IT v = tv.template index<IT>(o, q);
-                const int lin = threadIdx.x + q * kThreads;
-                float x0, x1, x2;
-                if (v >= 0 && pos(g, o, lin, x0, x1, x2))
-                    push_tile_fallback<DP, OP, IT>(a, o.b, (long long)v, x0, x1, x2);
-            }
-        } else if (box.mode == 1) {
-            const unsigned lo_off = 4u * (unsigned)box.size;
-            int* acc_hi = reinterpret_cast<int*>(accf);
-            int* acc_lo = acc_hi + box.size;
-            const float* inb = a.in + (long long)o.b * g.nc * NCOMP * n1;
-            // the box geometry in registers: the scatter's reductions are memory
-            // barriers to the compiler, which would reload it from shared memory
-            const int bxo = box.xo, by0 = box.lo[1], bz0 = box.lo[2], bP = box.P, bQ = box.Q;
-            for (int c = 0; c < g.nc; ++c) {
-                int b0, b1, b2;
-                bnd_code(a, c, b0, b1, b2);
-                int E = box.E;
-                if (c > 0) {
-                    // values of channel c straight from global memory, and their scale bound
-                    float bound = 0.f;
-#pragma unroll
-                    for (int q = 0; q < V; ++q) {
-                        const IT v = tv.template index<IT>(o, q);
-                        const int lin = threadIdx.x + q * kThreads;
-                        float x0, x1, x2;
-                        if (v < 0 || !pos(g, o, lin, x0, x1, x2))
-                            continue;
-                        bool fin = true;
-                        float s1 = 0.f;
-#pragma unroll
-                        for (int p = 0; p < NCOMP; ++p) {
-                            const float vv = __ldg(inb + (long long)c * NCOMP * n1 + v + p * n1);
-                            fin = fin && finitef(vv);
-                            s1 += fabsf(vv);
-                        }
-                        if (fin) bound += OP == kPushGrad ? 2.f * s1 : s1;
-                    }
-#pragma unroll
-                    for (int off = 16; off > 0; off >>= 1) bound += __shfl_xor_sync(0xffffffffu, bound, off);
-                    __syncthreads();   // the previous channel's flush is done
-                    if (lane == 0) sred[warp] = bound;
-                    __syncthreads();
-                    float S = 0.f;
-                    for (int w = 0; w < kThreads / 32; ++w) S += sred[w];
-                    E = scale_exponent(S);
-                }
-                if (E == INT_MAX) continue;   // every value of this channel is zero or skipped
-                const bool fixed = E != INT_MIN;
-                FixedScale fs;
-                fs.set(fixed ? E : 0);
-                auto thread_scatter = [&]() {
-#pragma unroll
-                for (int q = 0; q < V; ++q) {
-                    const IT v = tv.template index<IT>(o, q);
-                    const int lin = threadIdx.x + q * kThreads;
-                    float x0, x1, x2;
-                    if (v < 0 || !pos(g, o, lin, x0, x1, x2)) continue;
-                    float val[NCOMP];
-                    bool fin = true;
-#pragma unroll
-                    for (int p = 0; p < NCOMP; ++p) {
-                        val[p] = c == 0 ? slot[(3 + p) * NV + lin] : __ldg(inb + (long long)c * NCOMP * n1 + v + p * n1);
-                        fin = fin && finitef(val[p]);
-                    }
-                    if (!fin) continue;
-                    W3<DP, ORD> wx, wy, wz;
-                    const int ox = spline_taps32<DP, ORD>(x0, wx.w, wx.dw, wx.hw) - bxo;
-                    const int oy = spline_taps32<DP, ORD>(x1, wy.w, wy.dw, wy.hw) - by0;
-                    const int oz = spline_taps32<DP, ORD>(x2, wz.w, wz.dw, wz.hw) - bz0;
-                    const unsigned P4 = 4u * bP, Q4 = 4u * bQ;
-                    const unsigned base = acc_base + 4u * (unsigned)(oz * bQ + oy * bP + ox);
-                    const float sc = fixed ? fs.inv_q1 : 1.f;
-                    const float w0 = val[0] * sc;
-                    const float w1 = NCOMP > 1 ? val[NCOMP > 1 ? 1 : 0] * sc : 0.f;
-                    const float w2 = NCOMP > 2 ? val[NCOMP > 2 ? 2 : 0] * sc : 0.f;
-                    if (fixed) push_scatter<DP, OP, true>(wx, wy, wz, w0, w1, w2, base, P4, Q4, lo_off);
-                    else push_scatter<DP, OP, false>(wx, wy, wz, w0, w1, w2, base, P4, Q4, lo_off);
-                }
-                };
-                if constexpr (WSC) {
-                if (box.wsc) {
-                    const float sc = fixed ? fs.inv_q1 : 1.f;
-                    // each thread records its own voxels ...
-#pragma unroll
-                    for (int q = 0; q < V; ++q) {
-                        const IT v = tv.template index<IT>(o, q);
-                        const int lin = threadIdx.x + q * kThreads;
-                        int base = -1;
-                        float x0, x1, x2;
-                        if (v >= 0 && pos(g, o, lin, x0, x1, x2)) {
-                            float val[NCOMP];
-                            bool fin = true;
-#pragma unroll
-                            for (int p = 0; p < NCOMP; ++p) {
-                                val[p] = c == 0 ? slot[(3 + p) * NV + lin]
-                                                : __ldg(inb + (long long)c * NCOMP * n1 + v + p * n1);
-                                fin = fin && finitef(val[p]);
-                            }
-                            if (fin) {
-                                // one 16-byte store per record array (DPP = 4; unused taps 0),
-                                // one axis at a time
-                                auto w4 = [&](const float* w, float m) {
-                                    return make_float4(w[0] * m, DP > 1 ? w[DP > 1 ? 1 : 0] * m : 0.f,
-                                                       DP > 2 ? w[DP > 2 ? 2 : 0] * m : 0.f,
-                                                       DP > 3 ? w[DP > 3 ? 3 : 0] * m : 0.f);
-                                };
-                                float4* R4 = reinterpret_cast<float4*>(rx) + lin;
-                                W3<DP, ORD> wa;
-                                const int ox = spline_taps32<DP, ORD>(x0, wa.w, wa.dw, wa.hw) - bxo;
-                                if constexpr (OP == kPushGrad) {
-                                    R4[0] = w4(wa.dw, val[0] * sc);
-                                    R4[NV] = w4(wa.w, val[NCOMP > 1 ? 1 : 0] * sc);
-                                    R4[2 * NV] = w4(wa.w, val[NCOMP > 2 ? 2 : 0] * sc);
-                                } else {
-                                    R4[0] = w4(wa.w, 1.f);
-                                }
-                                const int oy = spline_taps32<DP, ORD>(x1, wa.w, wa.dw, wa.hw) - by0;
-                                if constexpr (OP == kPushGrad) {
-                                    R4[3 * NV] = w4(wa.w, 1.f);
-                                    R4[4 * NV] = w4(wa.dw, 1.f);
-                                } else {
-                                    R4[NV] = w4(wa.w, val[0] * sc);
-                                }
-                                const int oz = spline_taps32<DP, ORD>(x2, wa.w, wa.dw, wa.hw) - bz0;
-                                if constexpr (OP == kPushGrad) {
-                                    R4[5 * NV] = w4(wa.w, 1.f);
-                                    R4[6 * NV] = w4(wa.dw, 1.f);
-                                } else {
-                                    R4[2 * NV] = w4(wa.w, 1.f);
-                                }
-                                base = oz * bQ + oy * bP + ox;
-                            }
-                        }
-                        rb[lin] = base;
-                    }
-                    __syncthreads();   // records complete
-                    // ... then every warp scatters whole voxels, one tap per lane
-                    warp_scatter_tile<DP, OP, DPP, NV>(rx, rb, bP, bQ, acc_base, lo_off, fixed);
-                } else {
-                    thread_scatter();
-                }
-                } else {
-                    thread_scatter();
-                }
-                __syncthreads();   // the scatter is complete
-                float* f0 = a.out + ((long long)o.b * g.nc + c) * g.n0;
-                if (fixed)
-                    flush_fixed<IT>(box, g, b0, b1, b2, f0, acc_hi, acc_lo, fs);
-                else
-                    flush_box<IT>(box, g, b0, b1, b2, f0, [&](int si) {
-                        const float v = accf[si];
-                        accf[si] = 0.f;
-                        return v;
-                    });
-            }
-        }
-        if constexpr (WSC) {
-            if (box.mode == 1 && box.wsc) {   // the records sat in the accumulator budget: clear them
-                __syncthreads();
-                for (int i = threadIdx.x; i < kRec / 4; i += kThreads)
-                    reinterpret_cast<float4*>(rx)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-        }
-        __syncthreads();   // ring slot j is free and the accumulator is clear
-        if (j + kStages < ntl)
-            ring_fill<V, NCOMP, TMA, IT, AFF>(ring, j + kStages, T0 + (j + kStages) * G, a, t, tv, phimap, valmap,
-                                              a.in);
-        if (!TMA) __syncthreads();
-    }
 }
 
 // ---- fused forward + adjoint step ------------------------------------------
@@ -2107,6 +1708,8 @@ TileGrid make_grid(const LaunchArgs& a, const TileCfg& c) {
     const int tx = 1 << c.lx;
     t.pmod = tx >= 32 ? 0 : tx;
     t.img_tma = 0;
+    t.nv = tx << (c.ly + c.lz);
+    t.stages = 0;
     return t;
 }
 
@@ -2192,47 +1795,36 @@ bool encode_box_map(CUtensorMap* map, const float* base, const long long d[3], l
 }
 
 template <typename K, typename... Args>
-cudaError_t launch_persistent(K kern, const TileGrid& t, size_t smem, cudaStream_t s, const Args&... args) {
+cudaError_t launch_persistent(K kern, const TileGrid& t, size_t smem, cudaStream_t s, int threads,
+                              const Args&... args) {
     cudaError_t e = opt_in(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     const long long want = (long long)sm_count() * per_sm;
     const int grid = (int)(t.ntiles < want ? t.ntiles : want);
-    kern<<<grid, kThreads, smem, s>>>(args...);
+    kern<<<grid, threads, smem, s>>>(args...);
     return cudaGetLastError();
 }
 
-// AFF (push only): the affine push, positions from `aff` instead of a.phi.
-template <int DP, int OP, int V, typename IT, bool PUSH, bool AFF = false>
-cudaError_t launch_v(const LaunchArgs& a, const TileGrid& t, cudaStream_t s, const AffineMap& aff = AffineMap{}) {
+template <int DP, int OP, int V, typename IT>
+cudaError_t launch_v(const LaunchArgs& a, const TileGrid& t, cudaStream_t s) {
     constexpr int NV = kThreads * V;
-    CUtensorMap phimap, valmap;
+    CUtensorMap phimap, imgmap;
     std::memset(&phimap, 0, sizeof phimap);
-    std::memset(&valmap, 0, sizeof valmap);
+    std::memset(&imgmap, 0, sizeof imgmap);
     const long long nb = a.g.nb, nc = a.g.nc;
-    bool tma = AFF || encode_tile_map(&phimap, a.phi, a.g.d1, 3 * nb, t, 3);
-    if constexpr (PUSH) {
-        constexpr int NCOMP = OP == kPushGrad ? 3 : 1;
-        tma = tma && encode_tile_map(&valmap, a.in, a.g.d1, NCOMP * nc * nb, t, NCOMP);
-        const size_t smem = (size_t)kStages * (3 + NCOMP) * NV * 4 + (size_t)t.cap * 4 + 8 * kStages;
-        if (tma) return launch_persistent(k_push_tiled<DP, OP, V, IT, true, AFF>, t, smem, s, a, t, phimap, valmap, aff);
-        return launch_persistent(k_push_tiled<DP, OP, V, IT, false, AFF>, t, smem, s, a, t, phimap, valmap, aff);
-    } else {
-        static_assert(!AFF, "affine pull runs on the warp-specialised kernels");
-        // interior boxes as one TMA copy of a fixed window when the tile is 8 wide
-        // (the window's row pitch is bank-conflict free for 8-wide warp tiles)
-        CUtensorMap imgmap;
-        std::memset(&imgmap, 0, sizeof imgmap);
-        TileGrid tt = t;
-        tt.img_tma = t.lx == 3 && t.cap >= kTmaBoxFloats && (t.cap & 31) == 0 &&
-                     encode_box_map(&imgmap, a.in, a.g.d0, nc * nb);
-        const size_t smem = (size_t)kStages * 3 * NV * 4 + 2 * (size_t)t.cap * 4 + 8 * kStages + 16;
-        if (tma) return launch_persistent(k_pull_tiled<DP, OP, V, IT, true>, tt, smem, s, a, tt, phimap, imgmap);
-        return launch_persistent(k_pull_tiled<DP, OP, V, IT, false>, tt, smem, s, a, tt, phimap, imgmap);
-    }
+    const bool tma = encode_tile_map(&phimap, a.phi, a.g.d1, 3 * nb, t, 3);
+    // interior boxes as one TMA copy of a fixed window when the tile is 8 wide
+    // (the window's row pitch is bank-conflict free for 8-wide warp tiles)
+    TileGrid tt = t;
+    tt.img_tma = t.lx == 3 && t.cap >= kTmaBoxFloats && (t.cap & 31) == 0 &&
+                 encode_box_map(&imgmap, a.in, a.g.d0, nc * nb);
+    const size_t smem = (size_t)kStages * 3 * NV * 4 + 2 * (size_t)t.cap * 4 + 8 * kStages + 16;
+    if (tma) return launch_persistent(k_pull_tiled<DP, OP, V, IT, true>, tt, smem, s, kThreads, a, tt, phimap, imgmap);
+    return launch_persistent(k_pull_tiled<DP, OP, V, IT, false>, tt, smem, s, kThreads, a, tt, phimap, imgmap);
 }
 
 template <int DP, int V, typename IT>
@@ -2265,22 +1857,21 @@ cudaError_t launch_fused_dp(const LaunchArgs& a, const TileCfg& c, cudaStream_t 
     return launch_fused_v<DP, 1, IT>(a, t, s, grid);
 }
 
-template <int DP, int OP, typename IT, bool PUSH, bool AFF = false>
-cudaError_t launch_one(const LaunchArgs& a, const TileCfg& c, cudaStream_t s, const AffineMap& aff) {
+template <int DP, int OP, typename IT>
+cudaError_t launch_one(const LaunchArgs& a, const TileCfg& c, cudaStream_t s) {
     const TileGrid t = make_grid(a, c);
-    const int vox = 1 << (c.lx + c.ly + c.lz);
-    if (vox > kThreads) return launch_v<DP, OP, 2, IT, PUSH, AFF>(a, t, s, aff);
-    return launch_v<DP, OP, 1, IT, PUSH, AFF>(a, t, s, aff);
+    if (t.nv > kThreads) return launch_v<DP, OP, 2, IT>(a, t, s);
+    return launch_v<DP, OP, 1, IT>(a, t, s);
 }
 
-template <int OP, typename IT, bool PUSH, bool AFF = false>
-cudaError_t dispatch(const LaunchArgs& a, const TileCfg& t, cudaStream_t s, const AffineMap& aff = AffineMap{}) {
+template <int OP, typename IT>
+cudaError_t dispatch(const LaunchArgs& a, const TileCfg& t, cudaStream_t s) {
     switch (a.g.dp[0]) {
-        case 1: return launch_one<1, OP, IT, PUSH, AFF>(a, t, s, aff);
-        case 2: return launch_one<2, OP, IT, PUSH, AFF>(a, t, s, aff);
-        case 3: return launch_one<3, OP, IT, PUSH, AFF>(a, t, s, aff);
-        case 4: return launch_one<4, OP, IT, PUSH, AFF>(a, t, s, aff);
-        default: return launch_one<5, OP, IT, PUSH, AFF>(a, t, s, aff);
+        case 1: return launch_one<1, OP, IT>(a, t, s);
+        case 2: return launch_one<2, OP, IT>(a, t, s);
+        case 3: return launch_one<3, OP, IT>(a, t, s);
+        case 4: return launch_one<4, OP, IT>(a, t, s);
+        default: return launch_one<5, OP, IT>(a, t, s);
     }
 }
 
