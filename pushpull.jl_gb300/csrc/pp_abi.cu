@@ -55,8 +55,9 @@ int sm_count() {
 void set_error_message(const char* msg) { g_err = msg ? msg : ""; }
 
 // Stream-ordered scratch comes from a memory pool owned by this library, one per
-// device, that keeps its memory between calls (the device's default pool returns
-// memory to the system at every synchronisation, which would re-map it per call).
+// device, that keeps its memory (up to kScratchKeep) between calls: the device's
+// default pool returns memory to the system at every synchronisation, which would
+// re-map it per call.
 static cudaError_t scratch_pool(cudaMemPool_t* out) {
     static std::mutex mu;
     static cudaMemPool_t pools[64] = {};
@@ -72,7 +73,7 @@ static cudaError_t scratch_pool(cudaMemPool_t* out) {
         props.location.id = dev;
         cudaMemPool_t p;
         if ((e = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return e;
-        unsigned long long keep = ~0ULL;
+        unsigned long long keep = kScratchKeep;
         if ((e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) return e;
         pools[dev] = p;
     }
@@ -210,6 +211,32 @@ int prepare_args(LaunchArgs& a, float* out, const float* phi, const float* in, c
     return prepare(a, out, phi, in, d0, d1, nc, nb, bnd, nbnd, deg, ext);
 }
 
+// Sample grids on which the per-voxel kernels beat the warp-specialised ones:
+// small ones, because those take 1920 voxels per CTA at a time, and larger ones
+// where their boxes do not arrive by TMA alone (odd x extents, circulant margins).
+// Device us per-voxel / warp-specialised, one channel, pull, GB300.  Clean: linear
+// 128^3 29 / 33, 192^3 78 / 80 (pull_grad 111 / 95); quadratic 64^3 15 / 15,
+// 92x108x92 25 / 25, 128^3 56 / 42; cubic 48^3 11 / 15, 64^3 17 / 19, 92x108x92
+// 38 / 33; quartic 64^3 23 / 23, 92x108x92 62 / 50.  Odd extents: linear
+// 181x217x181 76 / 133; quadratic 121x145x121 46 / 57, 181x217x181 138 / 151; cubic
+// 91x109x91 40 / 43, 121x145x121 (two channels) 121 / 118; quartic 61x73x61 27 /
+// 32, 91x109x91 66 / 63.  Circulant: quadratic 128^3 54 / 58, cubic 76 / 74.
+static bool prefer_per_voxel(const LaunchArgs& a) {
+    const Geometry& g = a.g;
+    if (g.dp[0] != g.dp[1] || g.dp[1] != g.dp[2] || g.n0 >= (1LL << 31) - 1) return false;
+    const long long n = g.n1 * g.nb;
+    const bool odd = (g.d1[0] & 3) || (reinterpret_cast<uintptr_t>(a.phi) & 15);
+    bool rough = odd || (g.d0[0] & 3) || (reinterpret_cast<uintptr_t>(a.in) & 15);
+    for (int c = 0; c < g.nbnd; ++c)
+        rough = rough || !a.bnd.code[c][0] || !a.bnd.code[c][1] || !a.bnd.code[c][2];
+    switch (g.dp[0]) {
+        case 2: return rough || n <= (1LL << 21);
+        case 3: return odd || n <= (rough ? 1LL << 21 : 1LL << 19);
+        case 4: return n <= (rough ? 1LL << 21 : 1LL << 19);
+        default: return n <= (rough ? 1LL << 20 : 1LL << 18);
+    }
+}
+
 static int run_pull(int op, float* out, const float* phi, const float* f0, const pp_usize d0[3],
                     const pp_usize d1[3], int nc, int nb, const int* bnd, int nbnd, const int deg[3],
                     int ext, void* stream, const float* up = nullptr) {
@@ -225,8 +252,9 @@ static int run_pull(int op, float* out, const float* phi, const float* f0, const
     cudaError_t e = cudaErrorNotSupported;
     const bool auto_path = current_path() != PP_PATH_DIRECT;
     if (auto_path && is_ws_tile(t)) {
-        if (ws_supported(a)) e = launch_ws_pull(op, a, (cudaStream_t)stream);
-        if (e == cudaErrorNotSupported) {
+        if (prefer_per_voxel(a)) t.cap = 0;
+        else if (ws_supported(a)) e = launch_ws_pull(op, a, (cudaStream_t)stream);
+        if (e == cudaErrorNotSupported && t.cap > 0) {
             (void)cudaGetLastError();
             // ops or geometries the warp-specialised kernels do not take: the
             // block-synchronous kernels, or the per-voxel ones at one or two taps per axis

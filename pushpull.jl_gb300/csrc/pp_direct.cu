@@ -1,5 +1,5 @@
-// pp_direct.cu -- pull / pull_grad / pull_hess / push / push_grad, one thread per
-// sample voxel against global memory.
+// pp_direct.cu -- pull / pull_grad / pull_hess / push / push_grad, per sample voxel
+// against global memory.
 //
 // The general path: any degree triple (including anisotropic ones), any sample
 // grid shape (the host-pointer ABI passes only n1), any deformation.  Weights are
@@ -15,7 +15,7 @@ namespace pp {
 namespace {
 
 template <int DP, int OP, typename IT>
-__global__ void __launch_bounds__(256) k_pull_direct(LaunchArgs a) {
+__global__ void __launch_bounds__(256, DP >= 4 ? 2 : 0) k_pull_direct(LaunchArgs a) {
     const Geometry& g = a.g;
     const long long n1 = g.n1;
     const int b = blockIdx.y;
@@ -30,128 +30,105 @@ __global__ void __launch_bounds__(256) k_pull_direct(LaunchArgs a) {
     }
 }
 
-// Channel c of the pull family for one valid voxel into registers: the same
-// arithmetic as pull_voxel_global for that channel.
-template <int DP, int OP, typename IT>
-__device__ __forceinline__ void pull_voxel_regs(const LaunchArgs& a, int b, int c, float x0, float x1, float x2,
-                                                float (&r)[6]) {
-    const Geometry& g = a.g;
-    const IT sy = (IT)g.d0[0];
-    const IT sz = (IT)(g.d0[0] * g.d0[1]);
-    Axis<DP, op_order(OP), IT> ax, ay, az;
-    constexpr int N = Axis<DP, op_order(OP), IT>::N;
-    int b0, b1, b2;
-    bnd_code(a, c, b0, b1, b2);
-    ax.setup(x0, g.dp[0], b0, g.d0[0], (IT)1);
-    ay.setup(x1, g.dp[1], b1, g.d0[1], sy);
-    az.setup(x2, g.dp[2], b2, g.d0[2], sz);
-    const float* f0 = a.in + ((long long)b * g.nc + c) * g.n0;
-    contract<OP, N>(ax, ay, az, ax.n, ay.n, az.n, DP == 0,
-                    [&](int k, int j, int i) { return __ldg(f0 + (az.off[k] + ay.off[j] + ax.off[i])); }, r);
+// A voxel whose taps do not all lie inside the image: the general per-voxel path,
+// out of line so that its 64-bit folding does not weigh on the registers of the
+// common one.
+template <int DP, int OP>
+__device__ __noinline__ void pull_voxel_folded(const LaunchArgs& a, int b, long long v, float x0, float x1, float x2) {
+    pull_voxel_global<DP, OP, int>(a, b, v, x0, x1, x2);
 }
 
-// One axis of a voxel whose taps all lie inside the image: weights only.
+// Weights of one voxel whose taps all lie inside the image.
 template <int DP, int ORD>
-struct InAxis {
+struct InWeights {
     float w[DP];
     float dw[ORD >= 1 ? DP : 1];
     float hw[ORD >= 2 ? DP : 1];
 };
 
-// Channel c of pull / pull_grad for a voxel whose taps all lie inside the image (no folding, 32-bit offsets): false, with
-// nothing computed, otherwise.  The weights and the contraction are
-// pull_voxel_global's, so the bits are the same.
-template <int DP, int OP>
-__device__ __forceinline__ bool pull_voxel_inside(const float* f0, const Geometry& g, int sy, int sz, float x0,
-                                                  float x1, float x2, float (&r)[6]) {
+// The pull family at one to three taps per axis for images of fewer than 2^31
+// elements.  V voxels per thread, one block width apart, so that every load of a warp is
+// contiguous at any alignment while a thread keeps 12 V bytes of deformation
+// reads in flight.  Voxels whose taps all lie inside the image take a path of
+// 32-bit offsets from one address with weights shared by the channels; the others
+// the general one.  The arithmetic is pull_voxel_global's, bit for bit.
+// What bounds it is latency (a DRAM load, then dependent L2 gathers) and, from two
+// taps on, the gathers' L1 wavefronts.  GB300, 181x217x181, one channel, pull /
+// pull_grad, us, against one voxel per thread with folded 64-bit indices: degree 0
+// 76 / 81 -> 38 / 50 (192^3: 42 / 52 with 16-byte loads of four consecutive voxels
+// per thread, which odd sizes cannot use, 38 / 50 here), degree 1 91 / 140 -> 72 /
+// 107, degree 2 189 / 234 -> 124 / 154.  At four and five taps the 64 or 125
+// gathers in flight leave no registers for it (cubic 128^3 97 us, k_pull_direct 72).
+template <int DP, int OP_, int V>
+__global__ void __launch_bounds__(256, DP == 3 && op_order(OP_) <= 1 && !pull_is_dot<OP_>() ? 3 : 0) k_pull_lean(const __grid_constant__ LaunchArgs a) {
+    constexpr int OP = pull_base_op<OP_>();
     constexpr int ORD = op_order(OP);
-    InAxis<DP, ORD> ax, ay, az;
-    const int ox = spline_taps32<DP, ORD>(x0, ax.w, ax.dw, ax.hw);
-    const int oy = spline_taps32<DP, ORD>(x1, ay.w, ay.dw, ay.hw);
-    const int oz = spline_taps32<DP, ORD>(x2, az.w, az.dw, az.hw);
-    if (ox < 0 || oy < 0 || oz < 0 || ox > (int)g.d0[0] - DP || oy > (int)g.d0[1] - DP || oz > (int)g.d0[2] - DP)
-        return false;
-    const float* p = f0 + (oz * sz + oy * sy + ox);
-    contract<OP, DP>(ax, ay, az, DP, DP, DP, false, [&](int k, int j, int i) { return __ldg(p + (k * sz + j * sy + i)); },
-                     r);
-    return true;
-}
-
-struct Res6 {
-    float v[6];
-};
-
-// Any other voxel: the general per-voxel path, out of line so that its 64-bit
-// folding does not weigh on the registers of the common path.
-template <int DP, int OP>
-__device__ __noinline__ Res6 pull_voxel_folded(const LaunchArgs& a, int b, int c, float x0, float x1, float x2) {
-    Res6 o;
-    pull_voxel_regs<DP, OP, int>(a, b, c, x0, x1, x2, o.v);
-    return o;
-}
-
-// pull and pull_grad at one tap per axis (degree 0, nearest neighbour): four
-// consecutive sample voxels per thread and iteration.  The deformation arrives
-// by 16-byte loads, the next group's while this group gathers, so each thread
-// keeps 48 bytes of DRAM reads in flight (one voxel per thread leaves the
-// kernel latency-bound far below HBM bandwidth: 192^3, GB300, 0.080 -> 0.048
-// ms).  Channel by channel, the four voxels' results stay in registers up to
-// 16-byte stores, so their gathers overlap.  Voxels whose tap is inside the
-// image take a lean path; the rest the general one.  Same arithmetic as
-// k_pull_direct.  Needs n1 % 4 == 0, 16-byte aligned phi and output, and an
-// image of fewer than 2^31 elements.  (At two taps per axis the same scheme
-// measured slower than the warp-specialised kernels.)
-template <int OP>
-__global__ void __launch_bounds__(256, 4) k_pull_nearest(LaunchArgs a) {
-    constexpr int DP = 1;
-    constexpr int NCOMP = OP == kPull ? 1 : 3;
     const Geometry& g = a.g;
-    const long long n1 = g.n1, n4 = n1 >> 2;
+    const long long n1 = g.n1;
     const int b = blockIdx.y;
+    const int dx = (int)g.d0[0] - DP, dy = (int)g.d0[1] - DP, dz = (int)g.d0[2] - DP;
     const int sy = (int)g.d0[0], sz = (int)(g.d0[0] * g.d0[1]);
     const float* phi = a.phi + (long long)b * 3 * n1;
-    const float4* p0 = reinterpret_cast<const float4*>(phi);
-    const float4* p1 = reinterpret_cast<const float4*>(phi + n1);
-    const float4* p2 = reinterpret_cast<const float4*>(phi + 2 * n1);
-    const long long step = (long long)gridDim.x * blockDim.x;
-    long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0, c2 = c0;
-    if (q < n4) {
-        c0 = __ldg(p0 + q);
-        c1 = __ldg(p1 + q);
-        c2 = __ldg(p2 + q);
-    }
-    for (; q < n4; q += step) {
-        const float X[4] = {c0.x, c0.y, c0.z, c0.w};
-        const float Y[4] = {c1.x, c1.y, c1.z, c1.w};
-        const float Z[4] = {c2.x, c2.y, c2.z, c2.w};
-        if (q + step < n4) {
-            c0 = __ldg(p0 + q + step);
-            c1 = __ldg(p1 + q + step);
-            c2 = __ldg(p2 + q + step);
+    const float* fb = a.in + (long long)b * g.nc * g.n0;
+    for (long long v0 = (long long)blockIdx.x * (256 * V) + threadIdx.x; v0 < n1; v0 += (long long)gridDim.x * (256 * V)) {
+        float X[V][3];
+#pragma unroll
+        for (int u = 0; u < V; ++u) {
+            const long long v = v0 + u * 256;
+            const bool in = V == 1 || v < n1;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) X[u][k] = in ? __ldg(phi + v + k * n1) : qnan();
         }
-        const long long v0 = 4 * q;
+        int at[V];   // element of the first tap; -1 nothing left to do
+        InWeights<DP, ORD> wx[V], wy[V], wz[V];
+#pragma unroll
+        for (int u = 0; u < V; ++u) {
+            const long long v = v0 + u * 256;
+            float x0, x1, x2;
+            const bool ok = load_valid(X[u][0], X[u][1], X[u][2], g, x0, x1, x2);
+            const int ox = spline_taps32<DP, ORD>(x0, wx[u].w, wx[u].dw, wx[u].hw);
+            const int oy = spline_taps32<DP, ORD>(x1, wy[u].w, wy[u].dw, wy[u].hw);
+            const int oz = spline_taps32<DP, ORD>(x2, wz[u].w, wz[u].dw, wz[u].hw);
+            const bool inside = ok & (ox >= 0) & (oy >= 0) & (oz >= 0) & (ox <= dx) & (oy <= dy) & (oz <= dz);
+            at[u] = inside ? oz * sz + oy * sy + ox : -1;
+            if (!inside && (V == 1 || v < n1)) {
+                if (ok) pull_voxel_folded<DP, OP_>(a, b, v, x0, x1, x2);
+                else pull_voxel_nan<OP_>(a, b, v);
+            }
+        }
+        float acc[pull_is_dot<OP_>() ? V : 1][3];
+        if constexpr (pull_is_dot<OP_>()) {
+#pragma unroll
+            for (int u = 0; u < V; ++u) acc[u][0] = acc[u][1] = acc[u][2] = 0.f;
+        }
 #pragma unroll 1
         for (int c = 0; c < g.nc; ++c) {
-            const float* f0 = a.in + ((long long)b * g.nc + c) * g.n0;
-            float r[4][6];
-            bool ok[4];
+            const float* f0 = fb + (long long)c * g.n0;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                float x0, x1, x2;
-                ok[u] = load_valid(X[u], Y[u], Z[u], g, x0, x1, x2);
-                if (ok[u] && !pull_voxel_inside<DP, OP>(f0, g, sy, sz, x0, x1, x2, r[u])) {
-                    const Res6 o = pull_voxel_folded<DP, OP>(a, b, c, x0, x1, x2);
+            for (int u = 0; u < V; ++u) {
+                if (at[u] < 0) continue;
+                const float* p = f0 + at[u];
+                float r[6];
+                contract_rolled<OP, DP, DP>(
+                    wx[u], wy[u], wz[u],
+                    [&](int j, float(&f)[DP]) {
 #pragma unroll
-                    for (int p = 0; p < 6; ++p) r[u][p] = o.v[p];
-                }
+                        for (int i = 0; i < DP; ++i) f[i] = __ldg(p + j * sy + i);
+                    },
+                    [&]() { p += sz; }, r);
+                if constexpr (pull_is_dot<OP_>()) dot_accumulate<OP_>(a, b, c, v0 + u * 256, r, acc[u]);
+                else pull_store<OP>(pull_out<OP_>(a, b, c, v0 + u * 256), n1, r);
             }
-            float* o = pull_out<OP>(a, b, c, v0);
+        }
+        if constexpr (pull_is_dot<OP_>()) {
 #pragma unroll
-            for (int p = 0; p < NCOMP; ++p)
-                *reinterpret_cast<float4*>(o + p * n1) =
-                    make_float4(ok[0] ? r[0][p] : qnan(), ok[1] ? r[1][p] : qnan(), ok[2] ? r[2][p] : qnan(),
-                                ok[3] ? r[3][p] : qnan());
+            for (int u = 0; u < V; ++u) {
+                if (at[u] < 0) continue;
+                float* o = pull_out<OP_>(a, b, 0, v0 + u * 256);
+                o[0] = acc[u][0];
+                o[n1] = acc[u][1];
+                o[2 * n1] = acc[u][2];
+            }
         }
     }
 }
@@ -172,8 +149,22 @@ __global__ void __launch_bounds__(256) k_push_direct(LaunchArgs a) {
 
 template <int DP, int OP, typename IT, bool PUSH>
 void launch_one(const LaunchArgs& a, dim3 grid, cudaStream_t s) {
-    if constexpr (PUSH) k_push_direct<DP, OP, IT><<<grid, 256, 0, s>>>(a);
-    else k_pull_direct<DP, OP, IT><<<grid, 256, 0, s>>>(a);
+    if constexpr (PUSH) {
+        k_push_direct<DP, OP, IT><<<grid, 256, 0, s>>>(a);
+    } else if constexpr (DP > 0 && DP <= 3 && sizeof(IT) == 4) {
+        // four voxels per thread only at one tap per axis, and only when that still
+        // fills the chip (121^3, degree 0: 17 us against 19 with one; 181x217x181:
+        // 38 against 66; 64^3: 11 against 9)
+        if (DP == 1 && a.g.n1 * a.g.nb >= (1LL << 20)) {
+            constexpr int V = DP == 1 ? 4 : 1;
+            const long long blocks = (a.g.n1 + 256 * V - 1) / (256 * V), cap = (long long)sm_count() * 8;
+            k_pull_lean<DP, OP, V><<<dim3((unsigned)(blocks < cap ? blocks : cap), grid.y), 256, 0, s>>>(a);
+        } else {
+            k_pull_lean<DP, OP, 1><<<grid, 256, 0, s>>>(a);
+        }
+    } else {
+        k_pull_direct<DP, OP, IT><<<grid, 256, 0, s>>>(a);
+    }
 }
 
 template <int OP, typename IT, bool PUSH>
@@ -199,26 +190,7 @@ dim3 direct_grid(const LaunchArgs& a) {
 
 }  // namespace
 
-// k_pull_nearest for pull and pull_grad at degree 0 when the sample count is a
-// multiple of 4, phi and the output are 16-byte aligned and the image has fewer
-// than 2^31 elements.
-cudaError_t launch_pull_nearest(int op, const LaunchArgs& a, cudaStream_t s) {
-    const Geometry& g = a.g;
-    if ((op != kPull && op != kPullGrad) || g.dp[0] != 1 || g.dp[1] != 1 || g.dp[2] != 1) return cudaErrorNotSupported;
-    if ((g.n1 & 3) || (reinterpret_cast<uintptr_t>(a.phi) & 15) || (reinterpret_cast<uintptr_t>(a.out) & 15) ||
-        g.n0 >= (1LL << 31) - 1)
-        return cudaErrorNotSupported;
-    const long long blocks_needed = ((g.n1 >> 2) + 255) / 256;
-    const long long cap = (long long)sm_count() * 4;
-    const dim3 grid((unsigned)(blocks_needed < cap ? blocks_needed : cap), (unsigned)g.nb);
-    if (op == kPull) k_pull_nearest<kPull><<<grid, 256, 0, s>>>(a);
-    else k_pull_nearest<kPullGrad><<<grid, 256, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_pull_direct(int op, const LaunchArgs& a, cudaStream_t s) {
-    const cudaError_t en = launch_pull_nearest(op, a, s);
-    if (en != cudaErrorNotSupported) return en;
     const dim3 grid = direct_grid(a);
     const bool small = a.g.n0 < (1LL << 31) - 1;
     switch (op) {

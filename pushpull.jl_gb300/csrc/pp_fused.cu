@@ -47,9 +47,20 @@ __global__ void __launch_bounds__(256) k_fused_direct(const __grid_constant__ La
             }
             const float* f0 = a.in + ((long long)b * g.nc + c) * g.n0;
             float r[6];
-            contract<kPullValGrad, N>(ax, ay, az, ax.n, ay.n, az.n, DP == 0,
-                                      [&](int k, int j, int i) { return __ldg(f0 + (az.off[k] + ay.off[j] + ax.off[i])); },
-                                      r);
+            if constexpr (DP > 0) {
+                int k = 0;
+                contract_rolled<kPullValGrad, DP, DP>(
+                    ax, ay, az,
+                    [&](int j, float(&f)[DP]) {
+#pragma unroll
+                        for (int i = 0; i < DP; ++i) f[i] = __ldg(f0 + (az.off[k] + ay.off[j] + ax.off[i]));
+                    },
+                    [&]() { ++k; }, r);
+            } else {
+                contract<kPullValGrad, N>(
+                    ax, ay, az, ax.n, ay.n, az.n,
+                    [&](int k, int j, int i) { return __ldg(f0 + (az.off[k] + ay.off[j] + ax.off[i])); }, r);
+            }
             const float res = r[3] - __ldg(a.up + ((long long)b * g.nc + c) * n1 + v);
             loss += (double)(res * res);
             const float d = 2.f * res;

@@ -49,6 +49,12 @@ cudaError_t launch_sum_partials(const double* partial, int n, double* out, cudaS
 // max |f| of each of `planes` contiguous volumes of n voxels into out[planes] (zeroed by the caller)
 cudaError_t launch_absmax(const float* f, long long n, int planes, unsigned* out, cudaStream_t s);
 
+// Stream-ordered scratch from a pool owned by this library (one per device),
+// which keeps up to kScratchKeep bytes between calls and gives back the rest;
+// freed with cudaFreeAsync.
+constexpr size_t kScratchKeep = 512u << 20;
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+
 // number of SMs of the current device (cached per device)
 int sm_count();
 

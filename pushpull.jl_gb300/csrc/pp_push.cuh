@@ -23,7 +23,7 @@
 // element (about 2.3 q for 64 contributions) by 7e-8 of the tile's mean value;
 // it is 1e-8 for image-like values and 3e-8 for noise, below the rounding of the
 // float32 weights.  Other tiles (a few values among zeros, large dynamic range)
-// scatter in two passes: the upper and the lower word of a 43-bit fixed point,
+// scatter in two passes: the upper and the lower word of a 42-bit fixed point,
 // each flushed by itself.
 //
 // Lanes: a warp covers 2^lx voxels in x and 32 / 2^lx rows.  The row pitch is

@@ -39,6 +39,7 @@ struct TileGrid {
     int cap;            // box budget in floats
     int pmod;           // box row pitch P is chosen with P % 32 == pmod
     int img_tma;        // pull: interior boxes may be loaded with one TMA copy (image tensor map valid)
+    int phi_tma;        // warp-specialised pull: the deformation streams by TMA
     int nv, stages;     // push: voxels per tile, ring slots
 };
 

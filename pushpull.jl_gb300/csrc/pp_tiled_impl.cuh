@@ -134,8 +134,10 @@ struct Box {
     int ext[3];     // box extent (x counted from xo)
     int P, Q, size; // row pitch (P % 32 == pmod, P % 4 == 0), plane pitch (multiple of 32), floats
     int mode;       // 0 no valid voxel, 1 shared memory, 2 per-voxel global fallback
+    int base;       // warp-specialised pull: first word of the box in its buffer (0..3)
     int interior;   // bit k: the box lies inside the image along dimension k (no folding)
-    int tma;        // 1: the box is a fixed window loaded by one TMA copy; 2: the same, with mirrored margins to complete
+    int tma;        // 1: the box is a fixed window loaded by one TMA copy; 2: the same, with mirrored margins to
+                    // complete; 3: loaded row by row; 4: the same, DST-II signs to apply
     float S;        // block sum of the caller's per-thread value (push: bound on sum |contribution|)
     int E;          // scale exponent of the fixed-point accumulator for S (see scale_exponent)
 };
@@ -686,127 +688,16 @@ __device__ __forceinline__ void tile_bounds(const Geometry& g, const TileOrigin&
     tile_bounds_pos<DP, V, IT>(g, o, tv, TilePos<kThreads * V, false>{slot, nullptr, 0, 0}, mn, mx);
 }
 
-// The patch contraction of contract() (pp_voxel.cuh) with the z loop rolled:
-// the z weights rotate through slot 0 and `next()` advances the loader to the
-// next plane, so only one plane of rows is in flight (a fully unrolled patch
-// needs more registers than two resident CTAs per SM leave).  Rows are taken in
-// pairs on the packed f32x2 pipe.  `row(j, f)` loads row j of the current plane
-// into f[0..DP).
-template <int OP, int DP, class WT, class ROW, class NEXT>
-__device__ __forceinline__ void contract_rolled(const WT& ax, const WT& ay, WT az, ROW row, NEXT next,
-                                                float (&r)[6]) {
-    constexpr int ORD = op_order(OP);
-    constexpr int NJ = OP == kPull ? 1 : (ORD == 1 ? 3 : 6);   // y-level accumulators
-#pragma unroll
-    for (int q = 0; q < 6; ++q) r[q] = 0.f;
-    // x weights duplicated into f32x2 pairs once: rows are contracted two at a
-    // time on the packed pipe (lane 0: row j, lane 1: row j + 1)
-    float2 wx2[DP], dwx2[ORD >= 1 ? DP : 1], hwx2[ORD >= 2 ? DP : 1];
-#pragma unroll
-    for (int i = 0; i < DP; ++i) {
-        wx2[i] = make_float2(ax.w[i], ax.w[i]);
-        if constexpr (ORD >= 1) dwx2[i] = make_float2(ax.dw[i], ax.dw[i]);
-        if constexpr (ORD >= 2) hwx2[i] = make_float2(ax.hw[i], ax.hw[i]);
-    }
-    // pull keeps two planes in flight; the derivative ops, with more
-    // accumulators, one (two would need more registers than 2 CTAs/SM leave)
-    constexpr int KU = OP == kPull ? 2 : 1;
-#pragma unroll KU
-    for (int k = 0; k < DP; ++k) {
-        float2 J[NJ];
-#pragma unroll
-        for (int q = 0; q < NJ; ++q) J[q] = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j + 1 < DP; j += 2) {
-            float fa[DP], fb[DP];
-            row(j, fa);
-            row(j + 1, fb);
-            float2 I0 = make_float2(0.f, 0.f), I1 = I0, I2 = I0;
-#pragma unroll
-            for (int i = 0; i < DP; ++i) {
-                const float2 f2 = make_float2(fa[i], fb[i]);
-                I0 = __ffma2_rn(wx2[i], f2, I0);
-                if constexpr (ORD >= 1) I1 = __ffma2_rn(dwx2[i], f2, I1);
-                if constexpr (ORD >= 2) I2 = __ffma2_rn(hwx2[i], f2, I2);
-            }
-            const float2 wy = make_float2(ay.w[j], ay.w[j + 1]);
-            if constexpr (OP == kPull) {
-                J[0] = __ffma2_rn(wy, I0, J[0]);
-            } else if constexpr (ORD == 1) {
-                const float2 dwy = make_float2(ay.dw[j], ay.dw[j + 1]);
-                J[0] = __ffma2_rn(wy, I1, J[0]);
-                J[1] = __ffma2_rn(dwy, I0, J[1]);
-                J[2] = __ffma2_rn(wy, I0, J[2]);
-            } else {
-                const float2 dwy = make_float2(ay.dw[j], ay.dw[j + 1]);
-                const float2 hwy = make_float2(ay.hw[j], ay.hw[j + 1]);
-                J[0] = __ffma2_rn(wy, I2, J[0]);
-                J[1] = __ffma2_rn(hwy, I0, J[1]);
-                J[2] = __ffma2_rn(wy, I0, J[2]);
-                J[3] = __ffma2_rn(dwy, I1, J[3]);
-                J[4] = __ffma2_rn(wy, I1, J[4]);
-                J[5] = __ffma2_rn(dwy, I0, J[5]);
-            }
-        }
-        if constexpr (DP & 1) {   // the last row alone, into lane 0
-            constexpr int j = DP - 1;
-            float f[DP];
-            row(j, f);
-            float i0 = 0.f, i1 = 0.f, i2 = 0.f;
-#pragma unroll
-            for (int i = 0; i < DP; ++i) {
-                i0 = fmaf(ax.w[i], f[i], i0);
-                if constexpr (ORD >= 1) i1 = fmaf(ax.dw[i], f[i], i1);
-                if constexpr (ORD >= 2) i2 = fmaf(ax.hw[i], f[i], i2);
-            }
-            if constexpr (OP == kPull) {
-                J[0].x = fmaf(ay.w[j], i0, J[0].x);
-            } else if constexpr (ORD == 1) {
-                J[0].x = fmaf(ay.w[j], i1, J[0].x);
-                J[1].x = fmaf(ay.dw[j], i0, J[1].x);
-                J[2].x = fmaf(ay.w[j], i0, J[2].x);
-            } else {
-                J[0].x = fmaf(ay.w[j], i2, J[0].x);
-                J[1].x = fmaf(ay.hw[j], i0, J[1].x);
-                J[2].x = fmaf(ay.w[j], i0, J[2].x);
-                J[3].x = fmaf(ay.dw[j], i1, J[3].x);
-                J[4].x = fmaf(ay.w[j], i1, J[4].x);
-                J[5].x = fmaf(ay.dw[j], i0, J[5].x);
-            }
-        }
-        float jv[NJ];
-#pragma unroll
-        for (int q = 0; q < NJ; ++q) jv[q] = J[q].x + J[q].y;
-        if constexpr (OP == kPull) {
-            r[0] = fmaf(az.w[0], jv[0], r[0]);
-        } else if constexpr (ORD == 1) {
-            r[0] = fmaf(az.w[0], jv[0], r[0]);
-            r[1] = fmaf(az.w[0], jv[1], r[1]);
-            r[2] = fmaf(az.dw[0], jv[2], r[2]);
-            if constexpr (OP == kPullValGrad) r[3] = fmaf(az.w[0], jv[2], r[3]);
-        } else {
-            r[0] = fmaf(az.w[0], jv[0], r[0]);
-            r[1] = fmaf(az.w[0], jv[1], r[1]);
-            r[2] = fmaf(az.hw[0], jv[2], r[2]);
-            r[3] = fmaf(az.w[0], jv[3], r[3]);
-            r[4] = fmaf(az.dw[0], jv[4], r[4]);
-            r[5] = fmaf(az.dw[0], jv[5], r[5]);
-        }
-#pragma unroll
-        for (int i = 0; i + 1 < DP; ++i) {
-            az.w[i] = az.w[i + 1];
-            if constexpr (ORD >= 1) az.dw[i] = az.dw[i + 1];
-            if constexpr (ORD >= 2) az.hw[i] = az.hw[i + 1];
-        }
-        next();
-    }
-}
+// Planes in flight in the tiled kernels: two for pull; the derivative ops, with
+// more accumulators, one (two would need more registers than 2 CTAs/SM leave).
+template <int OP>
+constexpr int kRolled = OP == kPull ? 2 : 1;
 
 // contract_rolled over the shared box: row (k, j) starts at p + k*Q4 + j*P4.
 template <int OP, int DP, class WT>
 __device__ __forceinline__ void contract_smem(const WT& ax, const WT& ay, const WT& az, unsigned p, unsigned P4,
                                               unsigned Q4, float (&r)[6]) {
-    contract_rolled<OP, DP>(
+    contract_rolled<OP, DP, kRolled<OP>>(
         ax, ay, az, [&](int j, float (&f)[DP]) { lds_row<DP>(p + j * P4, f); }, [&]() { p += Q4; }, r);
 }
 
@@ -837,7 +728,7 @@ __device__ __forceinline__ void pull_voxel_lean(const LaunchArgs& a, int b, long
 #pragma unroll
         for (int i = 0; i < DP; ++i) zo[i] = az.off[i];
         float r[6];
-        contract_rolled<OP, DP>(
+        contract_rolled<OP, DP, kRolled<OP>>(
             ax, ay, az,
             [&](int j, float (&f)[DP]) {
 #pragma unroll
@@ -1213,7 +1104,7 @@ __device__ __forceinline__ float fused_voxel_global(const LaunchArgs& a, int b, 
 #pragma unroll
     for (int i = 0; i < DP; ++i) zo[i] = az.off[i];
     float r[6];
-    contract_rolled<kPullValGrad, DP>(
+    contract_rolled<kPullValGrad, DP, 1>(
         ax, ay, az,
         [&](int j, float (&f)[DP]) {
 #pragma unroll
@@ -1630,7 +1521,7 @@ __device__ __noinline__ void batch_tile_any(const BatchItem& it, int lt) {
             }
             const float* f0 = a.in + (long long)c * g.n0;
             float r[6];
-            contract<kPull, N>(ax, ay, az, ax.n, ay.n, az.n, true,
+            contract<kPull, N>(ax, ay, az, ax.n, ay.n, az.n,
                                [&](int k, int j, int i) { return __ldg(f0 + (az.off[k] + ay.off[j] + ax.off[i])); }, r);
             a.out[(long long)c * n1 + v] = r[0];
             if (!finitef(r[0])) continue;
@@ -1707,7 +1598,7 @@ TileGrid make_grid(const LaunchArgs& a, const TileCfg& c) {
     magic(t.ntz, t.mz, t.sz);
     const int tx = 1 << c.lx;
     t.pmod = tx >= 32 ? 0 : tx;
-    t.img_tma = 0;
+    t.img_tma = t.phi_tma = 0;
     t.nv = tx << (c.ly + c.lz);
     t.stages = 0;
     return t;

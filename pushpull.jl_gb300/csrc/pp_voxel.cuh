@@ -96,25 +96,137 @@ __device__ __forceinline__ void pull_store(float* o, long long n1, const float (
     }
 }
 
-// Separable patch contraction.  `tap(k, j, i)` returns the (signed) image value of
-// tap (i, j, k); weights come from the three axes.  Results in r[] as pull_store
-// expects; kPullValGrad returns the gradient in r[0..2] and the value in r[3].
+// The separable patch contraction of every isotropic pull path (so that they all
+// give the same bits).  The z weights rotate through slot 0 and `next()` advances
+// the loader to the next plane; KU planes are unrolled and so in flight.  Rows are
+// taken in pairs on the packed f32x2 pipe.  `row(j, f)` loads row j of the current
+// plane into f[0..DP).  Results in r[] as pull_store expects; kPullValGrad returns
+// the gradient in r[0..2] and the value in r[3].
+template <int OP, int DP, int KU, class WT, class ROW, class NEXT>
+__device__ __forceinline__ void contract_rolled(const WT& ax, const WT& ay, WT az, ROW row, NEXT next,
+                                                float (&r)[6]) {
+    constexpr int ORD = op_order(OP);
+    constexpr int NJ = OP == kPull ? 1 : (ORD == 1 ? 3 : 6);   // y-level accumulators
+#pragma unroll
+    for (int q = 0; q < 6; ++q) r[q] = 0.f;
+    // x weights duplicated into f32x2 pairs once: rows are contracted two at a
+    // time on the packed pipe (lane 0: row j, lane 1: row j + 1)
+    float2 wx2[DP], dwx2[ORD >= 1 ? DP : 1], hwx2[ORD >= 2 ? DP : 1];
+#pragma unroll
+    for (int i = 0; i < DP; ++i) {
+        wx2[i] = make_float2(ax.w[i], ax.w[i]);
+        if constexpr (ORD >= 1) dwx2[i] = make_float2(ax.dw[i], ax.dw[i]);
+        if constexpr (ORD >= 2) hwx2[i] = make_float2(ax.hw[i], ax.hw[i]);
+    }
+#pragma unroll KU
+    for (int k = 0; k < DP; ++k) {
+        float2 J[NJ];
+#pragma unroll
+        for (int q = 0; q < NJ; ++q) J[q] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j + 1 < DP; j += 2) {
+            float fa[DP], fb[DP];
+            row(j, fa);
+            row(j + 1, fb);
+            float2 I0 = make_float2(0.f, 0.f), I1 = I0, I2 = I0;
+#pragma unroll
+            for (int i = 0; i < DP; ++i) {
+                const float2 f2 = make_float2(fa[i], fb[i]);
+                I0 = __ffma2_rn(wx2[i], f2, I0);
+                if constexpr (ORD >= 1) I1 = __ffma2_rn(dwx2[i], f2, I1);
+                if constexpr (ORD >= 2) I2 = __ffma2_rn(hwx2[i], f2, I2);
+            }
+            const float2 wy = make_float2(ay.w[j], ay.w[j + 1]);
+            if constexpr (OP == kPull) {
+                J[0] = __ffma2_rn(wy, I0, J[0]);
+            } else if constexpr (ORD == 1) {
+                const float2 dwy = make_float2(ay.dw[j], ay.dw[j + 1]);
+                J[0] = __ffma2_rn(wy, I1, J[0]);
+                J[1] = __ffma2_rn(dwy, I0, J[1]);
+                J[2] = __ffma2_rn(wy, I0, J[2]);
+            } else {
+                const float2 dwy = make_float2(ay.dw[j], ay.dw[j + 1]);
+                const float2 hwy = make_float2(ay.hw[j], ay.hw[j + 1]);
+                J[0] = __ffma2_rn(wy, I2, J[0]);
+                J[1] = __ffma2_rn(hwy, I0, J[1]);
+                J[2] = __ffma2_rn(wy, I0, J[2]);
+                J[3] = __ffma2_rn(dwy, I1, J[3]);
+                J[4] = __ffma2_rn(wy, I1, J[4]);
+                J[5] = __ffma2_rn(dwy, I0, J[5]);
+            }
+        }
+        if constexpr (DP & 1) {   // the last row alone, into lane 0
+            constexpr int j = DP - 1;
+            float f[DP];
+            row(j, f);
+            float i0 = 0.f, i1 = 0.f, i2 = 0.f;
+#pragma unroll
+            for (int i = 0; i < DP; ++i) {
+                i0 = fmaf(ax.w[i], f[i], i0);
+                if constexpr (ORD >= 1) i1 = fmaf(ax.dw[i], f[i], i1);
+                if constexpr (ORD >= 2) i2 = fmaf(ax.hw[i], f[i], i2);
+            }
+            if constexpr (OP == kPull) {
+                J[0].x = fmaf(ay.w[j], i0, J[0].x);
+            } else if constexpr (ORD == 1) {
+                J[0].x = fmaf(ay.w[j], i1, J[0].x);
+                J[1].x = fmaf(ay.dw[j], i0, J[1].x);
+                J[2].x = fmaf(ay.w[j], i0, J[2].x);
+            } else {
+                J[0].x = fmaf(ay.w[j], i2, J[0].x);
+                J[1].x = fmaf(ay.hw[j], i0, J[1].x);
+                J[2].x = fmaf(ay.w[j], i0, J[2].x);
+                J[3].x = fmaf(ay.dw[j], i1, J[3].x);
+                J[4].x = fmaf(ay.w[j], i1, J[4].x);
+                J[5].x = fmaf(ay.dw[j], i0, J[5].x);
+            }
+        }
+        float jv[NJ];
+#pragma unroll
+        for (int q = 0; q < NJ; ++q) jv[q] = J[q].x + J[q].y;
+        if constexpr (OP == kPull) {
+            r[0] = fmaf(az.w[0], jv[0], r[0]);
+        } else if constexpr (ORD == 1) {
+            r[0] = fmaf(az.w[0], jv[0], r[0]);
+            r[1] = fmaf(az.w[0], jv[1], r[1]);
+            r[2] = fmaf(az.dw[0], jv[2], r[2]);
+            if constexpr (OP == kPullValGrad) r[3] = fmaf(az.w[0], jv[2], r[3]);
+        } else {
+            r[0] = fmaf(az.w[0], jv[0], r[0]);
+            r[1] = fmaf(az.w[0], jv[1], r[1]);
+            r[2] = fmaf(az.hw[0], jv[2], r[2]);
+            r[3] = fmaf(az.w[0], jv[3], r[3]);
+            r[4] = fmaf(az.dw[0], jv[4], r[4]);
+            r[5] = fmaf(az.dw[0], jv[5], r[5]);
+        }
+#pragma unroll
+        for (int i = 0; i + 1 < DP; ++i) {
+            az.w[i] = az.w[i + 1];
+            if constexpr (ORD >= 1) az.dw[i] = az.dw[i + 1];
+            if constexpr (ORD >= 2) az.hw[i] = az.hw[i + 1];
+        }
+        next();
+    }
+}
+
+// The same for runtime widths nx, ny, nz (per-dimension degrees), up to N taps per
+// axis: `tap(k, j, i)` returns the (signed) image value of tap (i, j, k).
 template <int OP, int N, class AX, class AY, class AZ, class TAP>
 __device__ __forceinline__ void contract(const AX& ax, const AY& ay, const AZ& az, int nx, int ny, int nz,
-                                         bool runtime_n, TAP tap, float (&r)[6]) {
+                                         TAP tap, float (&r)[6]) {
 #pragma unroll
     for (int q = 0; q < 6; ++q) r[q] = 0.f;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-        if (runtime_n && k >= nz) break;
+        if (k >= nz) break;
         float j0 = 0.f, j1 = 0.f, j2 = 0.f, j3 = 0.f, j4 = 0.f, j5 = 0.f;
 #pragma unroll
         for (int j = 0; j < N; ++j) {
-            if (runtime_n && j >= ny) break;
+            if (j >= ny) break;
             float i0 = 0.f, i1 = 0.f, i2 = 0.f;
 #pragma unroll
             for (int i = 0; i < N; ++i) {
-                if (runtime_n && i >= nx) break;
+                if (i >= nx) break;
                 const float f = tap(k, j, i);
                 i0 = fmaf(ax.w[i], f, i0);
                 if constexpr (op_order(OP) >= 1) i1 = fmaf(ax.dw[i], f, i1);
@@ -177,8 +289,19 @@ __device__ __forceinline__ void pull_voxel_global(const LaunchArgs& a, int b, lo
         }
         const float* f0 = a.in + ((long long)b * g.nc + c) * g.n0;
         float r[6];
-        contract<OP, N>(ax, ay, az, ax.n, ay.n, az.n, DP == 0,
-                        [&](int k, int j, int i) { return __ldg(f0 + (az.off[k] + ay.off[j] + ax.off[i])); }, r);
+        if constexpr (DP > 0) {
+            int k = 0;
+            contract_rolled<OP, DP, DP>(
+                ax, ay, az,
+                [&](int j, float(&f)[DP]) {
+#pragma unroll
+                    for (int i = 0; i < DP; ++i) f[i] = __ldg(f0 + (az.off[k] + ay.off[j] + ax.off[i]));
+                },
+                [&]() { ++k; }, r);
+        } else {
+            contract<OP, N>(ax, ay, az, ax.n, ay.n, az.n,
+                            [&](int k, int j, int i) { return __ldg(f0 + (az.off[k] + ay.off[j] + ax.off[i])); }, r);
+        }
         if constexpr (pull_is_dot<OP_>()) dot_accumulate<OP_>(a, b, c, v, r, acc);
         else pull_store<OP>(pull_out<OP_>(a, b, c, v), n1, r);
     }

@@ -18,12 +18,23 @@
 //     still evaluate the previous unit; it then publishes the box record;
 //   * boundary boxes whose margins mirror (DCT-II, DST-II) onto elements of the
 //     box itself arrive by the same TMA copy, zero-filled outside the image,
-//     and the consumers complete the margins in shared memory; other boundary
-//     boxes (circulant margins) are gathered by all the consumers when they
-//     take the unit, 16-byte chunks where a row is in range.  Both sit behind
-//     consumer-only named barriers.
+//     and the consumers complete the margins in shared memory behind
+//     consumer-only named barriers;
+//   * other boundary boxes (circulant margins) are loaded by the consumers when
+//     they take the unit, row by row with cp.async, folded on the way, 16-byte
+//     chunks where a row allows it (pitches congruent to the image's make that
+//     the rule for odd extents too), then signed if a margin is DST-II;
+//   * of an image whose rows are not multiples of 16 bytes, every box is loaded
+//     that way, but one unit ahead: bounds are published two tiles ahead, and the
+//     copies of unit q + 1 are in flight while unit q is evaluated (one producer
+//     warp issuing them instead took 25 us a box);
+//   * a deformation that TMA cannot address (odd x extent) is copied by the
+//     consumer threads themselves, each the words of its own voxels, with
+//     cp.async groups as deep as the ring.
 // Interior units therefore pass no CTA-wide barrier at all.  Boxes larger than
 // a buffer take the per-voxel global path for that tile.
+// 181x217x181, cubic, GB300: pull 0.186 ms, pull_grad 0.217 ms (0.308 and 0.324 ms
+// on the block-synchronous kernels).
 //
 // Reference kernels replaced: pull_element / pullg_element / pullh_element
 // (artifacts/C/pushpull.cu:33-109); per-voxel math pull1 / pullg1 / pullh1
@@ -41,7 +52,7 @@ constexpr int kWsThreads = kWsCons + 32;       // plus the producer warp
 constexpr int kWsV = 4;                        // sample voxels per consumer thread
 constexpr int kWsTz = 30;                      // tile: 8 x 8 x 30 sample voxels
 constexpr int kWsNV = kWsCons * kWsV;          // 1920 voxels per tile
-constexpr int kWsStages = 3;                   // deformation ring slots
+constexpr int kWsStages = 4;                   // deformation ring slots
 constexpr int kWsBufs = 2;                     // box buffers
 constexpr int kWsWinX = 24, kWsWinY = 16, kWsWinZ = 40;   // TMA image window (row pitch 24)
 constexpr int kWsCap = kWsWinX * kWsWinY * kWsWinZ;         // floats per box buffer
@@ -139,6 +150,7 @@ __device__ __forceinline__ Box ws_tile_box(const Geometry& g, const int (*wrec)[
     box.S = 0.f;
     box.E = 0;
     box.tma = 0;
+    box.base = 0;
     if (mn[0] > mx[0]) {   // no valid voxel in the tile
         box.mode = 0;
         box.interior = 0;
@@ -171,72 +183,117 @@ __device__ __forceinline__ Box ws_tile_box(const Geometry& g, const int (*wrec)[
         box.ext[2] = (int)e2;
         return box;
     }
-    // gathered box: row pitch P % 32 == 8 keeps an 8 x 4 warp tile's rows in
-    // disjoint banks; pack tightly when the padding does not fit
-    long long P = (e0 + 3) & ~3LL;
-    const long long Pp = P + (((8 - (int)(P & 31)) + 32) & 31);
-    long long Q = (Pp * e1 + 31) & ~31LL;
-    if (Q * e2 <= kWsCap) {
-        P = Pp;
-    } else {
-        Q = (P * e1 + 3) & ~3LL;
-    }
-    const bool fits = e0 <= 4096 && e1 <= 4096 && e2 <= 4096 && Q * e2 <= kWsCap;
+    // boundary box, or an image TMA cannot address: provisional record with the
+    // window's extents; the producer decides per channel how it is loaded
+    const bool fits = e0 <= 4096 && e1 <= 4096 && e2 <= 4096;
     box.mode = fits ? 1 : 2;
     box.ext[0] = fits ? (int)e0 : 0;
     box.ext[1] = fits ? (int)e1 : 0;
     box.ext[2] = fits ? (int)e2 : 0;
-    box.P = fits ? (int)P : 0;
-    box.Q = fits ? (int)Q : 0;
-    box.size = fits ? (int)(Q * e2) : 0;
+    box.P = box.Q = box.size = 0;
+    box.lo[0] = mn[0];
     return box;
 }
 
-// Gather one channel of a box into shared memory with `nthreads` threads
-// (tid = 0 .. nthreads-1, nthreads a multiple of 32), folding (and signing)
-// out-of-range taps; in-range 16-byte row chunks are one vector load each.
-// Threads split over (row, chunk) pairs.
+// Pitches of a box that is loaded row by row (ws_async_box): congruent
+// to the image's row and plane modulo 4 elements, so that 16-byte chunks of a row
+// are aligned in both; the row pitch 8 or 24 modulo 32 (plus that remainder)
+// keeps an 8 x 4 warp tile's rows in nearly disjoint banks.  Three words lie
+// between rows: a row's first and last chunk may overwrite them.
+__device__ __forceinline__ void ws_async_pitch(Box& box, const Geometry& g, int lo0, int e0) {
+    const int rm = (int)(g.d0[0] & 3), pm = (int)((g.d0[0] * g.d0[1]) & 3);
+    box.xo = lo0;
+    box.ext[0] = e0;
+    const int least = e0 + 3;
+    int P = least + ((rm - least) & 3);
+    int Pb = 8 + rm;
+    while (Pb < least) Pb += 16;
+    const long long e1 = box.ext[1], e2 = box.ext[2];
+    long long Q = (long long)Pb * e1;
+    Q += (pm - Q) & 31;
+    if (Q * e2 + 8 <= kWsCap) {
+        P = Pb;
+    } else {
+        Q = (long long)P * e1;
+        Q += (pm - Q) & 3;
+    }
+    const bool fits = Q * e2 + 8 <= kWsCap;
+    box.mode = fits ? 1 : 2;
+    box.P = fits ? P : 0;
+    box.Q = fits ? (int)Q : 0;
+    box.size = fits ? (int)(Q * e2) : 0;
+    box.tma = 3;
+}
+
+// All consumer threads load one channel of a box row by row with cp.async,
+// eight lanes to a row, folding rows and elements outside the image onto their
+// sources (no signs: see ws_sign_box).  The caller commits and waits.
+// Rows that have the same 16-byte alignment in the image and in the box copy
+// whole chunks; chunks at the image's x ends, and rows whose source lies
+// elsewhere in an image of odd extents, copy elements.
 template <typename IT>
-__device__ __forceinline__ void ws_stage_gather(const Box& box, const Geometry& g, int b0, int b1, int b2,
-                                                const float* f0, float* sm, int tid, int nthreads) {
-    const int ex = box.ext[0], ey = box.ext[1], ez = box.ext[2];
-    const int n4 = (ex + 3) >> 2;
-    const int nn = n4 < 1 ? 1 : (n4 > 32 ? 32 : n4);
-    const int lg = 32 - __clz(nn - 1);          // threads per row = 1 << lg
-    const int lpr = 1 << lg;
-    const int sub = tid >> lg, e4 = tid & (lpr - 1), step = nthreads >> lg;
-    const bool vec = (g.d0[0] & 3) == 0 && (reinterpret_cast<uintptr_t>(f0) & 15) == 0;
+__device__ __forceinline__ void ws_async_box(const Box& box, const Geometry& g, int b0, int b1, int b2,
+                                             const float* f0, float* sm, int tid) {
+    const int ex = box.ext[0], ey = box.ext[1], rows = ey * box.ext[2], dx = (int)g.d0[0];
     const IT sy = (IT)g.d0[0];
     const IT sz = (IT)(g.d0[0] * g.d0[1]);
-    const long long dx = g.d0[0];
-    const int nrows = ey * ez;
-    for (int r = sub; r < nrows; r += step) {
-        const int rz = r / ey, ry = r - rz * ey;
-        float sgy = 1.f, sgz = 1.f;
-        const IT gy = (box.interior & 2) ? (IT)(box.lo[1] + ry)
-                                         : (IT)fold_tap(b1, (long long)box.lo[1] + ry, g.d0[1], sgy);
-        const IT gz = (box.interior & 4) ? (IT)(box.lo[2] + rz)
-                                         : (IT)fold_tap(b2, (long long)box.lo[2] + rz, g.d0[2], sgz);
-        const float s = sgy * sgz;
-        const float* grow = f0 + (gz * sz + gy * sy);
-        float* srow = sm + (rz * box.Q + ry * box.P);
-        for (int ch = e4; ch < n4; ch += lpr) {
-            const long long x = (long long)box.xo + 4 * ch;
-            if (vec && x >= 0 && x + 4 <= dx) {
-                float4 v = __ldg(reinterpret_cast<const float4*>(grow + (IT)x));
-                v.x *= s;
-                v.y *= s;
-                v.z *= s;
-                v.w *= s;
-                *reinterpret_cast<float4*>(srow + 4 * ch) = v;
+    constexpr int RS = kWsCons / 8;   // rows at a time
+    const int sub = tid >> 3, l8 = tid & 7;
+    int rz = sub / ey, ry = sub - rz * ey;
+    const int sz_step = RS / ey, sy_step = RS - sz_step * ey;
+    const int fw = (int)((reinterpret_cast<uintptr_t>(f0) >> 2) & 3) + box.xo;
+    const bool fold = (box.interior & 6) != 6;
+    for (int r = sub; r < rows; r += RS) {
+        IT gy = (IT)(box.lo[1] + ry), gz = (IT)(box.lo[2] + rz);
+        if (fold) {
+            float s;
+            gy = (IT)fold_tap(b1, (long long)box.lo[1] + ry, g.d0[1], s);
+            gz = (IT)fold_tap(b2, (long long)box.lo[2] + rz, g.d0[2], s);
+        }
+        const IT ro = gz * sz + gy * sy;
+        const float* grow = f0 + ro;
+        const int si = box.base + rz * box.Q + ry * box.P;
+        const int mis = (fw + (int)(ro & 3)) & 3;
+        const bool same = (si & 3) == mis;
+        for (int e = 4 * l8 - mis; e < ex; e += 32) {
+            const int gx = box.xo + e;
+            if (same && gx >= 0 && gx + 4 <= dx) {
+                cp_async16(sm + si + e, grow + gx);
             } else {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    float sgx;
-                    const IT gx = (IT)fold_tap(b0, x + u, dx, sgx);
-                    srow[4 * ch + u] = s * sgx * __ldg(grow + gx);
+                    if (e + u < 0 || e + u >= ex) continue;
+                    float s;
+                    const IT fx = (IT)fold_tap(b0, (long long)gx + u, g.d0[0], s);
+                    cp_async4(sm + si + e + u, grow + fx);
                 }
             }
+        }
+        ry += sy_step;
+        rz += sz_step;
+        if (ry >= ey) {
+            ry -= ey;
+            ++rz;
+        }
+    }
+}
+
+// DST-II signs of a box loaded by ws_async_box (all consumer threads; the caller
+// synchronises them afterwards).
+__device__ __forceinline__ void ws_sign_box(const Box& box, const Geometry& g, int b0, int b1, int b2, float* sm,
+                                            int tid, int nthreads) {
+    const int ex = box.ext[0], ey = box.ext[1], rows = ey * box.ext[2];
+    const int lane16 = tid & 15;
+    for (int r = tid >> 4; r < rows; r += nthreads >> 4) {
+        const int rz = r / ey, ry = r - rz * ey;
+        float s1, s2;
+        (void)fold_tap(b1, (long long)box.lo[1] + ry, g.d0[1], s1);
+        (void)fold_tap(b2, (long long)box.lo[2] + rz, g.d0[2], s2);
+        float* row = sm + box.base + rz * box.Q + ry * box.P;
+        for (int e = lane16; e < ex; e += 16) {
+            float s0;
+            (void)fold_tap(b0, (long long)box.xo + e, g.d0[0], s0);
+            if (s0 * s1 * s2 < 0.f) row[e] = -row[e];
         }
     }
 }
@@ -245,8 +302,8 @@ __device__ __forceinline__ void ws_stage_gather(const Box& box, const Geometry& 
 // DST-II) onto elements inside the box itself can be loaded by the TMA window
 // like an interior box (the margins arrive zero-filled) and completed in shared
 // memory by ws_mirror_fixup.  True when the box fits the window and every
-// margin qualifies; circulant margins (whose sources lie across the image) and
-// margins wider than the in-image part take the gather instead.
+// margin qualifies; boxes with circulant margins (whose sources lie across the
+// image) or margins wider than the in-image part are loaded row by row instead.
 __device__ __forceinline__ bool ws_mirror_ok(const Box& box, const Geometry& g, int b0, int b1, int b2) {
     if (box.mode != 1 || box.ext[0] > kWsWinX || box.ext[1] > kWsWinY || box.ext[2] > kWsWinZ) return false;
     const int bk[3] = {b0, b1, b2};
@@ -346,6 +403,7 @@ __device__ __forceinline__ void ws_pull_unit(const LaunchArgs& a, const TileOrig
     // the box record in registers: the output stores would otherwise make the
     // compiler reload it from shared memory for every voxel
     const int bmode = box.mode, bxo = box.xo, by0 = box.lo[1], bz0 = box.lo[2], bP = box.P, bQ = box.Q;
+    sm += box.base;
     auto voxel = [&](int q) {
         const int lin = ctid + q * kWsCons;
         const IT v = ws_index<IT>(o, lin, D0, D1, D2);
@@ -400,7 +458,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
                                                            const __grid_constant__ CUtensorMap imgmap,
                                                            const __grid_constant__ AffineMap aff) {
     extern __shared__ __align__(128) float4 smem4[];
-    __shared__ __align__(8) unsigned long long bars[kWsStages + 2 * kWsBufs + 2];
+    __shared__ __align__(8) unsigned long long bars[kWsStages + 3 * kWsBufs + 2];
     __shared__ Box rec[kWsBufs];
     __shared__ int wrec[2][kWsCons / 32][6];   // per-warp first-tap bounds, by tile parity
     __shared__ volatile int s_abort;
@@ -417,12 +475,17 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
     const unsigned box_full = smem_addr(&bars[kWsStages]);
     const unsigned box_empty = smem_addr(&bars[kWsStages + kWsBufs]);
     const unsigned bnd_full = smem_addr(&bars[kWsStages + 2 * kWsBufs]);   // two, by tile parity
+    const unsigned rec_full = smem_addr(&bars[kWsStages + 2 * kWsBufs + 2]);   // box record published
+    // an image TMA cannot address: the consumers load every box themselves, one
+    // unit ahead, and publish their bounds two tiles ahead
+    const bool ahead = t.img_tma == 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         s_abort = 0;
         for (int k = 0; k < kWsStages; ++k) mbar_init(phi_full + 8u * k, 1);
         for (int k = 0; k < kWsBufs; ++k) {
             mbar_init(box_full + 8u * k, 1);
+            mbar_init(rec_full + 8u * k, 1);
             mbar_init(box_empty + 8u * k, kWsCons / 32);
         }
         mbar_init(bnd_full, kWsCons / 32);
@@ -434,7 +497,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
     if (warp == kWsCons / 32) {
         // ---------------- producer warp ----------------
         auto load_phi = [&](int j) {   // lane 0: tile j's deformation into slot j % kWsStages
-            if (!AFF && lane == 0) {
+            if (!AFF && t.phi_tma && lane == 0) {
                 const TileOrigin o = ws_origin(t, T0 + j * G);
                 const unsigned bar = phi_full + 8u * (j % kWsStages);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -449,7 +512,16 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
                 s_abort = 1;
                 break;
             }
-            const Box box = ws_tile_box<DP>(g, wrec[j & 1], t.img_tma != 0, lane);
+            Box box = ws_tile_box<DP>(g, wrec[j & 1], t.img_tma != 0, lane);
+            if (box.mode == 1 && !box.tma) {
+                // one mode for every channel: a box too large to be loaded row by row
+                // stays in shared memory only if all its channels take the window
+                Box rows = box;
+                ws_async_pitch(rows, g, box.lo[0], box.ext[0] - (box.lo[0] - box.xo));
+                if (rows.mode == 2 &&
+                    !(g.nbnd == 1 && t.img_tma && ws_mirror_ok(box, g, a.bnd.code[0][0], a.bnd.code[0][1], a.bnd.code[0][2])))
+                    box.mode = 2;
+            }
             for (int c = 0; c < nc; ++c) {
                 const int q = j * nc + c, b = q % kWsBufs, k = q / kWsBufs;
                 if (k >= 1 && !mbar_wait(box_empty + 8u * b, (unsigned)((k - 1) & 1))) {
@@ -461,28 +533,35 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
                 if (c == 0 && j >= 2 && j - 2 + kWsStages < ntl) load_phi(j - 2 + kWsStages);
                 // interior boxes, and boundary boxes whose margins are mirrors
                 // of their own elements (tma = 2: completed by the consumers),
-                // arrive by one TMA copy; the consumers gather all others
-                // themselves when they take the unit
+                // arrive by one TMA copy; all others are loaded row by row by the
+                // consumers (tma = 3; with DST-II margins, 4: and signed)
                 Box ub = box;
-                if (ub.mode == 1 && !ub.tma && t.img_tma) {
-                    int b0, b1, b2;
-                    bnd_code(a, c, b0, b1, b2);
-                    if (ws_mirror_ok(ub, g, b0, b1, b2)) {
+                int b0, b1, b2;
+                bnd_code(a, c, b0, b1, b2);
+                const float* f0 = a.in + ((long long)o.b * nc + c) * g.n0;
+                if (ub.mode == 1 && !ub.tma) {
+                    if (t.img_tma && ws_mirror_ok(ub, g, b0, b1, b2)) {
                         ub.tma = 2;
                         ub.P = kWsWinX;
                         ub.Q = kWsWinX * kWsWinY;
                         ub.size = kWsCap;
+                    } else {
+                        ws_async_pitch(ub, g, ub.lo[0], ub.ext[0] - (ub.lo[0] - ub.xo));
+                        ub.base = (int)(((long long)(reinterpret_cast<uintptr_t>(f0) >> 2) + ub.lo[0] +
+                                         g.d0[0] * (ub.lo[1] + g.d0[1] * (long long)ub.lo[2])) & 3);
+                        if ((b0 == 2 && !(ub.interior & 1)) || (b1 == 2 && !(ub.interior & 2)) ||
+                            (b2 == 2 && !(ub.interior & 4)))
+                            ub.tma = 4;
                     }
                 }
-                if (lane == 0) rec[b] = ub;
-                float* buf = bufs + b * kWsCap;
-                const unsigned fb = box_full + 8u * b;
-                __syncwarp();
                 if (lane == 0) {
-                    if (ub.mode == 1 && ub.tma) {
+                    rec[b] = ub;
+                    mbar_arrive(rec_full + 8u * b);
+                    const unsigned fb = box_full + 8u * b;
+                    if (ub.mode == 1 && ub.tma <= 2) {
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         mbar_expect_tx(fb, (unsigned)(kWsCap * sizeof(float)));
-                        tma_load_4d(smem_addr(buf), &imgmap, fb, ub.xo, ub.lo[1], ub.lo[2], o.b * nc + c);
+                        tma_load_4d(smem_addr(bufs + b * kWsCap), &imgmap, fb, ub.xo, ub.lo[1], ub.lo[2], o.b * nc + c);
                     } else {
                         mbar_arrive(fb);
                     }
@@ -496,10 +575,40 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
     // Each warp reduces the first-tap bounds of its voxels of tile j + 1 before
     // it evaluates tile j, so the producer can stage box j + 1 meanwhile.
     const int ctid = threadIdx.x;
-    auto publish_bounds = [&](int j) -> bool {
+    // A deformation TMA cannot address: every thread copies the words of its own
+    // voxels, one cp.async group per tile, and waits for its own groups only.
+    const bool own_phi = !AFF && !t.phi_tma;
+    auto copy_phi = [&](int j) {
+        if (j < ntl) {
+            const TileOrigin o = ws_origin(t, T0 + j * G);
+            float* slot = ring + (j % kWsStages) * 3 * kWsNV;
+            const float* phi = a.phi + (long long)o.b * 3 * g.n1;
+#pragma unroll
+            for (int q = 0; q < kWsV; ++q) {
+                const int lin = ctid + q * kWsCons;
+                const IT v = ws_index<IT>(o, lin, D0, D1, D2);
+                if (v < 0) continue;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) cp_async4(slot + k * kWsNV + lin, phi + v + k * g.n1);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (own_phi)
+        for (int j = 0; j < kWsStages; ++j) copy_phi(j);
+    // wait until at most n of this thread's latest cp.async groups are in flight
+    auto wait_groups = [&](int n) {
+        if (n == 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        else if (n == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else if (n == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else asm volatile("cp.async.wait_group 3;" ::: "memory");
+    };
+    // later_groups: groups committed after tile j's deformation (own_phi)
+    auto publish_bounds = [&](int j, int later_groups) -> bool {
         const TileOrigin o = ws_origin(t, T0 + j * G);
         const WsPos<AFF> pos{ring + (j % kWsStages) * 3 * kWsNV, &aff};
-        if (!AFF && !mbar_wait(phi_full + 8u * (j % kWsStages), (unsigned)((j / kWsStages) & 1))) return false;
+        if (own_phi) wait_groups(later_groups);
+        else if (!AFF && !mbar_wait(phi_full + 8u * (j % kWsStages), (unsigned)((j / kWsStages) & 1))) return false;
         int mn[3], mx[3];
         ws_warp_bounds<DP, IT>(g, o, pos, ctid, D0, D1, D2, mn, mx);
         if (lane == 0) {
@@ -512,27 +621,65 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
         }
         return true;
     };
-    if (!publish_bounds(0)) s_abort = 1;
+    if (!publish_bounds(0, 3)) s_abort = 1;
+    // load the rows of unit q's box (all consumers) and commit one group
+    auto load_rows = [&](int q) {
+        const int j = q / nc, c = q - j * nc;
+        const Box& box = rec[q % kWsBufs];
+        if (box.mode == 1) {
+            const TileOrigin o = ws_origin(t, T0 + j * G);
+            int b0, b1, b2;
+            bnd_code(a, c, b0, b1, b2);
+            ws_async_box<IT>(box, g, b0, b1, b2, a.in + ((long long)o.b * nc + c) * g.n0, bufs + (q % kWsBufs) * kWsCap,
+                             ctid);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (ahead) {
+        if (ntl > 1 && !publish_bounds(1, 2)) s_abort = 1;
+        if (!mbar_wait(rec_full, 0u)) s_abort = 1;
+        if (!s_abort) load_rows(0);
+    }
+    const int nq = ntl * nc;
     for (int j = 0; j < ntl && !s_abort; ++j) {
         const TileOrigin o = ws_origin(t, T0 + j * G);
         const WsPos<AFF> pos{ring + (j % kWsStages) * 3 * kWsNV, &aff};
-        if (j + 1 < ntl && !publish_bounds(j + 1)) s_abort = 1;
+        // committed after the deformation of the tile whose bounds come next: two
+        // later tiles'; ahead: the next tile's and this unit's rows
+        const int la = ahead ? 2 : 1;
+        if (j + la < ntl && !publish_bounds(j + la, 2)) s_abort = 1;
         if (s_abort) break;
         for (int c = 0; c < nc; ++c) {
             const int q = j * nc + c, b = q % kWsBufs, k = q / kWsBufs;
+            if (ahead && q + 1 < nq) {
+                const int b1 = (q + 1) % kWsBufs;
+                if (!mbar_wait(rec_full + 8u * b1, (unsigned)(((q + 1) / kWsBufs) & 1))) s_abort = 1;
+                if (s_abort) break;
+                load_rows(q + 1);
+            }
             if (!mbar_wait(box_full + 8u * b, (unsigned)(k & 1))) s_abort = 1;
             if (s_abort) break;
             const Box& box = rec[b];
             float* buf = bufs + b * kWsCap;
-            if (box.mode == 1 && box.tma != 1) {   // boundary box: all consumers complete or gather it
+            if (box.mode == 1 && box.tma >= 2) {   // all consumers load or complete the box
                 int b0, b1, b2;
                 bnd_code(a, c, b0, b1, b2);
                 if (box.tma == 2) {
                     ws_mirror_fixup(box, g, b0, b1, b2, buf, ctid, kWsCons);
                 } else {
-                    ws_stage_gather<IT>(box, g, b0, b1, b2, a.in + ((long long)o.b * nc + c) * g.n0, buf, ctid,
-                                        kWsCons);
+                    if (!ahead) {
+                        load_rows(q);
+                        wait_groups(0);
+                    } else {
+                        // this unit's rows; later: the deformation copied after the
+                        // previous tile (first channel), the next unit's rows
+                        wait_groups((q + 1 < nq ? 1 : 0) + (own_phi && c == 0 && j > 0 ? 1 : 0));
+                    }
                     asm volatile("bar.sync 1, %0;" ::"n"(kWsCons) : "memory");
+                    if (box.tma == 4) {
+                        ws_sign_box(box, g, b0, b1, b2, buf, ctid, kWsCons);
+                        asm volatile("bar.sync 1, %0;" ::"n"(kWsCons) : "memory");
+                    }
                 }
             }
             ws_pull_unit<DP, OP, IT>(a, o, ctid, pos, c, box, buf, D0, D1, D2);
@@ -540,7 +687,9 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
             if (lane == 0) mbar_arrive(box_empty + 8u * b);
         }
         if (s_abort) break;
+        if (own_phi) copy_phi(j + kWsStages);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // Tile grid of 8 x 8 x 30 tiles over the sample grid (all batches), with the
@@ -565,7 +714,9 @@ TileGrid ws_make_grid(const LaunchArgs& a) {
     magic(t.nty, t.my, t.sy);
     magic(t.ntz, t.mz, t.sz);
     t.pmod = 8;
-    t.img_tma = 0;
+    t.img_tma = t.phi_tma = 0;
+    t.nv = kWsNV;
+    t.stages = kWsStages;
     return t;
 }
 
@@ -590,17 +741,17 @@ bool encode_ws_phi_map(CUtensorMap* map, const float* base, const long long d[3]
     return r == CUDA_SUCCESS;
 }
 
-// 4-D map over an image stack (d0, d1, d2, planes) whose box is the fixed
-// kWsWin* window; false when TMA cannot address the image.
-bool encode_window_map(CUtensorMap* map, const float* base, const long long d[3], long long planes) {
+// 4-D map over an image stack (d0, d1, d2, planes) with rows of `pitch` elements
+// whose box is the fixed kWsWin* window; false when TMA cannot address the image.
+bool encode_window_map(CUtensorMap* map, const float* base, const long long d[3], long long pitch, long long planes) {
     auto fn = encode_fn();
     if (!fn) return false;
-    if ((reinterpret_cast<uintptr_t>(base) & 15) || (d[0] & 3)) return false;
+    if ((reinterpret_cast<uintptr_t>(base) & 15) || (pitch & 3)) return false;
     const cuuint64_t dims[4] = {(cuuint64_t)d[0], (cuuint64_t)d[1], (cuuint64_t)d[2], (cuuint64_t)planes};
     for (int k = 0; k < 4; ++k)
         if (dims[k] == 0 || dims[k] > (1ULL << 32)) return false;
-    const cuuint64_t strides[3] = {(cuuint64_t)d[0] * 4, (cuuint64_t)(d[0] * d[1]) * 4,
-                                   (cuuint64_t)(d[0] * d[1] * d[2]) * 4};
+    const cuuint64_t strides[3] = {(cuuint64_t)pitch * 4, (cuuint64_t)(pitch * d[1]) * 4,
+                                   (cuuint64_t)(pitch * d[1] * d[2]) * 4};
     for (int k = 0; k < 3; ++k)
         if (strides[k] >= (1ULL << 40)) return false;
     const cuuint32_t box[4] = {(cuuint32_t)kWsWinX, (cuuint32_t)kWsWinY, (cuuint32_t)kWsWinZ, 1};
@@ -611,19 +762,77 @@ bool encode_window_map(CUtensorMap* map, const float* base, const long long d[3]
     return r == CUDA_SUCCESS;
 }
 
+// Rows of n floats copied to rows of `pitch` floats (the padding stays as it is).
+__global__ void __launch_bounds__(256) k_pad_rows(const float* __restrict__ in, float* __restrict__ out, unsigned n,
+                                                  unsigned pitch, unsigned rows) {
+    const unsigned lane = threadIdx.x & 31;
+    for (unsigned r = blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8) {
+        const float* src = in + (size_t)r * n;
+        float* dst = out + (size_t)r * pitch;
+        for (unsigned x = lane; x < n; x += 32) dst[x] = __ldg(src + x);
+    }
+}
+
+// Image of a launch as TMA reads it: the caller's, or a copy with its rows padded
+// to 16 bytes when the caller's rows are not multiples of that.  The copy moves
+// 8 bytes per image voxel and channel (28 MB of image: about 10 us) and saves the
+// consumers loading every box themselves (181x217x181 cubic pull, GB300: 186 us
+// with it, 279 us without).  It is not made for images much larger than the
+// sample grid, above the scratch the library keeps, or while the stream is being
+// captured into a graph.
+struct WsImage {
+    float* copy = nullptr;
+    bool tma = false;
+};
+
+inline cudaError_t ws_image(const LaunchArgs& a, CUtensorMap* map, WsImage& im, cudaStream_t s) {
+    const Geometry& g = a.g;
+    const long long planes = (long long)g.nc * g.nb;
+    im.tma = encode_window_map(map, a.in, g.d0, g.d0[0], planes);
+    if (im.tma) return cudaSuccess;
+    const long long pitch = (g.d0[0] + 3) & ~3LL, rows = g.d0[1] * g.d0[2] * planes;
+    const long long bytes = pitch * rows * 4;
+    if (g.n0 > 4 * g.n1 || bytes > (long long)kScratchKeep / 2 || rows > 0x7fffffffLL) return cudaSuccess;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return cudaSuccess;
+    }
+    if (scratch_alloc(reinterpret_cast<void**>(&im.copy), (size_t)bytes, s) != cudaSuccess) {
+        (void)cudaGetLastError();   // no memory for the copy: the consumers load the boxes
+        im.copy = nullptr;
+        return cudaSuccess;
+    }
+    const long long want = (rows + 7) / 8, cap_grid = 16LL * sm_count();
+    k_pad_rows<<<(unsigned)(want < cap_grid ? want : cap_grid), 256, 0, s>>>(a.in, im.copy, (unsigned)g.d0[0],
+                                                                            (unsigned)pitch, (unsigned)rows);
+    const cudaError_t e = cudaGetLastError();
+    im.tma = e == cudaSuccess && encode_window_map(map, im.copy, g.d0, pitch, planes);
+    return e;
+}
+
 template <int DP, int OP, typename IT, bool AFF>
 cudaError_t launch_ws_one(const LaunchArgs& a, const TileGrid& t, const CUtensorMap& phimap, const AffineMap& aff,
                           cudaStream_t s) {
     CUtensorMap imgmap;
     std::memset(&imgmap, 0, sizeof imgmap);
     TileGrid tt = t;
-    tt.img_tma = encode_window_map(&imgmap, a.in, a.g.d0, (long long)a.g.nc * a.g.nb) ? 1 : 0;
     auto kern = k_pull_ws<DP, OP, IT, AFF>;
     cudaError_t e = opt_in(kern, kWsSmem);
     if (e != cudaSuccess) return e;
-    const int grid = tt.ntiles < sm_count() ? tt.ntiles : sm_count();
-    kern<<<grid, kWsThreads, kWsSmem, s>>>(a, tt, phimap, imgmap, aff);
-    return cudaGetLastError();
+    WsImage im;
+    e = ws_image(a, &imgmap, im, s);
+    if (e == cudaSuccess) {
+        tt.img_tma = im.tma ? 1 : 0;
+        const int grid = tt.ntiles < sm_count() ? tt.ntiles : sm_count();
+        kern<<<grid, kWsThreads, kWsSmem, s>>>(a, tt, phimap, imgmap, aff);
+        e = cudaGetLastError();
+    }
+    if (im.copy) {
+        const cudaError_t ef = cudaFreeAsync(im.copy, s);
+        if (e == cudaSuccess) e = ef;
+    }
+    return e;
 }
 
 template <int OP, typename IT, bool AFF = false>

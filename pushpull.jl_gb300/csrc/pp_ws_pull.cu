@@ -20,14 +20,12 @@ bool ws_supported(const LaunchArgs& a) {
     return ntx * nty * ntz * g.nb < 0x7fffffffLL;
 }
 
-// Warp-specialised pull family; cudaErrorNotSupported when the deformation
-// cannot be streamed by TMA (unaligned base or x extent), so the caller can
-// fall back to the other kernels.
+// Warp-specialised pull family; cudaErrorNotSupported for ops it does not take.
 cudaError_t launch_ws_pull(int op, const LaunchArgs& a, cudaStream_t s) {
-    const TileGrid t = ws_make_grid(a);
+    TileGrid t = ws_make_grid(a);
     CUtensorMap phimap;
     std::memset(&phimap, 0, sizeof phimap);
-    if (!encode_ws_phi_map(&phimap, a.phi, a.g.d1, 3LL * a.g.nb)) return cudaErrorNotSupported;
+    t.phi_tma = encode_ws_phi_map(&phimap, a.phi, a.g.d1, 3LL * a.g.nb) ? 1 : 0;
     switch (op) {
         case kPull: return ws_dispatch_op<kPull>(a, t, phimap, s);
         case kPullGrad: return ws_dispatch_op<kPullGrad>(a, t, phimap, s);
