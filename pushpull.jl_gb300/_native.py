@@ -6,6 +6,7 @@ raises.  Build it with ``__graft_entry__.build()`` or ``python pushpull.jl_gb300
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 import threading
 
@@ -94,6 +95,8 @@ def library_path() -> str:
 def lib() -> C.CDLL:
     """Load (once) the native library; raises if it has not been built."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
@@ -120,9 +123,20 @@ def check(fn: str, rc: int) -> None:
         raise PushPullError(fn, rc, msg.decode() if msg else "")
 
 
-def u64x3(v) -> "C.Array":
+# Argument arrays, built once per value (the library only reads them).
+@functools.lru_cache(maxsize=512)
+def _u64(v: tuple) -> "C.Array":
     return _u64x3(*[int(x) for x in v])
 
 
+@functools.lru_cache(maxsize=512)
+def ints(v: tuple) -> "C.Array":
+    return (C.c_int * len(v))(*[int(x) for x in v])
+
+
+def u64x3(v) -> "C.Array":
+    return _u64(tuple(v))
+
+
 def i32x3(v) -> "C.Array":
-    return _i32x3(*[int(x) for x in v])
+    return ints(tuple(v))

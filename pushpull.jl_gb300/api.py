@@ -18,46 +18,65 @@ from . import layout as L
 from .settings import Settings
 
 
+try:
+    _raw_stream = torch._C._cuda_getCurrentRawStream      # the handle alone: no Stream object per call
+except AttributeError:                                    # a torch build without CUDA, or without the accessor
+    def _raw_stream(index: int) -> int:
+        return torch.cuda.current_stream(index).cuda_stream
+
+
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _raw_stream(t.get_device())
 
 
 def _require_cuda(*ts):
     dev = None
     for t in ts:
-        if not isinstance(t, torch.Tensor) or t.device.type != "cuda":
+        if not isinstance(t, torch.Tensor) or not t.is_cuda:
             raise TypeError("pushpull_gb300 operates on CUDA tensors (no CPU path)")
-        if t.dtype != torch.float32:
+        if t.dtype is not torch.float32:
             raise TypeError("arrays must be Float32")
+        d = t.get_device()
         if dev is None:
-            dev = t.device
-        elif t.device != dev:
+            dev = d
+        elif d != dev:
             raise ValueError("all arrays must be on the same device")
-    return dev
+
+
+def _chan_batch(shape, lead: int):
+    """Channels and batch of an array whose first ``lead`` axes are something else."""
+    n = len(shape)
+    return (shape[lead] if n > lead else 1), (shape[lead + 1] if n > lead + 1 else 1)
+
+
+def _phi_shape(phi):
+    """Shape, grid and batch of a deformation."""
+    sp = phi.shape
+    assert 4 <= len(sp) <= 5, "`ϕ` must have 4 or 5 dimensions"
+    assert sp[3] == 3, "`ϕ` must have three channels"
+    return sp, sp[:3], (sp[4] if len(sp) == 5 else 1)
 
 
 def _pull_family(fn: str, f0, phi, sett: Settings, ncomp_shape, out=None):
-    assert 3 <= f0.dim() <= 5, "`f₀` must have between 3 & 5 dimensions"
-    assert 4 <= phi.dim() <= 5, "`ϕ` must have 4 or 5 dimensions"
-    assert L.jsize(phi, 4) == 3, "`ϕ` must have three channels"
-    assert L.jsize(phi, 5) == L.jsize(f0, 5), "`ϕ` & `f₀` must have the same batch size"
-    assert len(sett.bnd) == L.jsize(f0, 4) or len(sett.bnd) == 1
+    s0 = f0.shape
+    assert 3 <= len(s0) <= 5, "`f₀` must have between 3 & 5 dimensions"
+    sp, d1, nbp = _phi_shape(phi)
+    nc, nb = _chan_batch(s0, 3)
+    assert nbp == nb, "`ϕ` & `f₀` must have the same batch size"
+    assert len(sett.bnd) == nc or len(sett.bnd) == 1
     _require_cuda(f0, phi)
     f0, phi = L.colmajor(f0), L.colmajor(phi)
-    nc, nb = L.jsize(f0, 4), L.jsize(f0, 5)
-    d0 = tuple(f0.shape[:3])
-    d1 = tuple(phi.shape[:3])
-    shape = d1 + ncomp_shape + tuple(f0.shape[3:])
+    shape = d1 + ncomp_shape + s0[3:]
     if out is None:
         out = L.empty(shape, device=f0.device)
     else:
         _require_cuda(out)
-        assert tuple(out.shape) == shape and L.is_colmajor(out)
-    lib = _native.lib()
-    rc = getattr(lib, fn)(out.data_ptr(), phi.data_ptr(), f0.data_ptr(), _native.u64x3(d0),
-                          _native.u64x3(d1), nc, nb, sett.bnd_array(), sett.nbnd,
-                          _native.i32x3(sett.deg), sett.ext, _stream(f0))
-    _native.check(fn, rc)
+        assert tuple(out.shape) == tuple(shape) and L.is_colmajor(out)
+    rc = getattr(_native.lib(), fn)(out.data_ptr(), phi.data_ptr(), f0.data_ptr(), _native.u64x3(s0[:3]),
+                                    _native.u64x3(d1), nc, nb, _native.ints(sett._packed), sett.nbnd,
+                                    _native.ints(sett.deg), sett.ext, _stream(f0))
+    if rc:
+        _native.check(fn, rc)
     return out
 
 
@@ -79,39 +98,39 @@ def pull_hess(f0: torch.Tensor, phi: torch.Tensor, sett: Settings = Settings(), 
 
 
 def _push_family(fn: str, f1, phi, d0, sett: Settings, grad: bool, out=None, accumulate=False):
+    s1 = f1.shape
     if grad:
-        assert 4 <= f1.dim() <= 6, "`∇f` must have between 4 & 6 dimensions"
-        assert 4 <= phi.dim() <= 5, "`ϕ` must have 4 or 5 dimensions"
-        assert L.jsize(phi, 4) == 3, "`ϕ` must have three channels"
-        assert L.jsize(f1, 4) == 3, "`∇f` must have three components"
-        assert L.jsize(phi, 5) == L.jsize(f1, 6), "`ϕ` & `∇f` must have the same batch size"
-        assert tuple(f1.shape[:3]) == tuple(phi.shape[:3]), "`∇f` and `ϕ` must have the same volume dimensions"
-        nc, nb, lead = L.jsize(f1, 5), L.jsize(f1, 6), 4
+        assert 4 <= len(s1) <= 6, "`∇f` must have between 4 & 6 dimensions"
+        sp, d1, nbp = _phi_shape(phi)
+        assert s1[3] == 3, "`∇f` must have three components"
+        nc, nb = _chan_batch(s1, 4)
+        assert nbp == nb, "`ϕ` & `∇f` must have the same batch size"
+        assert s1[:3] == d1, "`∇f` and `ϕ` must have the same volume dimensions"
+        rest = s1[4:]
     else:
-        assert 3 <= f1.dim() <= 5, "`f₁` must have between 3 & 5 dimensions"
-        assert 4 <= phi.dim() <= 5, "`ϕ` must have 4 or 5 dimensions"
-        assert L.jsize(phi, 4) == 3, "`ϕ` must have three channels"
-        assert L.jsize(phi, 5) == L.jsize(f1, 5), "`ϕ` & `f₀` must have the same batch size"
-        assert tuple(f1.shape[:3]) == tuple(phi.shape[:3]), "`f₁` and `ϕ` must have the same volume dimensions"
-        nc, nb, lead = L.jsize(f1, 4), L.jsize(f1, 5), 3
+        assert 3 <= len(s1) <= 5, "`f₁` must have between 3 & 5 dimensions"
+        sp, d1, nbp = _phi_shape(phi)
+        nc, nb = _chan_batch(s1, 3)
+        assert nbp == nb, "`ϕ` & `f₀` must have the same batch size"
+        assert s1[:3] == d1, "`f₁` and `ϕ` must have the same volume dimensions"
+        rest = s1[3:]
     assert len(sett.bnd) == nc or len(sett.bnd) == 1
     _require_cuda(f1, phi)
     f1, phi = L.colmajor(f1), L.colmajor(phi)
     d0 = tuple(int(v) for v in d0)
     assert len(d0) == 3
-    d1 = tuple(phi.shape[:3])
-    shape = d0 + tuple(f1.shape[lead:])
+    shape = d0 + tuple(rest)
     if out is None:
         out = L.empty(shape, device=f1.device)
         accumulate = False
     else:
         _require_cuda(out)
         assert tuple(out.shape) == shape and L.is_colmajor(out)
-    lib = _native.lib()
-    rc = getattr(lib, fn)(out.data_ptr(), phi.data_ptr(), f1.data_ptr(), _native.u64x3(d0),
-                          _native.u64x3(d1), nc, nb, sett.bnd_array(), sett.nbnd,
-                          _native.i32x3(sett.deg), sett.ext, int(bool(accumulate)), _stream(f1))
-    _native.check(fn, rc)
+    rc = getattr(_native.lib(), fn)(out.data_ptr(), phi.data_ptr(), f1.data_ptr(), _native.u64x3(d0),
+                                    _native.u64x3(d1), nc, nb, _native.ints(sett._packed), sett.nbnd,
+                                    _native.ints(sett.deg), sett.ext, int(bool(accumulate)), _stream(f1))
+    if rc:
+        _native.check(fn, rc)
     return out
 
 
@@ -150,7 +169,7 @@ def push_count(f1: torch.Tensor, phi: torch.Tensor, d0, sett: Settings = Setting
         assert tuple(t.shape) == shape and L.is_colmajor(t)
     lib = _native.lib()
     rc = lib.pp_push_count(out.data_ptr(), count.data_ptr(), phi.data_ptr(), f1.data_ptr(), _native.u64x3(d0),
-                           _native.u64x3(tuple(phi.shape[:3])), nc, nb, sett.bnd_array(), sett.nbnd,
+                           _native.u64x3(tuple(phi.shape[:3])), nc, nb, _native.ints(sett._packed), sett.nbnd,
                            _native.i32x3(sett.deg), sett.ext, int(bool(accumulate)), _stream(f1))
     _native.check("pp_push_count", rc)
     return out, count
@@ -188,12 +207,12 @@ def _affine_family(push: bool, x, Aff, d_other, sett: Settings, out=None, accumu
     lib = _native.lib()
     if push:
         rc = lib.pp_push_affine(out.data_ptr(), x.data_ptr(), A, _native.u64x3(d0), _native.u64x3(d1), nc, nb,
-                                sett.bnd_array(), sett.nbnd, _native.i32x3(sett.deg), sett.ext,
+                                _native.ints(sett._packed), sett.nbnd, _native.i32x3(sett.deg), sett.ext,
                                 int(bool(accumulate)), _stream(x))
         _native.check("pp_push_affine", rc)
     else:
         rc = lib.pp_pull_affine(out.data_ptr(), x.data_ptr(), A, _native.u64x3(d0), _native.u64x3(d1), nc, nb,
-                                sett.bnd_array(), sett.nbnd, _native.i32x3(sett.deg), sett.ext, _stream(x))
+                                _native.ints(sett._packed), sett.nbnd, _native.i32x3(sett.deg), sett.ext, _stream(x))
         _native.check("pp_pull_affine", rc)
     return out
 
@@ -248,7 +267,7 @@ def _dot_family(fn: str, f0, phi, up, sett: Settings, up_comps: int):
     out = L.empty(tuple(phi.shape), device=f0.device)
     lib = _native.lib()
     rc = getattr(lib, fn)(out.data_ptr(), phi.data_ptr(), f0.data_ptr(), up.data_ptr(),
-                          _native.u64x3(f0.shape[:3]), _native.u64x3(d1), nc, nb, sett.bnd_array(), sett.nbnd,
+                          _native.u64x3(f0.shape[:3]), _native.u64x3(d1), nc, nb, _native.ints(sett._packed), sett.nbnd,
                           _native.i32x3(sett.deg), sett.ext, _stream(f0))
     _native.check(fn, rc)
     return out
@@ -293,7 +312,7 @@ def fused_step(f0: torch.Tensor, phi: torch.Tensor, g: torch.Tensor, sett: Setti
     lib = _native.lib()
     rc = lib.pp_fused_step(loss.data_ptr(), df.data_ptr(), dphi.data_ptr(), f0.data_ptr(), phi.data_ptr(),
                            g.data_ptr(), _native.u64x3(f0.shape[:3]), _native.u64x3(d1), nc, nb,
-                           sett.bnd_array(), sett.nbnd, _native.i32x3(sett.deg), sett.ext, int(bool(accumulate)),
+                           _native.ints(sett._packed), sett.nbnd, _native.i32x3(sett.deg), sett.ext, int(bool(accumulate)),
                            _stream(f0))
     _native.check("pp_fused_step", rc)
     return loss, df, dphi

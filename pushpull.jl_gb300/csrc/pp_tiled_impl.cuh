@@ -1685,15 +1685,36 @@ bool encode_box_map(CUtensorMap* map, const float* base, const long long d[3], l
     return r == CUDA_SUCCESS;
 }
 
+// Resident CTAs per SM of a kernel with `smem` bytes of dynamic shared memory,
+// asked of the runtime once per (device, kernel, size).
+template <typename K>
+cudaError_t resident_ctas(K kern, int threads, size_t smem, int* per_sm) {
+    static std::mutex mu;
+    static std::map<std::pair<std::pair<int, const void*>, size_t>, int> known;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const auto key = std::make_pair(std::make_pair(dev, reinterpret_cast<const void*>(kern)), smem);
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = known.find(key);
+    if (it == known.end()) {
+        int n = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem);
+        if (e != cudaSuccess) return e;
+        it = known.emplace(key, n < 1 ? 1 : n).first;
+    }
+    *per_sm = it->second;
+    return cudaSuccess;
+}
+
 template <typename K, typename... Args>
 cudaError_t launch_persistent(K kern, const TileGrid& t, size_t smem, cudaStream_t s, int threads,
                               const Args&... args) {
     cudaError_t e = opt_in(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+    e = resident_ctas(kern, threads, smem, &per_sm);
     if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
     const long long want = (long long)sm_count() * per_sm;
     const int grid = (int)(t.ntiles < want ? t.ntiles : want);
     kern<<<grid, threads, smem, s>>>(args...);

@@ -21,8 +21,14 @@ def colmajor_strides(shape) -> tuple:
 
 
 def is_colmajor(t: torch.Tensor) -> bool:
-    want = colmajor_strides(t.shape)
-    return all(d == 1 or st == w for d, st, w in zip(t.shape, t.stride(), want))
+    # the strides of length-1 axes do not matter; axes are walked one by one, which
+    # for the few axes of a volume is cheaper than building the strides to compare
+    w = 1
+    for d, st in zip(t.shape, t.stride()):
+        if st != w and d != 1:
+            return False
+        w *= d
+    return True
 
 
 def _rev(n: int) -> tuple:
@@ -31,7 +37,11 @@ def _rev(n: int) -> tuple:
 
 def empty(shape, device="cuda", dtype=torch.float32) -> torch.Tensor:
     shape = tuple(int(s) for s in shape)
-    return torch.empty(shape[::-1], device=device, dtype=dtype).permute(*_rev(len(shape)))
+    strides, w = [], 1
+    for d in shape:
+        strides.append(w)
+        w *= d or 1
+    return torch.empty_strided(shape, strides, device=device, dtype=dtype)
 
 
 def zeros(shape, device="cuda", dtype=torch.float32) -> torch.Tensor:
