@@ -114,6 +114,13 @@ int pp_push_grad(float *g0, const float *phi, const float *g1,
                  const int *bnd, int nbnd, const int deg[3], int ext,
                  int accumulate, void *stream);
 
+/* One step of the exponential of a velocity field: out = u o (id + u), plus id
+ * when add_id is set (src/compositions.jl:26-50), for a displacement u (d, 3):
+ * degree 1, extrapolated, component k with a DST-II boundary along axis k and
+ * DCT-II along the other two.  out and u must not overlap.  Volumes of 2^31 - 1
+ * voxels or more: PP_ERR_TOO_LARGE. */
+int pp_compose_step(float *out, const float *u, const pp_usize d[3], int add_id, void *stream);
+
 /* f0 (+)= push(f1, phi) and c0 (+)= push(1, phi) in one pass: the count image
  * holds the (signed) weight each image voxel received, from the same voxels
  * as f0 (non-finite f1 values and invalid voxels contribute to neither).

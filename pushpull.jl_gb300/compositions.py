@@ -13,9 +13,10 @@ from __future__ import annotations
 
 import torch
 
+from . import _native
 from . import layout as L
+from .api import _require_cuda, _stream, pull
 from .api import id as identity
-from .api import pull
 from .settings import Settings
 
 COMPOSE_SETTINGS = Settings(1, ((2, 1, 1), (1, 2, 1), (1, 1, 2)), True)
@@ -29,13 +30,33 @@ def compose(phi: torch.Tensor, theta: torch.Tensor, *, out=None) -> torch.Tensor
     return pull(phi, theta, COMPOSE_SETTINGS, out=out)
 
 
+def _step(u: torch.Tensor, out: torch.Tensor, last: bool) -> None:
+    """out = u ∘ (id + u), plus id for the last step of the chain."""
+    rc = _native.lib().pp_compose_step(out.data_ptr(), u.data_ptr(), _native.u64x3(u.shape[:3]), int(last), _stream(u))
+    if rc:
+        _native.check("pp_compose_step", rc)
+
+
+def _fits(dim) -> bool:
+    n = int(dim[0]) * int(dim[1]) * int(dim[2])
+    return n < 2 ** 31 - 1 and max(dim) < 2 ** 24
+
+
 def Exp(v: torch.Tensor) -> torch.Tensor:  # noqa: N802 (the reference's name)
     """Exponentiate a stationary velocity field ``v (d…, 3)`` (src/compositions.jl:42-50)."""
-    Id = identity(v)
-    u = v / float(2 ** EXP_STEPS)
-    for _ in range(EXP_STEPS):
-        u = compose(u, Id + u)
-    return u + Id
+    assert v.dim() == 4 and v.shape[3] == 3, "`ϕ` must have three channels"
+    _require_cuda(v)
+    u = L.colmajor(v / float(2 ** EXP_STEPS))
+    if not _fits(v.shape[:3]):
+        Id = identity(v)
+        for _ in range(EXP_STEPS):
+            u = compose(u, Id + u)
+        return u + Id
+    spare = L.empty(tuple(v.shape), device=v.device)
+    for k in range(EXP_STEPS):
+        _step(u, spare, k == EXP_STEPS - 1)
+        u, spare = spare, u
+    return u
 
 
 class ExpPlan:
@@ -46,9 +67,8 @@ class ExpPlan:
     def __init__(self, dim, device="cuda"):
         dim = tuple(int(d) for d in dim)
         self.v = L.zeros(dim + (3,), device=device)
-        self.Id = identity(dim=dim, device=device)
+        self.Id = None if _fits(dim) else identity(dim=dim, device=device)
         self.u = L.empty(dim + (3,), device=device)
-        self.w = L.empty(dim + (3,), device=device)
         self.t = L.empty(dim + (3,), device=device)
         self.out = L.empty(dim + (3,), device=device)
         side = torch.cuda.Stream(device=device)
@@ -62,9 +82,16 @@ class ExpPlan:
 
     def _chain(self):
         torch.mul(self.v, 1.0 / float(2 ** EXP_STEPS), out=self.u)
+        if self.Id is None:
+            u, t = self.u, self.t
+            for k in range(EXP_STEPS):
+                last = k == EXP_STEPS - 1
+                _step(u, self.out if last else t, last)
+                u, t = t, u
+            return
         for _ in range(EXP_STEPS):
-            torch.add(self.Id, self.u, out=self.w)
-            compose(self.u, self.w, out=self.t)
+            torch.add(self.Id, self.u, out=self.out)
+            compose(self.u, self.out, out=self.t)
             self.u.copy_(self.t)
         torch.add(self.u, self.Id, out=self.out)
 
