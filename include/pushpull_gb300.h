@@ -243,7 +243,7 @@ enum pp_path { PP_PATH_AUTO = 0, PP_PATH_DIRECT = 1 };
  * (3, 3, 4) selects, for pull, pull_grad and pull_hess (and through their
  * entries pull_grad_dot and pull_hess_dot), the
  * warp-specialised kernels (one producer warp streams the deformation and
- * stages footprint boxes by TMA while fifteen consumer warps evaluate 8x8x30
+ * stages footprint boxes by TMA while fifteen consumer warps evaluate 8x16x15
  * tiles; their box budget is fixed); it is the default at degrees 1..4.  No
  * reference counterpart (the reference launches one thread per voxel with no
  * tiling, ext/pushpull_gpu.jl:386-391); used by the autotuner. */

@@ -98,7 +98,7 @@ int g_path = PP_PATH_AUTO;
 bool is_push_default(const TileCfg& t) { return t.lx == 3 && t.ly == 3 && t.lz == 3 && t.cap == 16384; }
 
 // The tile code (lx, ly, lz) = (3, 3, 4) selects the warp-specialised pull
-// kernels (pp_ws.cuh, 8 x 8 x 30 tiles); every other shape the
+// kernels (pp_ws.cuh, 8 x 16 x 15 tiles); every other shape the
 // block-synchronous ones.
 bool is_ws_tile(const TileCfg& t) { return t.lx == 3 && t.ly == 3 && t.lz == 4 && t.cap > 0; }
 
@@ -224,6 +224,14 @@ int prepare_args(LaunchArgs& a, float* out, const float* phi, const float* in, c
 static bool prefer_per_voxel(const LaunchArgs& a) {
     const Geometry& g = a.g;
     if (g.dp[0] != g.dp[1] || g.dp[1] != g.dp[2] || g.n0 >= (1LL << 31) - 1) return false;
+    // a sample grid that spans a finer image: an 8 x 16 x 15 tile's footprint does not
+    // fit its buffer of 640 rows of 24 (160^3, per-voxel / warp-specialised, pull: into
+    // 192^3 quadratic 87 / 76, cubic 156 / 138, quartic 278 / 230; into 205^3 91 / 122,
+    // 171 / 182, 304 / 304; quartic pull_grad into 220^3 314 / 498)
+    const double ry = g.d1[1] > 1 ? (double)(g.d0[1] - 1) / (double)(g.d1[1] - 1) : 1.0;
+    const double rz = g.d1[2] > 1 ? (double)(g.d0[2] - 1) / (double)(g.d1[2] - 1) : 1.0;
+    const double most = g.dp[0] == 5 ? 650.0 : (g.dp[0] == 4 ? 600.0 : 575.0);
+    if ((15.0 * ry + g.dp[1] + 2.5) * (14.0 * rz + g.dp[2] + 2.5) > most) return true;
     const long long n = g.n1 * g.nb;
     const bool odd = (g.d1[0] & 3) || (reinterpret_cast<uintptr_t>(a.phi) & 15);
     bool rough = odd || (g.d0[0] & 3) || (reinterpret_cast<uintptr_t>(a.in) & 15);

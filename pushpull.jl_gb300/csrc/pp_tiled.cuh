@@ -17,7 +17,7 @@ bool tiled_supported(const LaunchArgs& a, const TileCfg& t);
 bool push_supported(const LaunchArgs& a, const TileCfg& t);
 // the push tile for a launch when the registry holds its default entry (16x8x8)
 TileCfg push_default_tile(int op, const LaunchArgs& a);
-// warp-specialised pull family (8 x 8 x 30 tiles, pp_ws.cuh): geometry test and
+// warp-specialised pull family (8 x 16 x 15 tiles, pp_ws.cuh): geometry test and
 // launch (cudaErrorNotSupported for ops or layouts it does not take)
 bool ws_supported(const LaunchArgs& a);
 cudaError_t launch_ws_pull(int op, const LaunchArgs& a, cudaStream_t s);
@@ -40,6 +40,7 @@ struct TileGrid {
     int pmod;           // box row pitch P is chosen with P % 32 == pmod
     int img_tma;        // pull: interior boxes may be loaded with one TMA copy (image tensor map valid)
     int phi_tma;        // warp-specialised pull: the deformation streams by TMA
+    int winy, winz;     // ... rows and planes of its image window
     int nv, stages;     // push: voxels per tile, ring slots
 };
 

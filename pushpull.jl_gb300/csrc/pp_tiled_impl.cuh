@@ -688,16 +688,18 @@ __device__ __forceinline__ void tile_bounds(const Geometry& g, const TileOrigin&
     tile_bounds_pos<DP, V, IT>(g, o, tv, TilePos<kThreads * V, false>{slot, nullptr, 0, 0}, mn, mx);
 }
 
-// Planes in flight in the tiled kernels: two for pull; the derivative ops, with
-// more accumulators, one (two would need more registers than 2 CTAs/SM leave).
-template <int OP>
-constexpr int kRolled = OP == kPull ? 2 : 1;
+// Planes in flight in the tiled kernels: two for pull up to four taps; the
+// derivative ops, with more accumulators, and five taps one (two would need more
+// registers than 16 warps per SM leave: quartic pull of 192^3 281 us spilling, 240
+// with one).
+template <int OP, int DP>
+constexpr int kRolled = OP == kPull && DP <= 4 ? 2 : 1;
 
 // contract_rolled over the shared box: row (k, j) starts at p + k*Q4 + j*P4.
 template <int OP, int DP, class WT>
 __device__ __forceinline__ void contract_smem(const WT& ax, const WT& ay, const WT& az, unsigned p, unsigned P4,
                                               unsigned Q4, float (&r)[6]) {
-    contract_rolled<OP, DP, kRolled<OP>>(
+    contract_rolled<OP, DP, kRolled<OP, DP>>(
         ax, ay, az, [&](int j, float (&f)[DP]) { lds_row<DP>(p + j * P4, f); }, [&]() { p += Q4; }, r);
 }
 
@@ -728,7 +730,7 @@ __device__ __forceinline__ void pull_voxel_lean(const LaunchArgs& a, int b, long
 #pragma unroll
         for (int i = 0; i < DP; ++i) zo[i] = az.off[i];
         float r[6];
-        contract_rolled<OP, DP, kRolled<OP>>(
+        contract_rolled<OP, DP, kRolled<OP, DP>>(
             ax, ay, az,
             [&](int j, float (&f)[DP]) {
 #pragma unroll
@@ -1598,7 +1600,7 @@ TileGrid make_grid(const LaunchArgs& a, const TileCfg& c) {
     magic(t.ntz, t.mz, t.sz);
     const int tx = 1 << c.lx;
     t.pmod = tx >= 32 ? 0 : tx;
-    t.img_tma = t.phi_tma = 0;
+    t.img_tma = t.phi_tma = t.winy = t.winz = 0;
     t.nv = tx << (c.ly + c.lz);
     t.stages = 0;
     return t;

@@ -6,14 +6,15 @@
 // pp_ws_hess.cu, pp_ws_grad_dot.cu and pp_ws_hess_dot.cu.
 //
 // One CTA per SM: 15 consumer warps and one producer warp (512 threads, so
-// every thread keeps 128 registers).  The CTA walks tiles of 8 x 8 x 30 sample
+// every thread keeps 128 registers).  The CTA walks tiles of 8 x 16 x 15 sample
 // voxels, four per consumer thread, in (tile, channel) units:
 //   * the producer warp streams each tile's deformation into a ring of
 //     shared-memory slots with one TMA copy per tile (mbarrier complete_tx);
 //   * every consumer warp reduces the first taps of its own voxels of tile
 //     j + 1 before it evaluates tile j and publishes the warp's bounds;
 //   * the producer combines the fifteen records into the tile's footprint box
-//     and, for a box inside the image that fits a fixed 24 x 16 x 40 window,
+//     and, for a box inside the image that fits the launch's window (24 x 24 x 26
+//     for an undeformed grid, shaped to the map for an affine one),
 //     stages it with one TMA copy into one of two buffers while the consumers
 //     still evaluate the previous unit; it then publishes the box record;
 //   * boundary boxes whose margins mirror (DCT-II, DST-II) onto elements of the
@@ -42,6 +43,8 @@
 // pull_grad and pull_hess temporaries of the rrules (src/pushpull_pb.jl:11-35).
 #pragma once
 
+#include <cmath>
+
 #include "pp_tiled_impl.cuh"
 
 namespace pp {
@@ -50,27 +53,33 @@ namespace {
 constexpr int kWsCons = 480;                   // consumer threads (15 warps)
 constexpr int kWsThreads = kWsCons + 32;       // plus the producer warp
 constexpr int kWsV = 4;                        // sample voxels per consumer thread
-constexpr int kWsTz = 30;                      // tile: 8 x 8 x 30 sample voxels
+// The tile is about as wide as it is deep, so that a rotated or strained footprint
+// still fits the window and few samples of the last tiles are lost (192^3 cubic
+// pull 156 -> 154 us, pull_grad 179 -> 175, 181x217x181 200 -> 191 against 8 x 8 x
+// 30; affine pulls with rotations up to 10 degrees 191 -> 167).
+constexpr int kWsLy = 4, kWsTy = 1 << kWsLy, kWsTz = 15;   // tile: 8 x 16 x 15 sample voxels
 constexpr int kWsNV = kWsCons * kWsV;          // 1920 voxels per tile
 constexpr int kWsStages = 4;                   // deformation ring slots
 constexpr int kWsBufs = 2;                     // box buffers
-constexpr int kWsWinX = 24, kWsWinY = 16, kWsWinZ = 40;   // TMA image window (row pitch 24)
-constexpr int kWsCap = kWsWinX * kWsWinY * kWsWinZ;         // floats per box buffer
+// TMA image window: row pitch 24 (an undeformed 8 x 4 warp tile reads 32 distinct
+// banks), t.winy rows and t.winz planes chosen per launch (ws_window)
+constexpr int kWsWinX = 24, kWsRows = 640;
+constexpr int kWsCap = kWsWinX * kWsRows;      // floats per box buffer
 constexpr size_t kWsSmem = (size_t)(kWsStages * 3 * kWsNV + kWsBufs * kWsCap) * sizeof(float);
 
 __device__ __forceinline__ void mbar_arrive(unsigned bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// Tile-local voxel lin (x fastest, 8 x 8 x 30) -> linear sample index, or -1.
+// Tile-local voxel lin (x fastest, 8 x 16 x 15) -> linear sample index, or -1.
 template <typename IT>
 __device__ __forceinline__ IT ws_index(const TileOrigin& o, int lin, int D0, int D1, int D2) {
-    const int gx = o.x0 + (lin & 7), gy = o.y0 + ((lin >> 3) & 7), gz = o.z0 + (lin >> 6);
+    const int gx = o.x0 + (lin & 7), gy = o.y0 + ((lin >> 3) & (kWsTy - 1)), gz = o.z0 + (lin >> (3 + kWsLy));
     if (gx >= D0 || gy >= D1 || gz >= D2) return (IT)-1;
     return (IT)gx + (IT)D0 * ((IT)gy + (IT)D1 * (IT)gz);
 }
 
-// Origin of linear tile T (x fastest, batch slowest) of the 8 x 8 x 30 grid.
+// Origin of linear tile T (x fastest, batch slowest) of the tile grid.
 __device__ __forceinline__ TileOrigin ws_origin(const TileGrid& t, int T) {
     const unsigned u = (unsigned)T;
     const unsigned q1 = (unsigned)(((unsigned long long)u * t.mx) >> t.sx);
@@ -78,7 +87,7 @@ __device__ __forceinline__ TileOrigin ws_origin(const TileGrid& t, int T) {
     const unsigned q3 = (unsigned)(((unsigned long long)q2 * t.mz) >> t.sz);
     TileOrigin r;
     r.x0 = (int)(u - q1 * (unsigned)t.ntx) << 3;
-    r.y0 = (int)(q1 - q2 * (unsigned)t.nty) << 3;
+    r.y0 = (int)(q1 - q2 * (unsigned)t.nty) << kWsLy;
     r.z0 = (int)(q2 - q3 * (unsigned)t.ntz) * kWsTz;
     r.b = (int)q3;
     return r;
@@ -94,8 +103,8 @@ struct WsPos {
     __device__ __forceinline__ bool operator()(const Geometry& g, const TileOrigin& o, int lin, float& x0, float& x1,
                                                float& x2) const {
         if constexpr (AFF) {
-            affine_position(*A, (float)(o.x0 + (lin & 7)), (float)(o.y0 + ((lin >> 3) & 7)), (float)(o.z0 + (lin >> 6)),
-                            x0, x1, x2);
+            affine_position(*A, (float)(o.x0 + (lin & 7)), (float)(o.y0 + ((lin >> 3) & (kWsTy - 1))),
+                            (float)(o.z0 + (lin >> (3 + kWsLy))), x0, x1, x2);
             return position_valid(x0, x1, x2, g);
         } else {
             return load_valid(slot[lin], slot[kWsNV + lin], slot[2 * kWsNV + lin], g, x0, x1, x2);
@@ -135,10 +144,9 @@ __device__ __forceinline__ void ws_warp_bounds(const Geometry& g, const TileOrig
 }
 
 // Footprint box of a tile from the consumer warps' bound records (producer
-// warp; every lane ends with the same box).  win_ok: interior boxes may use
-// the TMA window.
+// warp; every lane ends with the same box).
 template <int DP>
-__device__ __forceinline__ Box ws_tile_box(const Geometry& g, const int (*wrec)[6], bool win_ok, int lane) {
+__device__ __forceinline__ Box ws_tile_box(const Geometry& g, const TileGrid& t, const int (*wrec)[6], int lane) {
     constexpr int NW = kWsCons / 32;
     int mn[3], mx[3];
 #pragma unroll
@@ -172,11 +180,11 @@ __device__ __forceinline__ Box ws_tile_box(const Geometry& g, const int (*wrec)[
     box.lo[0] = mn[0];
     box.lo[1] = mn[1];
     box.lo[2] = mn[2];
-    if (win_ok && interior == 7 && e0 <= kWsWinX && e1 <= kWsWinY && e2 <= kWsWinZ) {
+    if (t.img_tma && interior == 7 && e0 <= kWsWinX && e1 <= t.winy && e2 <= t.winz) {
         box.mode = 1;
         box.tma = 1;
         box.P = kWsWinX;
-        box.Q = kWsWinX * kWsWinY;
+        box.Q = kWsWinX * t.winy;
         box.size = kWsCap;
         box.ext[0] = (int)e0;
         box.ext[1] = (int)e1;
@@ -304,8 +312,9 @@ __device__ __forceinline__ void ws_sign_box(const Box& box, const Geometry& g, i
 // memory by ws_mirror_fixup.  True when the box fits the window and every
 // margin qualifies; boxes with circulant margins (whose sources lie across the
 // image) or margins wider than the in-image part are loaded row by row instead.
-__device__ __forceinline__ bool ws_mirror_ok(const Box& box, const Geometry& g, int b0, int b1, int b2) {
-    if (box.mode != 1 || box.ext[0] > kWsWinX || box.ext[1] > kWsWinY || box.ext[2] > kWsWinZ) return false;
+__device__ __forceinline__ bool ws_mirror_ok(const Box& box, const Geometry& g, const TileGrid& t, int b0, int b1,
+                                             int b2) {
+    if (box.mode != 1 || box.ext[0] > kWsWinX || box.ext[1] > t.winy || box.ext[2] > t.winz) return false;
     const int bk[3] = {b0, b1, b2};
     const int lo[3] = {box.xo, box.lo[1], box.lo[2]};
 #pragma unroll
@@ -321,15 +330,15 @@ __device__ __forceinline__ bool ws_mirror_ok(const Box& box, const Geometry& g, 
     return true;
 }
 
-// Fill the margins of a TMA-loaded boundary box (row pitch kWsWinX, plane pitch
-// kWsWinX * kWsWinY) from their mirror images inside the box, x margins first
+// Fill the margins of a TMA-loaded boundary box from their mirror images inside the box, x margins first
 // (rows inside the image in y and z), then whole y-margin rows (planes inside
 // in z), then whole z-margin planes, each step reading only elements the
 // previous steps completed.  DST-II margins take the sign -1.  All consumer
 // threads; named barrier 1 between the steps and at the end.
 __device__ __forceinline__ void ws_mirror_fixup(const Box& box, const Geometry& g, int b0, int b1, int b2,
                                                 float* sm, int tid, int nthreads) {
-    constexpr int P = kWsWinX, Q = kWsWinX * kWsWinY;
+    constexpr int P = kWsWinX;
+    const int Q = box.Q;
     const int e0 = box.ext[0], e1 = box.ext[1], e2 = box.ext[2];
     const int lx = box.xo, ly = box.lo[1], lz = box.lo[2];
     const int dx = (int)g.d0[0], dy = (int)g.d0[1], dz = (int)g.d0[2];
@@ -512,14 +521,14 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
                 s_abort = 1;
                 break;
             }
-            Box box = ws_tile_box<DP>(g, wrec[j & 1], t.img_tma != 0, lane);
+            Box box = ws_tile_box<DP>(g, t, wrec[j & 1], lane);
             if (box.mode == 1 && !box.tma) {
                 // one mode for every channel: a box too large to be loaded row by row
                 // stays in shared memory only if all its channels take the window
                 Box rows = box;
                 ws_async_pitch(rows, g, box.lo[0], box.ext[0] - (box.lo[0] - box.xo));
                 if (rows.mode == 2 &&
-                    !(g.nbnd == 1 && t.img_tma && ws_mirror_ok(box, g, a.bnd.code[0][0], a.bnd.code[0][1], a.bnd.code[0][2])))
+                    !(g.nbnd == 1 && t.img_tma && ws_mirror_ok(box, g, t, a.bnd.code[0][0], a.bnd.code[0][1], a.bnd.code[0][2])))
                     box.mode = 2;
             }
             for (int c = 0; c < nc; ++c) {
@@ -540,10 +549,10 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
                 bnd_code(a, c, b0, b1, b2);
                 const float* f0 = a.in + ((long long)o.b * nc + c) * g.n0;
                 if (ub.mode == 1 && !ub.tma) {
-                    if (t.img_tma && ws_mirror_ok(ub, g, b0, b1, b2)) {
+                    if (t.img_tma && ws_mirror_ok(ub, g, t, b0, b1, b2)) {
                         ub.tma = 2;
                         ub.P = kWsWinX;
-                        ub.Q = kWsWinX * kWsWinY;
+                        ub.Q = kWsWinX * t.winy;
                         ub.size = kWsCap;
                     } else {
                         ws_async_pitch(ub, g, ub.lo[0], ub.ext[0] - (ub.lo[0] - ub.xo));
@@ -560,7 +569,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
                     const unsigned fb = box_full + 8u * b;
                     if (ub.mode == 1 && ub.tma <= 2) {
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        mbar_expect_tx(fb, (unsigned)(kWsCap * sizeof(float)));
+                        mbar_expect_tx(fb, (unsigned)(kWsWinX * t.winy * t.winz * sizeof(float)));
                         tma_load_4d(smem_addr(bufs + b * kWsCap), &imgmap, fb, ub.xo, ub.lo[1], ub.lo[2], o.b * nc + c);
                     } else {
                         mbar_arrive(fb);
@@ -692,7 +701,24 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// Tile grid of 8 x 8 x 30 tiles over the sample grid (all batches), with the
+// Rows and planes of the image window for tiles that need about ny x nz of them:
+// the whole buffer is used, rows in multiples of four (plane pitches that are
+// multiples of 32 words) when the planes still fit.  A need beyond the buffer
+// keeps the window of an undeformed tile.
+void ws_window(TileGrid& t, double ny, double nz) {
+    const int y4 = ((int)std::ceil(ny) + 3) & ~3, y1 = (int)std::ceil(ny);
+    t.winy = 24;
+    t.winz = kWsRows / 24;
+    if (!(ny >= 1.0 && nz >= 1.0 && ny <= 256.0 && nz <= 256.0)) return;
+    for (int y : {y4, y1})
+        if (y <= 256 && kWsRows / y >= nz) {
+            t.winy = y;
+            t.winz = kWsRows / y < 256 ? kWsRows / y : 256;
+            return;
+        }
+}
+
+// Tile grid of 8 x 16 x 15 tiles over the sample grid (all batches), with the
 // multiply-shift constants of ws_origin.
 TileGrid ws_make_grid(const LaunchArgs& a) {
     TileGrid t;
@@ -700,7 +726,7 @@ TileGrid ws_make_grid(const LaunchArgs& a) {
     t.ly = 3;
     t.lz = 4;   // unused here: the z side of a tile is kWsTz
     t.ntx = (int)((a.g.d1[0] + 7) >> 3);
-    t.nty = (int)((a.g.d1[1] + 7) >> 3);
+    t.nty = (int)((a.g.d1[1] + kWsTy - 1) >> kWsLy);
     t.ntz = (int)((a.g.d1[2] + kWsTz - 1) / kWsTz);
     t.cap = kWsCap;
     t.ntiles = t.ntx * t.nty * t.ntz * a.g.nb;
@@ -717,11 +743,16 @@ TileGrid ws_make_grid(const LaunchArgs& a) {
     t.img_tma = t.phi_tma = 0;
     t.nv = kWsNV;
     t.stages = kWsStages;
+    // the sample grid usually spans the image: a tile's footprint scales with their
+    // ratio, plus the taps and some displacement
+    const double ry = a.g.d1[1] > 1 ? (double)(a.g.d0[1] - 1) / (double)(a.g.d1[1] - 1) : 1.0;
+    const double rz = a.g.d1[2] > 1 ? (double)(a.g.d0[2] - 1) / (double)(a.g.d1[2] - 1) : 1.0;
+    ws_window(t, (kWsTy - 1) * ry + a.g.dp[0] + 3.5, (kWsTz - 1) * rz + a.g.dp[0] + 3.5);
     return t;
 }
 
 // 4-D map over the deformation stack (d1, 3 * nb) whose box is one tile's
-// three components (8, 8, 15, 3); false when TMA cannot address it.
+// three components (8, 16, 15, 3); false when TMA cannot address it.
 bool encode_ws_phi_map(CUtensorMap* map, const float* base, const long long d[3], long long planes) {
     EncodeFn fn = encode_fn();
     if (!fn) return false;
@@ -733,7 +764,7 @@ bool encode_ws_phi_map(CUtensorMap* map, const float* base, const long long d[3]
                                    (cuuint64_t)(d[0] * d[1] * d[2]) * 4};
     for (int k = 0; k < 3; ++k)
         if (strides[k] >= (1ULL << 40)) return false;
-    const cuuint32_t box[4] = {8, 8, (cuuint32_t)kWsTz, 3};
+    const cuuint32_t box[4] = {8, (cuuint32_t)kWsTy, (cuuint32_t)kWsTz, 3};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -742,8 +773,9 @@ bool encode_ws_phi_map(CUtensorMap* map, const float* base, const long long d[3]
 }
 
 // 4-D map over an image stack (d0, d1, d2, planes) with rows of `pitch` elements
-// whose box is the fixed kWsWin* window; false when TMA cannot address the image.
-bool encode_window_map(CUtensorMap* map, const float* base, const long long d[3], long long pitch, long long planes) {
+// whose box is the image window of t; false when TMA cannot address the image.
+bool encode_window_map(CUtensorMap* map, const float* base, const long long d[3], long long pitch, long long planes,
+                       const TileGrid& t) {
     auto fn = encode_fn();
     if (!fn) return false;
     if ((reinterpret_cast<uintptr_t>(base) & 15) || (pitch & 3)) return false;
@@ -754,7 +786,7 @@ bool encode_window_map(CUtensorMap* map, const float* base, const long long d[3]
                                    (cuuint64_t)(pitch * d[1] * d[2]) * 4};
     for (int k = 0; k < 3; ++k)
         if (strides[k] >= (1ULL << 40)) return false;
-    const cuuint32_t box[4] = {(cuuint32_t)kWsWinX, (cuuint32_t)kWsWinY, (cuuint32_t)kWsWinZ, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)kWsWinX, (cuuint32_t)t.winy, (cuuint32_t)t.winz, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -785,10 +817,10 @@ struct WsImage {
     bool tma = false;
 };
 
-inline cudaError_t ws_image(const LaunchArgs& a, CUtensorMap* map, WsImage& im, cudaStream_t s) {
+inline cudaError_t ws_image(const LaunchArgs& a, const TileGrid& t, CUtensorMap* map, WsImage& im, cudaStream_t s) {
     const Geometry& g = a.g;
     const long long planes = (long long)g.nc * g.nb;
-    im.tma = encode_window_map(map, a.in, g.d0, g.d0[0], planes);
+    im.tma = encode_window_map(map, a.in, g.d0, g.d0[0], planes, t);
     if (im.tma) return cudaSuccess;
     const long long pitch = (g.d0[0] + 3) & ~3LL, rows = g.d0[1] * g.d0[2] * planes;
     const long long bytes = pitch * rows * 4;
@@ -807,7 +839,7 @@ inline cudaError_t ws_image(const LaunchArgs& a, CUtensorMap* map, WsImage& im, 
     k_pad_rows<<<(unsigned)(want < cap_grid ? want : cap_grid), 256, 0, s>>>(a.in, im.copy, (unsigned)g.d0[0],
                                                                             (unsigned)pitch, (unsigned)rows);
     const cudaError_t e = cudaGetLastError();
-    im.tma = e == cudaSuccess && encode_window_map(map, im.copy, g.d0, pitch, planes);
+    im.tma = e == cudaSuccess && encode_window_map(map, im.copy, g.d0, pitch, planes, t);
     return e;
 }
 
@@ -821,7 +853,7 @@ cudaError_t launch_ws_one(const LaunchArgs& a, const TileGrid& t, const CUtensor
     cudaError_t e = opt_in(kern, kWsSmem);
     if (e != cudaSuccess) return e;
     WsImage im;
-    e = ws_image(a, &imgmap, im, s);
+    e = ws_image(a, t, &imgmap, im, s);
     if (e == cudaSuccess) {
         tt.img_tma = im.tma ? 1 : 0;
         const int grid = tt.ntiles < sm_count() ? tt.ntiles : sm_count();

@@ -14,9 +14,9 @@ bool ws_supported(const LaunchArgs& a) {
     const Geometry& g = a.g;
     if (!(g.dp[0] == g.dp[1] && g.dp[1] == g.dp[2])) return false;
     // most of a tile inside the sample grid (degenerate grids go per voxel)
-    if (2 * g.d1[0] < 8 || 2 * g.d1[1] < 8 || 2 * g.d1[2] < kWsTz) return false;
+    if (2 * g.d1[0] < 8 || 2 * g.d1[1] < kWsTy || 2 * g.d1[2] < kWsTz) return false;
     if (g.d1[0] > 0x7fffffffLL || g.d1[1] > 0x7fffffffLL || g.d1[2] > 0x7fffffffLL) return false;
-    const long long ntx = (g.d1[0] + 7) >> 3, nty = (g.d1[1] + 7) >> 3, ntz = (g.d1[2] + kWsTz - 1) / kWsTz;
+    const long long ntx = (g.d1[0] + 7) >> 3, nty = (g.d1[1] + kWsTy - 1) >> kWsLy, ntz = (g.d1[2] + kWsTz - 1) / kWsTz;
     return ntx * nty * ntz * g.nb < 0x7fffffffLL;
 }
 
@@ -38,7 +38,11 @@ cudaError_t launch_ws_pull(int op, const LaunchArgs& a, cudaStream_t s) {
 
 // Affine pull (pp_pull_affine) on the same kernels, positions computed in place.
 cudaError_t launch_ws_pull_affine(const LaunchArgs& a, const AffineMap& A, cudaStream_t s) {
-    const TileGrid t = ws_make_grid(a);
+    TileGrid t = ws_make_grid(a);
+    // every tile has the same footprint: the map's image of the tile, and the taps
+    const float* m = A.m;
+    ws_window(t, std::fabs(m[1]) * 7.0 + std::fabs(m[4]) * (kWsTy - 1) + std::fabs(m[7]) * (kWsTz - 1) + a.g.dp[0] + 1.01,
+              std::fabs(m[2]) * 7.0 + std::fabs(m[5]) * (kWsTy - 1) + std::fabs(m[8]) * (kWsTz - 1) + a.g.dp[0] + 1.01);
     CUtensorMap none;
     std::memset(&none, 0, sizeof none);
     const bool small = a.g.n0 < (1LL << 31) - 1 && a.g.n1 < (1LL << 31) - 1;
