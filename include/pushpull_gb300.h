@@ -154,7 +154,7 @@ int pp_fused_step(double *loss, float *df, float *dphi, const float *f0, const f
  * allocator already holds (nearly) all device memory, or whose request path
  * forbids allocation, so a library allocating scratch would fail or fragment
  * their pool.  Same arguments, results and errors as pp_fused_step; its
- * scratch is an 80 KiB array compiled into the library (every device that
+ * scratch is a 64 KiB array compiled into the library (every device that
  * loads the library keeps it until the process exits), so it calls no
  * allocator.  Limits: at most PP_NOALLOC_MAX_PARTIALS loss partials (one per
  * thread block: at most 1216 per batch element on 152 SMs) and at most

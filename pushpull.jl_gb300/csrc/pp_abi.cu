@@ -335,20 +335,12 @@ static int run_fused(double* loss, float* df, float* dphi, const float* f0, cons
         const dim3 gd = fused_direct_grid(a);
         slots = (long long)gd.x * gd.y;
     }
-    // scratch, stream ordered: per-CTA loss partials and max |f0| per (channel, batch)
-    const int planes = a.g.nc * a.g.nb;
-    const size_t part_bytes = ((size_t)slots * sizeof(double) + 255) & ~(size_t)255;
+    // scratch, stream ordered: per-CTA loss partials
     double* partial = nullptr;
-    e = scratch_alloc(reinterpret_cast<void**>(&partial), part_bytes + (size_t)planes * sizeof(unsigned), s);
+    e = scratch_alloc(reinterpret_cast<void**>(&partial), (size_t)slots * sizeof(double), s);
     if (e != cudaSuccess) return cuda_fail(e, "allocate scratch");
-    unsigned* fmax = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(partial) + part_bytes);
     a.partial = partial;
-    a.fmax = fmax;
-    if (tiled) {
-        e = cudaMemsetAsync(fmax, 0, (size_t)planes * sizeof(unsigned), s);
-        if (e == cudaSuccess) e = launch_absmax(f0, a.g.n0, planes, fmax, s);
-    }
-    if (e == cudaSuccess) e = tiled ? launch_fused_tiled(a, t, s, grid) : launch_fused_direct(a, s);
+    e = tiled ? launch_fused_tiled(a, t, s, grid) : launch_fused_direct(a, s);
     if (e == cudaSuccess) e = launch_sum_partials(partial, (int)slots, loss, s);
     const cudaError_t ef = cudaFreeAsync(partial, s);
     if (e != cudaSuccess) return cuda_fail(e, "fused step launch");

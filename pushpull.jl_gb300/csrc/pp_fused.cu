@@ -114,17 +114,6 @@ __global__ void __launch_bounds__(256) k_sum_partials(const double* p, int n, do
     if (threadIdx.x == 0) *out = red[0];
 }
 
-// max |f| per plane; non-negative floats order like their bit patterns, and a
-// NaN (whose bits exceed +inf) propagates to the maximum.
-__global__ void __launch_bounds__(256) k_absmax(const float* f, long long n, unsigned* out) {
-    const float* p = f + (long long)blockIdx.y * n;
-    unsigned m = 0;
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256)
-        m = max(m, __float_as_uint(fabsf(__ldg(p + i))));
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) atomicMax(out + blockIdx.y, m);
-}
-
 template <typename IT>
 cudaError_t launch_direct_dp(const LaunchArgs& a, dim3 grid, cudaStream_t s) {
     const int d = a.g.dp[0];
@@ -153,14 +142,6 @@ cudaError_t launch_fused_direct(const LaunchArgs& a, cudaStream_t s) {
     const bool small = a.g.n0 < (1LL << 31) - 1;
     const dim3 grid = fused_direct_grid(a);
     return small ? launch_direct_dp<int>(a, grid, s) : launch_direct_dp<long long>(a, grid, s);
-}
-
-cudaError_t launch_absmax(const float* f, long long n, int planes, unsigned* out, cudaStream_t s) {
-    if (planes > 65535) return cudaErrorInvalidConfiguration;
-    const long long blocks = (n + 255) / 256;
-    const long long cap = (long long)sm_count() * 4;
-    k_absmax<<<dim3((unsigned)(blocks < cap ? blocks : cap), (unsigned)planes), 256, 0, s>>>(f, n, out);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_sum_partials(const double* partial, int n, double* out, cudaStream_t s) {

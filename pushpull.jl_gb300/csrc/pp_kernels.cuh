@@ -31,7 +31,6 @@ struct LaunchArgs {
                         // fused step: the target g, (d1, nc, nb)
     float* out2;        // fused step: deformation cotangent (d1, 3, nb); push: count image or NULL
     double* partial;    // fused step: one loss partial per CTA
-    const unsigned* fmax;   // fused step: max |f0| per (channel, batch), float bits
     Geometry g;
     BndTable bnd;
 };
@@ -46,9 +45,6 @@ cudaError_t launch_push_direct(int op, const LaunchArgs& a, cudaStream_t s);
 dim3 fused_direct_grid(const LaunchArgs& a);
 cudaError_t launch_fused_direct(const LaunchArgs& a, cudaStream_t s);
 cudaError_t launch_sum_partials(const double* partial, int n, double* out, cudaStream_t s);
-// max |f| of each of `planes` contiguous volumes of n voxels into out[planes] (zeroed by the caller)
-cudaError_t launch_absmax(const float* f, long long n, int planes, unsigned* out, cudaStream_t s);
-
 // Stream-ordered scratch from a pool owned by this library (one per device),
 // which keeps up to kScratchKeep bytes between calls and gives back the rest;
 // freed with cudaFreeAsync.

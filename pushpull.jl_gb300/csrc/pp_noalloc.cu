@@ -1,8 +1,7 @@
 // pp_noalloc.cu -- the fused step for callers that must not allocate device memory.
 //
 // pp_fused_step needs a little scratch memory (one loss partial per thread
-// block and the largest |f0| of every (channel, batch) plane), which it takes
-// from a stream-ordered pool owned by this library.  Some callers cannot let a
+// block), which it takes from a stream-ordered pool owned by this library.  Some callers cannot let a
 // library allocate: programs whose own caching allocator has already reserved
 // (almost) all device memory, so any further allocation fails or fragments
 // their pool, and services with a fixed memory budget that forbid allocation on
@@ -27,12 +26,10 @@ int current_path();
 
 namespace {
 
-// Scratch layout: PP_NOALLOC_MAX_PARTIALS doubles, then PP_NOALLOC_MAX_PLANES
-// unsigned words.  80 KiB in all, held by every device that loads the library
-// until the process exits.
-constexpr size_t kPartialBytes = (size_t)PP_NOALLOC_MAX_PARTIALS * sizeof(double);
-constexpr size_t kScratchBytes = kPartialBytes + (size_t)PP_NOALLOC_MAX_PLANES * sizeof(unsigned);
-static_assert(kPartialBytes % 256 == 0, "plane maxima must start 256-byte aligned");
+// Scratch: PP_NOALLOC_MAX_PARTIALS doubles, 64 KiB, held by every device that loads
+// the library until the process exits.  (Calls of more than PP_NOALLOC_MAX_PLANES
+// planes, whose maxima it used to hold as well, are still refused.)
+constexpr size_t kScratchBytes = (size_t)PP_NOALLOC_MAX_PARTIALS * sizeof(double);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -141,21 +138,12 @@ extern "C" int pp_fused_step_noalloc(double* loss, float* df, float* dphi, const
         e = cudaMemsetAsync(loss, 0, sizeof(double), s);
         return e == cudaSuccess ? PP_OK : fail_status(PP_ERR_CUDA, "zero loss: %s", cudaGetErrorString(e));
     }
-    const long long planes = (long long)a.g.nc * a.g.nb;
     void* base = nullptr;
     if ((rc = scratch_address(&base)) != PP_OK) return rc;
+    // the array keeps the previous call's contents: every partial is rewritten by its block
     double* partial = static_cast<double*>(base);
-    unsigned* fmax = reinterpret_cast<unsigned*>(static_cast<unsigned char*>(base) + kPartialBytes);
     a.partial = partial;
-    a.fmax = fmax;
-    // the array keeps the previous call's contents: every partial is rewritten by
-    // its block, the plane maxima are accumulated and so start from zero
-    e = cudaSuccess;
-    if (tiled) {
-        e = cudaMemsetAsync(fmax, 0, (size_t)planes * sizeof(unsigned), s);
-        if (e == cudaSuccess) e = launch_absmax(f0, a.g.n0, (int)planes, fmax, s);
-    }
-    if (e == cudaSuccess) e = tiled ? launch_fused_tiled(a, t, s, grid) : launch_fused_direct(a, s);
+    e = tiled ? launch_fused_tiled(a, t, s, grid) : launch_fused_direct(a, s);
     if (e == cudaSuccess) e = launch_sum_partials(partial, (int)slots, loss, s);
     if (e != cudaSuccess) return fail_status(PP_ERR_CUDA, "fused step launch: %s", cudaGetErrorString(e));
     return PP_OK;

@@ -26,8 +26,8 @@
 // scatter in two passes: the upper and the lower word of a 42-bit fixed point,
 // each flushed by itself.
 //
-// Lanes: a warp covers 2^lx voxels in x and 32 / 2^lx rows.  The row pitch is
-// congruent to 2^lx modulo 32 and the plane pitch to 0, so that a first tap one
+// Lanes: a warp covers 2^lx voxels in x and 32 / 2^lx rows.  The row pitch is an odd
+// multiple of 2^lx and the plane pitch a multiple of 32, so that a first tap one
 // row or plane off its neighbours' does not change its bank: of the pitches
 // tried on a smooth +-5 voxel field, 32-wide tiles with both pitches multiples
 // of 32 gave 2.0 wavefronts per reduction, 16 x 2 lanes 2.2, 8 x 4 lanes 2.3,
@@ -136,6 +136,104 @@ struct PushBox {
     int group;          // contracted tile: kCellChannels channels at once
     int vec;            // the box has the image's 16-byte alignment
 };
+
+// Block-wide minima, maxima, sum and maximum: one record per warp, which every
+// warp combines (in the same order), so the results are uniform after one barrier.
+// bounds: the minima and maxima too.
+__device__ __forceinline__ void tile_combine(int (&wrec)[kPushThreads / 32][8], bool bounds, int (&mn)[3], int (&mx)[3],
+                                             float& ssum, float& smax) {
+    constexpr int NW = kPushThreads / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (bounds) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            mn[k] = __reduce_min_sync(0xffffffffu, mn[k]);
+            mx[k] = __reduce_max_sync(0xffffffffu, mx[k]);
+        }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, d);
+    smax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(smax)));
+    if (lane == 0) {
+        if (bounds) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                wrec[warp][k] = mn[k];
+                wrec[warp][3 + k] = mx[k];
+            }
+        }
+        wrec[warp][6] = __float_as_int(ssum);
+        wrec[warp][7] = __float_as_int(smax);
+    }
+    __syncthreads();
+    const int* r = wrec[lane & (NW - 1)];
+    if (bounds) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            mn[k] = __reduce_min_sync(0xffffffffu, r[k]);
+            mx[k] = __reduce_max_sync(0xffffffffu, r[3 + k]);
+        }
+    }
+    ssum = __int_as_float(r[6]);
+#pragma unroll
+    for (int d = NW / 2; d > 0; d >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, d);
+    smax = __uint_as_float(__reduce_max_sync(0xffffffffu, (unsigned)r[7]));
+}
+
+// Position bounds of a tile (float_key images; the first tap is monotone in the
+// position) -> the box's place and extents.  True: mode 2 is set, pitches to
+// follow; false: no valid voxel (mode 0), or coordinates the accumulator does not
+// take (mode 2).
+template <int DP>
+__device__ __forceinline__ bool box_place(int (&mn)[3], int (&mx)[3], const Geometry& g, PushBox& box) {
+    box.mode = 0;
+    box.cells = 0;
+    box.size = 0;
+    if (mn[0] > mx[0]) return false;
+    box.mode = 2;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        mn[k] = first_tap32(key_float(mn[k]), DP);
+        mx[k] = first_tap32(key_float(mx[k]), DP);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (!(mn[k] > -kFarTap && mx[k] < kFarTap && mx[k] - mn[k] < 4096)) return false;
+        box.lo[k] = mn[k];
+        box.e[k] = mx[k] - mn[k] + DP;
+    }
+    box.xin = mn[0] >= 0 && mx[0] + DP <= g.d0[0];
+    box.yin = mn[1] >= 0 && mx[1] + DP <= g.d0[1];
+    box.zin = mn[2] >= 0 && mx[2] + DP <= g.d0[2];
+    return true;
+}
+
+// Conflict-free pitches of the box when they fit `cap` words, tight ones when only
+// those do (mode 1), else mode 2.
+__device__ __forceinline__ void box_pitches(const TileGrid& t, int cap, const Geometry& g, PushBox& box) {
+    // an odd multiple of the lanes' width in x: their rows start in distinct banks
+    long long P = box.e[0] + 3;
+    P += (t.pmod - P) & (t.pmod ? 2 * t.pmod - 1 : 31);
+    long long Q = P * box.e[1];
+    Q += -Q & 31;
+    if (Q * box.e[2] + 8 > cap) {      // pack tightly when the padding does not fit
+        P = (box.e[0] + 6) & ~3;
+        Q = P * box.e[1];
+    }
+    const bool fits = Q * box.e[2] + 8 <= cap;
+    box.size = fits ? (int)((Q * box.e[2] + 7) & ~3LL) : 0;
+    box.P = fits ? (int)P : 0;
+    box.Q = fits ? (int)Q : 0;
+    box.mode = fits ? 1 : 2;
+    box.vec = fits && (g.d0[0] & 3) == 0 && ((P | Q) & 3) == 0;
+}
+
+// First word of the box in the accumulator of a channel at f0: the image's
+// 16-byte alignment where the pitches share it.
+__device__ __forceinline__ int box_base(const PushBox& box, const Geometry& g, const float* f0) {
+    const long long org = box.lo[0] + g.d0[0] * (box.lo[1] + g.d0[1] * (long long)box.lo[2]);
+    return box.vec ? (int)(((long long)(reinterpret_cast<uintptr_t>(f0) >> 2) + org) & 3) : 0;
+}
 
 // Add the accumulator box into one channel of the image and clear it.  Four
 // consecutive elements of a row that are 16-byte aligned in the image go as one
@@ -295,13 +393,21 @@ __device__ __forceinline__ void scatter_part(const WT& wx, const WT& wy, const W
     }
 }
 
+// Wait until at most n (0..3) of this thread's latest cp.async groups are in flight.
+__device__ __forceinline__ void wait_groups(int n) {
+    if (n >= 3) asm volatile("cp.async.wait_group 3;\n" ::: "memory");
+    else if (n == 2) asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+    else if (n == 1) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+
 // Fill ring slot (j mod stages) with tile T: the deformation (not AFF) and
-// NVAL value components of channel 0.  TMA: thread 0 issues one bulk tensor copy
+// NVAL components of channel 0 of `vals`.  TMA: thread 0 issues one bulk tensor copy
 // per tensor.  Otherwise every thread copies the words it will read itself with
 // 4-byte cp.async and commits one group, so no thread waits for another's.
 template <int NVAL, bool TMA, typename IT, bool AFF>
 __device__ __forceinline__ void push_ring_fill(float* base, int slot_floats, int stages, unsigned bars, int j, int T,
-                                               bool live, const LaunchArgs& a, const TileGrid& t,
+                                               bool live, const LaunchArgs& a, const float* vals, const TileGrid& t,
                                                const CUtensorMap& phimap, const CUtensorMap& valmap) {
     const int nv = t.nv, sidx = j % stages;
     constexpr int NPHI = AFF ? 0 : 3;
@@ -321,7 +427,7 @@ __device__ __forceinline__ void push_ring_fill(float* base, int slot_floats, int
             const PushTile pt(o, t, a.g);
             const long long n1 = a.g.n1;
             const float* phi = AFF ? nullptr : a.phi + (long long)o.b * 3 * n1;
-            const float* val = a.in + (long long)o.b * a.g.nc * NVAL * n1;
+            const float* val = vals + (long long)o.b * a.g.nc * NVAL * n1;
 #pragma unroll 2
             for (int lin = threadIdx.x; lin < nv; lin += kPushThreads) {
                 if (!pt.inside(lin)) continue;
@@ -335,6 +441,149 @@ __device__ __forceinline__ void push_ring_fill(float* base, int slot_floats, int
             }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+}
+
+// Scatter one channel of a tile (values at vslot, NCOMP planes of the tile's
+// voxels; ssum, smax: block-wide sum and maximum of their absolute values) into the
+// accumulator and add it to the image at f0.  The accumulator is zero before and
+// after; the caller synchronises the block before either is used again.
+template <int DP, int OP, typename IT, class POS>
+__device__ __forceinline__ void push_channel(const Geometry& g, const TileGrid& t, const PushTile& pt, const POS& pos,
+                                             const float* vslot, const PushBox& box, int b0, int b1, int b2, float* f0,
+                                             float* accf, float ssum, float smax, unsigned* wmax) {
+    constexpr int ORD = OP == kPushGrad ? 1 : 0;
+    constexpr int NCOMP = OP == kPushGrad ? 3 : 1;
+    constexpr int NW = kPushThreads / 32;
+    if (smax == 0.f) return;   // every value of this channel is zero or skipped
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nv = t.nv;
+    int* acc = reinterpret_cast<int*>(accf);
+    const int bxo = box.lo[0], by0 = box.lo[1], bz0 = box.lo[2];
+    const unsigned P4 = 4u * box.P, Q4 = 4u * box.Q;
+    const int base0 = box_base(box, g, f0);
+    const unsigned cbase = smem_addr(accf) + 4u * base0;
+    auto values = [&](int lin, float (&val)[3]) -> bool {
+        bool fin = true;
+        val[1] = val[2] = 0.f;
+#pragma unroll
+        for (int p = 0; p < NCOMP; ++p) {
+            val[p] = vslot[p * nv + lin];
+            fin = fin & finitef(val[p]);
+        }
+        return fin;
+    };
+    // every valid voxel of this thread with finite values: fn(values, weights, element address)
+    auto each = [&](auto fn) {
+#pragma unroll 1
+        for (int lin = threadIdx.x; lin < nv; lin += kPushThreads) {
+            float x0, x1, x2, val[3];
+            if (!pt.inside(lin) || !pos(g, pt, lin, x0, x1, x2) || !values(lin, val)) continue;
+            W3<DP, ORD> wx, wy, wz;
+            const int ox = spline_taps32<DP, ORD>(x0, wx.w, wx.dw, wx.hw) - bxo;
+            const int oy = spline_taps32<DP, ORD>(x1, wy.w, wy.dw, wy.hw) - by0;
+            const int oz = spline_taps32<DP, ORD>(x2, wz.w, wz.dw, wz.hw) - bz0;
+            fn(val, wx, wy, wz, cbase + 4u * (unsigned)(oz * box.Q + oy * box.P + ox));
+        }
+    };
+    const float S = NCOMP == 3 ? 2.f * ssum : ssum;   // bound on the sum of |contributions|
+    int E = scale_exponent(S);
+    bool one = false;
+    if (E != INT_MIN) {
+        // ---- bound on any element's sum --------------------------
+        int em;
+        frexpf(smax, &em);                               // smax < 2^em
+        const float hs = pow2f(20 - em);                 // |value| * weight -> at most 2^20 units
+        // branch free like the first pass: skipped voxels add 0 to the box's first words
+#pragma unroll 2
+        for (int lin = threadIdx.x; lin < nv; lin += kPushThreads) {
+            float x0, x1, x2, val[3];
+            const bool ok = pos(g, pt, lin, x0, x1, x2) & values(lin, val) & pt.inside(lin);
+            W3<DP, ORD> wx;
+            const int ox = spline_taps32<DP, ORD>(x0, wx.w, wx.dw, wx.hw) - bxo;
+            const int oy = first_tap32(x1, DP) - by0, oz = first_tap32(x2, DP) - bz0;
+            const unsigned p = ok ? cbase + 4u * (unsigned)(oz * box.Q + oy * box.P + ox) : cbase;
+            const float s0 = fabsf(val[0]) * hs, s12 = (fabsf(val[1]) + fabsf(val[2])) * hs;
+#pragma unroll
+            for (int i = 0; i < DP; ++i) {
+                float h;
+                if constexpr (OP == kPushGrad) h = fmaf(s0, fabsf(wx.dw[i]), s12 * wx.w[i]);
+                else h = s0 * wx.w[i];
+                red_s32_nb(p + 4u * i, ok ? (int)__float2uint_ru(h) : 0);
+            }
+        }
+        __syncthreads();
+        unsigned hm = 0;
+        for (int i = threadIdx.x; i < (box.size >> 2); i += kPushThreads) {
+            uint4 v = reinterpret_cast<uint4*>(accf)[i];
+            reinterpret_cast<uint4*>(accf)[i] = make_uint4(0u, 0u, 0u, 0u);
+            hm = max(max(hm, max(v.x, v.y)), max(v.z, v.w));
+        }
+        hm = __reduce_max_sync(0xffffffffu, hm);
+        if (lane == 0) wmax[warp] = hm;
+        __syncthreads();
+        hm = __reduce_max_sync(0xffffffffu, wmax[lane & (NW - 1)]);
+        constexpr float pk = peak_sum<DP, OP>();
+        const float B = __uint2float_ru(hm) * (pk * pk) * pow2f(em - 20);
+        // mean |value| per voxel, and voxels per element where the tile is denser than the grid
+        const float cnt = (float)pt.count(t);
+        const float rho = 2.f * cnt / ((float)(box.e[0] - DP + 1) * (float)(box.e[1] - DP + 1) *
+                                       (float)(box.e[2] - DP + 1));
+        if (B * cnt <= kOneWordRatio * ssum * sqrtf(fmaxf(rho, 1.f))) {
+            const int EB = scale_exponent(B);
+            if (EB != INT_MIN && EB != INT_MAX) {
+                one = true;
+                E = EB;
+            }
+        }
+    }
+    auto ld1f = [&](int w) {
+        const float v = accf[w];
+        accf[w] = 0.f;
+        return v;
+    };
+    auto ld4f = [&](int w) {
+        const float4 v = *reinterpret_cast<const float4*>(accf + w);
+        *reinterpret_cast<float4*>(accf + w) = make_float4(0.f, 0.f, 0.f, 0.f);
+        return v;
+    };
+    auto flush_words = [&](float q) {
+        push_flush<IT>(box, g, b0, b1, b2, f0, base0, [&](int w) {
+            const int4 h = *reinterpret_cast<const int4*>(acc + w);
+            *reinterpret_cast<int4*>(acc + w) = make_int4(0, 0, 0, 0);
+            return make_float4(__int2float_rn(h.x) * q, __int2float_rn(h.y) * q, __int2float_rn(h.z) * q,
+                               __int2float_rn(h.w) * q);
+        }, [&](int w) {
+            const int h = acc[w];
+            acc[w] = 0;
+            return __int2float_rn(h) * q;
+        });
+    };
+    if (one) {
+        const float sc = pow2f(32 - kWeightBits<DP> + kWordBits<DP> - E);
+        each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
+            scatter_one<DP, OP>(wx, wy, wz, val[0] * sc, val[1] * sc, val[2] * sc, p, P4, Q4);
+        });
+        __syncthreads();
+        flush_words(pow2f(E - kWordBits<DP>));
+    } else if (E != INT_MIN) {
+        const float sc = pow2f(22 - E);
+        each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
+            scatter_part<DP, OP, 0>(wx, wy, wz, val[0] * sc, val[1] * sc, val[2] * sc, p, P4, Q4);
+        });
+        __syncthreads();
+        flush_words(pow2f(E - 22));
+        __syncthreads();
+        each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
+            scatter_part<DP, OP, 1>(wx, wy, wz, val[0] * sc, val[1] * sc, val[2] * sc, p, P4, Q4);
+        });
+        __syncthreads();
+        flush_words(pow2f(E - 22) * (1.f / kLoScale));
+    } else {
+        each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
+            scatter_part<DP, OP, 2>(wx, wy, wz, val[0], val[1], val[2], p, P4, Q4);
+        });
+        __syncthreads();
+        push_flush<IT>(box, g, b0, b1, b2, f0, base0, ld4f, ld1f);
     }
 }
 
@@ -510,7 +759,6 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
                                                             const __grid_constant__ CUtensorMap valmap,
                                                             const __grid_constant__ AffineMap aff) {
     extern __shared__ __align__(128) float4 smem4[];
-    constexpr int ORD = OP == kPushGrad ? 1 : 0;
     constexpr int NCOMP = OP == kPushGrad ? 3 : 1;
     constexpr int NPHI = AFF ? 0 : 3;
     constexpr int NW = kPushThreads / 32;
@@ -543,7 +791,7 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
     }
     __syncthreads();
     for (int j = 0; j < t.stages; ++j)
-        push_ring_fill<NCOMP, TMA, IT, AFF>(ring, slot_floats, t.stages, bars, j, T0 + j * G, j < ntl, a, t, phimap,
+        push_ring_fill<NCOMP, TMA, IT, AFF>(ring, slot_floats, t.stages, bars, j, T0 + j * G, j < ntl, a, a.in, t, phimap,
                                             valmap);
 
     const unsigned acc_base = smem_addr(accf);
@@ -554,10 +802,7 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
         if constexpr (TMA) {
             if (!mbar_wait(bars + 8u * (j % t.stages), (unsigned)((j / t.stages) & 1))) s_abort = 1;
         } else {   // this thread's own copies of tile j are done; up to stages - 1 later tiles' still in flight
-            if (t.stages >= 4) asm volatile("cp.async.wait_group 3;\n" ::: "memory");
-            else if (t.stages == 3) asm volatile("cp.async.wait_group 2;\n" ::: "memory");
-            else if (t.stages == 2) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-            else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            wait_groups(t.stages - 1);
         }
         const PushTile pt(o, t, g);
         const PushPos<AFF> pos{slot, nv, &aff};
@@ -597,106 +842,37 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
                 mx[k] = float_key(hi[k]);
             }
         }
-        // one record per warp; every warp combines the eight of them
-        auto combine = [&](bool bounds) {
-            if (bounds) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    mn[k] = __reduce_min_sync(0xffffffffu, mn[k]);
-                    mx[k] = __reduce_max_sync(0xffffffffu, mx[k]);
-                }
-            }
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, d);
-            smax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(smax)));
-            if (lane == 0) {
-                if (bounds) {
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        wrec[warp][k] = mn[k];
-                        wrec[warp][3 + k] = mx[k];
-                    }
-                }
-                wrec[warp][6] = __float_as_int(ssum);
-                wrec[warp][7] = __float_as_int(smax);
-            }
-            __syncthreads();
-            const int* r = wrec[lane & (NW - 1)];
-            if (bounds) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    mn[k] = __reduce_min_sync(0xffffffffu, r[k]);
-                    mx[k] = __reduce_max_sync(0xffffffffu, r[3 + k]);
-                }
-            }
-            ssum = __int_as_float(r[6]);
-#pragma unroll
-            for (int d = NW / 2; d > 0; d >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, d);
-            smax = __uint_as_float(__reduce_max_sync(0xffffffffu, (unsigned)r[7]));
-        };
+        auto combine = [&](bool bounds) { tile_combine(wrec, bounds, mn, mx, ssum, smax); };
         combine(true);
         if (s_abort) break;
         PushBox box;
-        box.mode = 0;
-        box.cells = 0;
-        if (mn[0] <= mx[0]) {
-            bool near = true;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                mn[k] = first_tap32(key_float(mn[k]), DP);
-                mx[k] = first_tap32(key_float(mx[k]), DP);
-            }
-#pragma unroll
-            for (int k = 0; k < 3; ++k) near = near && mn[k] > -kFarTap && mx[k] < kFarTap && mx[k] - mn[k] < 4096;
-            box.mode = 2;
-            if (near) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    box.lo[k] = mn[k];
-                    box.e[k] = mx[k] - mn[k] + DP;
-                }
-                box.xin = mn[0] >= 0 && mx[0] + DP <= g.d0[0];
-                box.yin = mn[1] >= 0 && mx[1] + DP <= g.d0[1];
-                box.zin = mn[2] >= 0 && mx[2] + DP <= g.d0[2];
-                long long P = 0, Q = 0;
-                if constexpr (CELLS) {
-                    // contracted: the two-word accumulators of a channel group, the
-                    // sorted voxels, their tags and the cell starts fit the budget
-                    const long long nce = (long long)(box.e[0] - DP + 1) * (box.e[1] - DP + 1) * (box.e[2] - DP + 1);
-                    if (nce * kCellMin <= pt.count(t) && nce < 1024) {
-                        P = box.e[0] + 3;
-                        P += (4 - P) & 7;                 // odd multiples of 4, and planes 16 banks apart:
-                        Q = P * box.e[1];                 // a cell's taps fall in distinct banks
-                        Q += (16 - Q) & 31;
-                        const long long sz = (Q * box.e[2] + 7) & ~3LL;
-                        const long long rows = (kCellBatch + nce + 2) / 2;
-                        const long long fixed = kCellBatch + nce + 1;
-                        const long long one = 2 * sz + rows * (OP == kPushGrad ? 12 : 8) + fixed;
-                        const long long grp = 2 * kCellChannels * sz + rows * 12 + fixed;
-                        if (one <= t.cap) {
-                            box.cells = (int)nce;
-                            box.group = OP == kPush && g.nc > 1 && grp <= t.cap;
-                            box.size = (int)sz;
-                        }
+        if (box_place<DP>(mn, mx, g, box)) {
+            if constexpr (CELLS) {
+                // contracted: the two-word accumulators of a channel group, the
+                // sorted voxels, their tags and the cell starts fit the budget
+                const long long nce = (long long)(box.e[0] - DP + 1) * (box.e[1] - DP + 1) * (box.e[2] - DP + 1);
+                if (nce * kCellMin <= pt.count(t) && nce < 1024) {
+                    long long P = box.e[0] + 3;
+                    P += (4 - P) & 7;                 // odd multiples of 4, and planes 16 banks apart:
+                    long long Q = P * box.e[1];       // a cell's taps fall in distinct banks
+                    Q += (16 - Q) & 31;
+                    const long long sz = (Q * box.e[2] + 7) & ~3LL;
+                    const long long rows = (kCellBatch + nce + 2) / 2;
+                    const long long fixed = kCellBatch + nce + 1;
+                    const long long one = 2 * sz + rows * (OP == kPushGrad ? 12 : 8) + fixed;
+                    const long long grp = 2 * kCellChannels * sz + rows * 12 + fixed;
+                    if (one <= t.cap) {
+                        box.cells = (int)nce;
+                        box.group = OP == kPush && g.nc > 1 && grp <= t.cap;
+                        box.size = (int)sz;
+                        box.P = (int)P;
+                        box.Q = (int)Q;
+                        box.vec = (g.d0[0] & 3) == 0;
+                        box.mode = 1;
                     }
                 }
-                if (!box.cells) {
-                    P = box.e[0] + 3;
-                    P += (t.pmod - P) & 31;
-                    Q = P * box.e[1];
-                    Q += -Q & 31;
-                    if (Q * box.e[2] + 8 > t.cap) {      // pack tightly when the padding does not fit
-                        P = (box.e[0] + 6) & ~3;
-                        Q = P * box.e[1];
-                    }
-                    box.size = (int)((Q * box.e[2] + 7) & ~3LL);
-                    if (Q * box.e[2] + 8 > t.cap) box.size = 0;
-                }
-                box.vec = (g.d0[0] & 3) == 0 && ((P | Q) & 3) == 0;
-                box.P = (int)P;
-                box.Q = (int)Q;
-                if (box.size > 0) box.mode = 1;
             }
+            if (!box.cells) box_pitches(t, t.cap, g, box);
         }
         if (box.mode == 2) {
             for (int lin = threadIdx.x; lin < nv; lin += kPushThreads) {
@@ -707,11 +883,6 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
         } else if (box.mode == 1) {
             const float* inb = a.in + (long long)o.b * g.nc * NCOMP * n1;
             const int bxo = box.lo[0], by0 = box.lo[1], bz0 = box.lo[2];
-            const unsigned P4 = 4u * box.P, Q4 = 4u * box.Q;
-            const long long org = bxo + g.d0[0] * (by0 + g.d0[1] * (long long)bz0);
-            auto base_of = [&](const float* f0) {
-                return box.vec ? (int)(((long long)(reinterpret_cast<uintptr_t>(f0) >> 2) + org) & 3) : 0;
-            };
             auto cell_tile = [&](auto nval_c) {
                 constexpr int NVAL = decltype(nval_c)::value;
                 constexpr int GRP = OP == kPush ? NVAL : 1;       // channels at once
@@ -776,7 +947,7 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
                     int base0[GRP];
 #pragma unroll
                     for (int q = 0; q < GRP; ++q)
-                        base0[q] = base_of(a.out + ((long long)o.b * g.nc + min(cg + q, g.nc - 1)) * g.n0);
+                        base0[q] = box_base(box, g, a.out + ((long long)o.b * g.nc + min(cg + q, g.nc - 1)) * g.n0);
                     for (int l0 = 0; l0 < nv; l0 += kCellBatch) {
                         const int nb = min(kCellBatch, nv - l0);
                         for (int i = threadIdx.x; i <= nce; i += kPushThreads) ca.start[i] = 0;
@@ -935,140 +1106,14 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
                     __syncthreads();   // the previous channel's flush and record reads are done
                     combine(false);
                 }
-                if (smax == 0.f) continue;   // every value of this channel is zero or skipped
-                // weights and first taps of the voxel at `off`; false: skip
-                float* f0 = a.out + ((long long)o.b * g.nc + c) * g.n0;
-                const int base0 = base_of(f0);
-                const unsigned cbase = acc_base + 4u * base0;
-                auto values = [&](int lin, float (&val)[3]) -> bool {
-                    bool fin = true;
-                    val[1] = val[2] = 0.f;
-#pragma unroll
-                    for (int p = 0; p < NCOMP; ++p) {
-                        val[p] = vslot[p * nv + lin];
-                        fin = fin & finitef(val[p]);
-                    }
-                    return fin;
-                };
-                // every valid voxel of this thread with finite values: fn(values, weights, element address)
-                auto each = [&](auto fn) {
-#pragma unroll 1
-                    for (int lin = threadIdx.x; lin < nv; lin += kPushThreads) {
-                        float x0, x1, x2, val[3];
-                        if (!pt.inside(lin) || !pos(g, pt, lin, x0, x1, x2) || !values(lin, val)) continue;
-                        W3<DP, ORD> wx, wy, wz;
-                        const int ox = spline_taps32<DP, ORD>(x0, wx.w, wx.dw, wx.hw) - bxo;
-                        const int oy = spline_taps32<DP, ORD>(x1, wy.w, wy.dw, wy.hw) - by0;
-                        const int oz = spline_taps32<DP, ORD>(x2, wz.w, wz.dw, wz.hw) - bz0;
-                        fn(val, wx, wy, wz, cbase + 4u * (unsigned)(oz * box.Q + oy * box.P + ox));
-                    }
-                };
-                const float S = NCOMP == 3 ? 2.f * ssum : ssum;   // bound on the sum of |contributions|
-                int E = scale_exponent(S);
-                bool one = false;
-                if (E != INT_MIN) {
-                    // ---- bound on any element's sum --------------------------
-                    int em;
-                    frexpf(smax, &em);                               // smax < 2^em
-                    const float hs = pow2f(20 - em);                 // |value| * weight -> at most 2^20 units
-                    // branch free like the first pass: skipped voxels add 0 to the box's first words
-#pragma unroll 2
-                    for (int lin = threadIdx.x; lin < nv; lin += kPushThreads) {
-                        float x0, x1, x2, val[3];
-                        const bool ok = pos(g, pt, lin, x0, x1, x2) & values(lin, val) & pt.inside(lin);
-                        W3<DP, ORD> wx;
-                        const int ox = spline_taps32<DP, ORD>(x0, wx.w, wx.dw, wx.hw) - bxo;
-                        const int oy = first_tap32(x1, DP) - by0, oz = first_tap32(x2, DP) - bz0;
-                        const unsigned p = ok ? cbase + 4u * (unsigned)(oz * box.Q + oy * box.P + ox) : cbase;
-                        const float s0 = fabsf(val[0]) * hs, s12 = (fabsf(val[1]) + fabsf(val[2])) * hs;
-#pragma unroll
-                        for (int i = 0; i < DP; ++i) {
-                            float h;
-                            if constexpr (OP == kPushGrad) h = fmaf(s0, fabsf(wx.dw[i]), s12 * wx.w[i]);
-                            else h = s0 * wx.w[i];
-                            red_s32_nb(p + 4u * i, ok ? (int)__float2uint_ru(h) : 0);
-                        }
-                    }
-                    __syncthreads();
-                    unsigned hm = 0;
-                    for (int i = threadIdx.x; i < (box.size >> 2); i += kPushThreads) {
-                        uint4 v = reinterpret_cast<uint4*>(accf)[i];
-                        reinterpret_cast<uint4*>(accf)[i] = make_uint4(0u, 0u, 0u, 0u);
-                        hm = max(max(hm, max(v.x, v.y)), max(v.z, v.w));
-                    }
-                    hm = __reduce_max_sync(0xffffffffu, hm);
-                    if (lane == 0) wmax[warp] = hm;
-                    __syncthreads();
-                    hm = __reduce_max_sync(0xffffffffu, wmax[lane & (NW - 1)]);
-                    constexpr float pk = peak_sum<DP, OP>();
-                    const float B = __uint2float_ru(hm) * (pk * pk) * pow2f(em - 20);
-                    // mean |value| per voxel, and voxels per element where the tile is denser than the grid
-                    const float cnt = (float)pt.count(t);
-                    const float rho = 2.f * cnt / ((float)(box.e[0] - DP + 1) * (float)(box.e[1] - DP + 1) *
-                                                   (float)(box.e[2] - DP + 1));
-                    if (B * cnt <= kOneWordRatio * ssum * sqrtf(fmaxf(rho, 1.f))) {
-                        const int EB = scale_exponent(B);
-                        if (EB != INT_MIN && EB != INT_MAX) {
-                            one = true;
-                            E = EB;
-                        }
-                    }
-                }
-                auto ld1f = [&](int w) {
-                    const float v = accf[w];
-                    accf[w] = 0.f;
-                    return v;
-                };
-                auto ld4f = [&](int w) {
-                    const float4 v = *reinterpret_cast<const float4*>(accf + w);
-                    *reinterpret_cast<float4*>(accf + w) = make_float4(0.f, 0.f, 0.f, 0.f);
-                    return v;
-                };
-                auto flush_words = [&](float q) {
-                    push_flush<IT>(box, g, b0, b1, b2, f0, base0, [&](int w) {
-                        const int4 h = *reinterpret_cast<const int4*>(acc + w);
-                        *reinterpret_cast<int4*>(acc + w) = make_int4(0, 0, 0, 0);
-                        return make_float4(__int2float_rn(h.x) * q, __int2float_rn(h.y) * q, __int2float_rn(h.z) * q,
-                                           __int2float_rn(h.w) * q);
-                    }, [&](int w) {
-                        const int h = acc[w];
-                        acc[w] = 0;
-                        return __int2float_rn(h) * q;
-                    });
-                };
-                if (one) {
-                    const float sc = pow2f(32 - kWeightBits<DP> + kWordBits<DP> - E);
-                    each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
-                        scatter_one<DP, OP>(wx, wy, wz, val[0] * sc, val[1] * sc, val[2] * sc, p, P4, Q4);
-                    });
-                    __syncthreads();
-                    flush_words(pow2f(E - kWordBits<DP>));
-                } else if (E != INT_MIN) {
-                    const float sc = pow2f(22 - E);
-                    each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
-                        scatter_part<DP, OP, 0>(wx, wy, wz, val[0] * sc, val[1] * sc, val[2] * sc, p, P4, Q4);
-                    });
-                    __syncthreads();
-                    flush_words(pow2f(E - 22));
-                    __syncthreads();
-                    each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
-                        scatter_part<DP, OP, 1>(wx, wy, wz, val[0] * sc, val[1] * sc, val[2] * sc, p, P4, Q4);
-                    });
-                    __syncthreads();
-                    flush_words(pow2f(E - 22) * (1.f / kLoScale));
-                } else {
-                    each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
-                        scatter_part<DP, OP, 2>(wx, wy, wz, val[0], val[1], val[2], p, P4, Q4);
-                    });
-                    __syncthreads();
-                    push_flush<IT>(box, g, b0, b1, b2, f0, base0, ld4f, ld1f);
-                }
+                push_channel<DP, OP, IT>(g, t, pt, pos, vslot, box, b0, b1, b2,
+                                         a.out + ((long long)o.b * g.nc + c) * g.n0, accf, ssum, smax, wmax);
             }
         }
         if (TMA && g.nc > 1) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();   // ring slot j is free and the accumulator is clear
         push_ring_fill<NCOMP, TMA, IT, AFF>(ring, slot_floats, t.stages, bars, j + t.stages, T0 + (j + t.stages) * G,
-                                            j + t.stages < ntl, a, t, phimap, valmap);
+                                            j + t.stages < ntl, a, a.in, t, phimap, valmap);
     }
     if constexpr (!TMA) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }

@@ -1,8 +1,15 @@
 // pp_tiled_fused.cu -- tiled fused forward + adjoint step kernels
-// (kernels and helpers: pp_tiled_impl.cuh).
-#include "pp_tiled_impl.cuh"
+// (pp_fused.cuh).
+#include "pp_fused.cuh"
 
 namespace pp {
+
+int fused_tiled_grid(const LaunchArgs& a, const TileCfg& c) {
+    size_t smem;
+    int ctas;
+    (void)fused_grid(a, c, smem, ctas);
+    return ctas;
+}
 
 cudaError_t launch_fused_tiled(const LaunchArgs& a, const TileCfg& t, cudaStream_t s, int grid) {
     const bool small = a.g.n0 < (1LL << 31) - 1 && a.g.n1 < (1LL << 31) - 1;

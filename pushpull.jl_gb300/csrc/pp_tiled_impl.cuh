@@ -356,6 +356,86 @@ __device__ __forceinline__ void stage_box(const Box& box, const Geometry& g, int
     });
 }
 
+// A footprint box as row loaders see it: origin in the image, extents, pitches, first
+// word, and whether rows fold (in y or z).
+struct RowBox {
+    int lo[3], e[3], P, Q, base;
+    bool fold;
+};
+
+// NT threads load one channel of a box row by row with cp.async, eight lanes to a
+// row, folding rows and elements outside the image onto their sources (no signs:
+// see sign_rows).  The caller commits and waits.  Rows that have the same 16-byte
+// alignment in the image and in the box copy whole chunks (three words lie between
+// rows: a row's first and last chunk may overwrite them); chunks at the image's x
+// ends, and rows whose alignment differs, copy elements.
+template <int NT, typename IT>
+__device__ __forceinline__ void load_rows(const RowBox& box, const Geometry& g, int b0, int b1, int b2, const float* f0,
+                                          float* sm, int tid) {
+    const int ex = box.e[0], ey = box.e[1], rows = ey * box.e[2], dx = (int)g.d0[0];
+    const IT sy = (IT)g.d0[0];
+    const IT sz = (IT)(g.d0[0] * g.d0[1]);
+    constexpr int RS = NT / 8;   // rows at a time
+    const int sub = tid >> 3, l8 = tid & 7;
+    int rz = sub / ey, ry = sub - rz * ey;
+    const int sz_step = RS / ey, sy_step = RS - sz_step * ey;
+    const int fw = (int)((reinterpret_cast<uintptr_t>(f0) >> 2) & 3) + box.lo[0];
+    for (int r = sub; r < rows; r += RS) {
+        IT gy = (IT)(box.lo[1] + ry), gz = (IT)(box.lo[2] + rz);
+        if (box.fold) {
+            float s;
+            gy = (IT)fold_tap(b1, (long long)box.lo[1] + ry, g.d0[1], s);
+            gz = (IT)fold_tap(b2, (long long)box.lo[2] + rz, g.d0[2], s);
+        }
+        const IT ro = gz * sz + gy * sy;
+        const float* grow = f0 + ro;
+        const int si = box.base + rz * box.Q + ry * box.P;
+        const int mis = (fw + (int)(ro & 3)) & 3;
+        const bool same = (si & 3) == mis;
+        for (int e = 4 * l8 - mis; e < ex; e += 32) {
+            const int gx = box.lo[0] + e;
+            if (same && gx >= 0 && gx + 4 <= dx) {
+                cp_async16(sm + si + e, grow + gx);
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (e + u < 0 || e + u >= ex) continue;
+                    float s;
+                    const IT fx = (IT)fold_tap(b0, (long long)gx + u, g.d0[0], s);
+                    cp_async4(sm + si + e + u, grow + fx);
+                }
+            }
+        }
+        ry += sy_step;
+        rz += sz_step;
+        if (ry >= ey) {
+            ry -= ey;
+            ++rz;
+        }
+    }
+}
+
+// DST-II signs of a box loaded by load_rows (all NT threads; the caller
+// synchronises them before and afterwards).
+template <int NT>
+__device__ __forceinline__ void sign_rows(const RowBox& box, const Geometry& g, int b0, int b1, int b2, float* sm,
+                                          int tid) {
+    const int ex = box.e[0], ey = box.e[1], rows = ey * box.e[2];
+    const int lane16 = tid & 15;
+    for (int r = tid >> 4; r < rows; r += NT >> 4) {
+        const int rz = r / ey, ry = r - rz * ey;
+        float s1, s2;
+        (void)fold_tap(b1, (long long)box.lo[1] + ry, g.d0[1], s1);
+        (void)fold_tap(b2, (long long)box.lo[2] + rz, g.d0[2], s2);
+        float* row = sm + box.base + rz * box.Q + ry * box.P;
+        for (int e = lane16; e < ex; e += 16) {
+            float s0;
+            (void)fold_tap(b0, (long long)box.lo[0] + e, g.d0[0], s0);
+            if (s0 * s1 * s2 < 0.f) row[e] = -row[e];
+        }
+    }
+}
+
 // ---- push accumulation -----------------------------------------------------
 // Each box element holds two int32 words (hi, lo) of a fixed-point sum.  With
 // S >= the sum of |contribution| over the tile's channel (B-spline weights are
@@ -1076,279 +1156,6 @@ __device__ __forceinline__ void red_f32_nb(unsigned a, float v) {
     asm volatile("red.shared.add.f32 [%0], %1;" ::"r"(a), "f"(v));
 }
 
-// ---- fused forward + adjoint step ------------------------------------------
-//
-// loss = sum_{b,c,v} (pull(f_c, phi)[v] - g_c[v])^2, df = push(2 r), and
-// dphi[v] = sum_c 2 r_c grad pull(f_c)[v]: the forward pull, the pull rrule's
-// two cotangents (src/pushpull_pb.jl:11-18) and the loss of the differentiable
-// step in one pass.  The image box is staged once per (tile, channel) and serves
-// both the value and the gradient; delta = 2 r is scattered into the shared
-// accumulator of the same box and flushed with global reductions.
-
-// Per-voxel global-memory version of one channel (tiles whose box does not fit):
-// returns the residual r and the gradient; scatters 2 r into df with atomics.
-// Inlined, with the rolled contraction and a rolled z loop in the scatter, so
-// that the fallback costs the tiled kernel no registers.
-template <int DP, typename IT>
-__device__ __forceinline__ float fused_voxel_global(const LaunchArgs& a, int b, int c, long long v, float x0,
-                                                    float x1, float x2, float gv, float (&grad)[3]) {
-    const Geometry& g = a.g;
-    const IT sy = (IT)g.d0[0];
-    const IT sz = (IT)(g.d0[0] * g.d0[1]);
-    int b0, b1, b2;
-    bnd_code(a, c, b0, b1, b2);
-    Axis<DP, 1, IT> ax, ay, az;
-    ax.setup(x0, g.dp[0], b0, g.d0[0], (IT)1);
-    ay.setup(x1, g.dp[1], b1, g.d0[1], sy);
-    az.setup(x2, g.dp[2], b2, g.d0[2], sz);
-    const float* f0 = a.in + ((long long)b * g.nc + c) * g.n0;
-    IT zo[DP];
-#pragma unroll
-    for (int i = 0; i < DP; ++i) zo[i] = az.off[i];
-    float r[6];
-    contract_rolled<kPullValGrad, DP, 1>(
-        ax, ay, az,
-        [&](int j, float (&f)[DP]) {
-#pragma unroll
-            for (int i = 0; i < DP; ++i) f[i] = __ldg(f0 + (zo[0] + ay.off[j] + ax.off[i]));
-        },
-        [&]() {
-#pragma unroll
-            for (int i = 0; i + 1 < DP; ++i) zo[i] = zo[i + 1];
-        },
-        r);
-    grad[0] = r[0];
-    grad[1] = r[1];
-    grad[2] = r[2];
-    const float res = r[3] - gv;
-    const float d = 2.f * res;
-    if (finitef(d)) {
-        float* df = a.out + ((long long)b * g.nc + c) * g.n0;
-#pragma unroll 1
-        for (int k = 0; k < DP; ++k) {
-#pragma unroll
-            for (int j = 0; j < DP; ++j) {
-                const float cb = d * (ay.w[j] * az.w[0]);
-#pragma unroll
-                for (int i = 0; i < DP; ++i) atomicAdd(df + (az.off[0] + ay.off[j] + ax.off[i]), cb * ax.w[i]);
-            }
-#pragma unroll
-            for (int i = 0; i + 1 < DP; ++i) {
-                az.w[i] = az.w[i + 1];
-                az.off[i] = az.off[i + 1];
-            }
-        }
-    }
-    return res;
-}
-
-template <int DP, int V, typename IT, bool TMA>
-__global__ void __launch_bounds__(kThreads, DP <= 3 ? 3 : 2) k_fused_tiled(const __grid_constant__ LaunchArgs a,
-                                                             const __grid_constant__ TileGrid t,
-                                                             const __grid_constant__ CUtensorMap phimap,
-                                                             const __grid_constant__ CUtensorMap gmap) {
-    extern __shared__ __align__(128) float4 smem4[];
-    constexpr int NV = kThreads * V;
-    __shared__ int red[8][7];
-    __shared__ float sred[8];
-    __shared__ double dred[8];
-    __shared__ Box boxm[2];
-    __shared__ int s_abort;
-    const Geometry& g = a.g;
-    const long long n1 = g.n1;
-    const int G = gridDim.x;
-    const int T0 = blockIdx.x;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ntl = T0 < t.ntiles ? (t.ntiles - T0 + G - 1) / G : 0;
-    const ThreadVox<V> tv(t, g);
-    double loss = 0.0;
-
-    float* sm = reinterpret_cast<float*>(smem4);
-    Ring ring;
-    ring.base = sm;
-    ring.slot_floats = 4 * NV;                       // deformation + channel-0 target
-    float* bufs = sm + kStages * 4 * NV;              // image box, double buffered
-    float* accf = bufs + 2 * t.cap;                   // adjoint accumulator: 2 words per element
-    ring.bars = smem_addr(accf + 2 * t.cap);
-    for (int i = threadIdx.x; i < (2 * t.cap) >> 2; i += kThreads)
-        reinterpret_cast<float4*>(accf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (threadIdx.x == 0) {
-        s_abort = 0;
-        if (TMA) {
-            for (int k = 0; k < kStages; ++k) mbar_init(ring.bars + 8u * k, 1);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-    }
-    __syncthreads();
-    for (int j = 0; j < kStages && j < ntl; ++j)
-        ring_fill<V, 1, TMA, IT>(ring, j, T0 + j * G, a, t, tv, phimap, gmap, a.up);
-    if (!TMA) __syncthreads();
-
-    // Box of tile j and the channel-0 scale bound: |r| <= max|f| + |g| because the
-    // B-spline weights are non-negative and sum to one, so the sum of |2 r w|
-    // over a voxel's taps is at most 2 (max|f| + |g|).
-    auto prepare = [&](int j) {
-        const TileOrigin o = tile_origin(t, T0 + j * G);
-        const float* slot = ring.base + (j % kStages) * ring.slot_floats;
-        if (!ring_wait<TMA>(ring, j)) s_abort = 1;
-        int mn[3], mx[3];
-        tile_bounds<DP, V, IT>(g, o, tv, slot, mn, mx);
-        const float M = __uint_as_float(a.fmax[(long long)o.b * g.nc]);
-        float bound = 0.f;
-#pragma unroll
-        for (int q = 0; q < V; ++q) {
-            const int lin = threadIdx.x + q * kThreads;
-            float x0, x1, x2;
-            if (tv.template index<IT>(o, q) >= 0 &&
-                load_valid(slot[lin], slot[NV + lin], slot[2 * NV + lin], g, x0, x1, x2))
-                bound += 2.f * (M + fabsf(slot[3 * NV + lin]));
-        }
-        reduce_box<DP>(mn, mx, t, g, 1, boxm[j & 1], red, bound);
-        if (boxm[j & 1].mode == 1) {
-            int b0, b1, b2;
-            bnd_code(a, 0, b0, b1, b2);
-            stage_box<IT>(boxm[j & 1], g, b0, b1, b2, a.in + (long long)o.b * g.nc * g.n0, bufs + (j & 1) * t.cap);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-
-    if (ntl > 0) prepare(0);
-    const unsigned acc_base = smem_addr(accf);
-    int* acc_hi = reinterpret_cast<int*>(accf);
-    for (int j = 0; j < ntl; ++j) {
-        if (j + 1 < ntl) {
-            prepare(j + 1);
-            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        }
-        __syncthreads();   // box j is in its buffer
-        if (s_abort) break;
-        const TileOrigin o = tile_origin(t, T0 + j * G);
-        const float* slot = ring.base + (j % kStages) * ring.slot_floats;
-        const Box& box = boxm[j & 1];
-        float* buf = bufs + (j & 1) * t.cap;
-        const unsigned lo_off = 4u * (unsigned)box.size;
-        int* acc_lo = acc_hi + box.size;
-        float dphi[V][3];
-        unsigned valid = 0;
-#pragma unroll
-        for (int q = 0; q < V; ++q) dphi[q][0] = dphi[q][1] = dphi[q][2] = 0.f;
-        for (int c = 0; c < g.nc; ++c) {
-            int b0, b1, b2;
-            bnd_code(a, c, b0, b1, b2);
-            const float* gc = a.up + ((long long)o.b * g.nc + c) * n1;
-            int E = box.E;
-            if (c > 0) {
-                __syncthreads();   // channel c-1 is done with the box and the accumulator
-                if (box.mode == 1) {
-                    stage_box<IT>(box, g, b0, b1, b2, a.in + ((long long)o.b * g.nc + c) * g.n0, buf);
-                    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-                }
-                const float M = __uint_as_float(a.fmax[(long long)o.b * g.nc + c]);
-                float bound = 0.f;
-#pragma unroll
-                for (int q = 0; q < V; ++q) {
-                    const IT v = tv.template index<IT>(o, q);
-                    if (v >= 0 && (valid >> q & 1)) bound += 2.f * (M + fabsf(__ldg(gc + v)));
-                }
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) bound += __shfl_xor_sync(0xffffffffu, bound, off);
-                if (lane == 0) sred[warp] = bound;
-                __syncthreads();   // the box of channel c and every warp's bound are in
-                float S = 0.f;
-                for (int w = 0; w < kThreads / 32; ++w) S += sred[w];
-                E = scale_exponent(S);
-            }
-            const bool fixed = E != INT_MIN && E != INT_MAX;
-            FixedScale fs;
-            fs.set(fixed ? E : 0);
-#pragma unroll
-            for (int q = 0; q < V; ++q) {
-                const IT v = tv.template index<IT>(o, q);
-                if (v < 0) continue;
-                const int lin = threadIdx.x + q * kThreads;
-                float x0, x1, x2;
-                if (!load_valid(slot[lin], slot[NV + lin], slot[2 * NV + lin], g, x0, x1, x2)) {
-                    loss += (double)qnan();   // pull is NaN here, and so is the loss
-                    continue;
-                }
-                valid |= 1u << q;
-                const float gv = c == 0 ? slot[3 * NV + lin] : __ldg(gc + v);
-                float res, grad[3];
-                if (box.mode == 1) {
-                    W3<DP, 1> wx, wy, wz;
-                    const int ox = spline_taps32<DP, 1>(x0, wx.w, wx.dw, wx.hw) - box.xo;
-                    const int oy = spline_taps32<DP, 1>(x1, wy.w, wy.dw, wy.hw) - box.lo[1];
-                    const int oz = spline_taps32<DP, 1>(x2, wz.w, wz.dw, wz.hw) - box.lo[2];
-                    const unsigned P4 = 4u * box.P, Q4 = 4u * box.Q;
-                    const unsigned off = 4u * (unsigned)(oz * box.Q + oy * box.P + ox);
-                    const unsigned p = smem_addr(buf) + off;
-                    float r[6];
-                    contract_smem<kPullValGrad, DP>(wx, wy, wz, p, P4, Q4, r);
-                    res = r[3] - gv;
-                    grad[0] = r[0];
-                    grad[1] = r[1];
-                    grad[2] = r[2];
-                    const float d = 2.f * res;
-                    if (finitef(d) && E != INT_MAX) {
-                        if (fixed)
-                            push_scatter<DP, kPush, true>(wx, wy, wz, d * fs.inv_q1, 0.f, 0.f, acc_base + off, P4, Q4,
-                                                          lo_off);
-                        else
-                            push_scatter<DP, kPush, false>(wx, wy, wz, d, 0.f, 0.f, acc_base + off, P4, Q4, lo_off);
-                    }
-                } else {
-                    res = fused_voxel_global<DP, IT>(a, o.b, c, (long long)v, x0, x1, x2, gv, grad);
-                }
-                loss += (double)(res * res);
-                const float d = 2.f * res;
-                dphi[q][0] = fmaf(d, grad[0], dphi[q][0]);
-                dphi[q][1] = fmaf(d, grad[1], dphi[q][1]);
-                dphi[q][2] = fmaf(d, grad[2], dphi[q][2]);
-            }
-            __syncthreads();   // the scatter is complete
-            if (box.mode == 1 && E != INT_MAX) {
-                float* df = a.out + ((long long)o.b * g.nc + c) * g.n0;
-                if (fixed)
-                    flush_fixed<IT>(box, g, b0, b1, b2, df, acc_hi, acc_lo, fs);
-                else
-                    flush_box<IT>(box, g, b0, b1, b2, df, [&](int si) {
-                        const float v = accf[si];
-                        accf[si] = 0.f;
-                        return v;
-                    });
-            }
-        }
-        // deformation cotangent of every sample voxel of the tile
-        float* dp = a.out2 + (long long)o.b * 3 * n1;
-#pragma unroll
-        for (int q = 0; q < V; ++q) {
-            const IT v = tv.template index<IT>(o, q);
-            if (v < 0) continue;
-            const bool ok = valid >> q & 1;
-            dp[v] = ok ? dphi[q][0] : qnan();
-            dp[v + n1] = ok ? dphi[q][1] : qnan();
-            dp[v + 2 * n1] = ok ? dphi[q][2] : qnan();
-        }
-        __syncthreads();   // ring slot j, the box buffer and the accumulator are free
-        if (j + kStages < ntl)
-            ring_fill<V, 1, TMA, IT>(ring, j + kStages, T0 + (j + kStages) * G, a, t, tv, phimap, gmap, a.up);
-        if (!TMA) __syncthreads();
-    }
-    // this CTA's loss partial
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
-    if (lane == 0) dred[warp] = loss;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double sum = 0.0;
-        for (int w = 0; w < kThreads / 32; ++w) sum += dred[w];
-        a.partial[blockIdx.x] = sum;
-    }
-}
-
-
 #ifdef PP_TILED_BATCH
 // ---- batched uneven workload ------------------------------------------------
 //
@@ -1739,36 +1546,6 @@ cudaError_t launch_v(const LaunchArgs& a, const TileGrid& t, cudaStream_t s) {
     const size_t smem = (size_t)kStages * 3 * NV * 4 + 2 * (size_t)t.cap * 4 + 8 * kStages + 16;
     if (tma) return launch_persistent(k_pull_tiled<DP, OP, V, IT, true>, tt, smem, s, kThreads, a, tt, phimap, imgmap);
     return launch_persistent(k_pull_tiled<DP, OP, V, IT, false>, tt, smem, s, kThreads, a, tt, phimap, imgmap);
-}
-
-template <int DP, int V, typename IT>
-cudaError_t launch_fused_v(const LaunchArgs& a, const TileGrid& t, cudaStream_t s, int grid) {
-    constexpr int NV = kThreads * V;
-    CUtensorMap phimap, gmap;
-    std::memset(&phimap, 0, sizeof phimap);
-    std::memset(&gmap, 0, sizeof gmap);
-    const long long nb = a.g.nb, nc = a.g.nc;
-    const bool tma = encode_tile_map(&phimap, a.phi, a.g.d1, 3 * nb, t, 3) &&
-                     encode_tile_map(&gmap, a.up, a.g.d1, nc * nb, t, 1);
-    const size_t smem = (size_t)kStages * 4 * NV * 4 + 4 * (size_t)t.cap * 4 + 8 * kStages;
-    cudaError_t e;
-    if (tma) {
-        auto k = k_fused_tiled<DP, V, IT, true>;
-        if ((e = opt_in(k, smem)) != cudaSuccess) return e;
-        k<<<grid, kThreads, smem, s>>>(a, t, phimap, gmap);
-    } else {
-        auto k = k_fused_tiled<DP, V, IT, false>;
-        if ((e = opt_in(k, smem)) != cudaSuccess) return e;
-        k<<<grid, kThreads, smem, s>>>(a, t, phimap, gmap);
-    }
-    return cudaGetLastError();
-}
-
-template <int DP, typename IT>
-cudaError_t launch_fused_dp(const LaunchArgs& a, const TileCfg& c, cudaStream_t s, int grid) {
-    const TileGrid t = make_grid(a, c);
-    if ((1 << (c.lx + c.ly + c.lz)) > kThreads) return launch_fused_v<DP, 2, IT>(a, t, s, grid);
-    return launch_fused_v<DP, 1, IT>(a, t, s, grid);
 }
 
 template <int DP, int OP, typename IT>

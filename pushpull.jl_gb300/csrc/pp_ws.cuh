@@ -203,7 +203,11 @@ __device__ __forceinline__ Box ws_tile_box(const Geometry& g, const TileGrid& t,
     return box;
 }
 
-// Pitches of a box that is loaded row by row (ws_async_box): congruent
+__device__ __forceinline__ RowBox box_rows(const Box& b) {
+    return RowBox{{b.xo, b.lo[1], b.lo[2]}, {b.ext[0], b.ext[1], b.ext[2]}, b.P, b.Q, b.base, (b.interior & 6) != 6};
+}
+
+// Pitches of a box that is loaded row by row (load_rows): congruent
 // to the image's row and plane modulo 4 elements, so that 16-byte chunks of a row
 // are aligned in both; the row pitch 8 or 24 modulo 32 (plus that remainder)
 // keeps an 8 x 4 warp tile's rows in nearly disjoint banks.  Three words lie
@@ -231,79 +235,6 @@ __device__ __forceinline__ void ws_async_pitch(Box& box, const Geometry& g, int 
     box.Q = fits ? (int)Q : 0;
     box.size = fits ? (int)(Q * e2) : 0;
     box.tma = 3;
-}
-
-// All consumer threads load one channel of a box row by row with cp.async,
-// eight lanes to a row, folding rows and elements outside the image onto their
-// sources (no signs: see ws_sign_box).  The caller commits and waits.
-// Rows that have the same 16-byte alignment in the image and in the box copy
-// whole chunks; chunks at the image's x ends, and rows whose source lies
-// elsewhere in an image of odd extents, copy elements.
-template <typename IT>
-__device__ __forceinline__ void ws_async_box(const Box& box, const Geometry& g, int b0, int b1, int b2,
-                                             const float* f0, float* sm, int tid) {
-    const int ex = box.ext[0], ey = box.ext[1], rows = ey * box.ext[2], dx = (int)g.d0[0];
-    const IT sy = (IT)g.d0[0];
-    const IT sz = (IT)(g.d0[0] * g.d0[1]);
-    constexpr int RS = kWsCons / 8;   // rows at a time
-    const int sub = tid >> 3, l8 = tid & 7;
-    int rz = sub / ey, ry = sub - rz * ey;
-    const int sz_step = RS / ey, sy_step = RS - sz_step * ey;
-    const int fw = (int)((reinterpret_cast<uintptr_t>(f0) >> 2) & 3) + box.xo;
-    const bool fold = (box.interior & 6) != 6;
-    for (int r = sub; r < rows; r += RS) {
-        IT gy = (IT)(box.lo[1] + ry), gz = (IT)(box.lo[2] + rz);
-        if (fold) {
-            float s;
-            gy = (IT)fold_tap(b1, (long long)box.lo[1] + ry, g.d0[1], s);
-            gz = (IT)fold_tap(b2, (long long)box.lo[2] + rz, g.d0[2], s);
-        }
-        const IT ro = gz * sz + gy * sy;
-        const float* grow = f0 + ro;
-        const int si = box.base + rz * box.Q + ry * box.P;
-        const int mis = (fw + (int)(ro & 3)) & 3;
-        const bool same = (si & 3) == mis;
-        for (int e = 4 * l8 - mis; e < ex; e += 32) {
-            const int gx = box.xo + e;
-            if (same && gx >= 0 && gx + 4 <= dx) {
-                cp_async16(sm + si + e, grow + gx);
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (e + u < 0 || e + u >= ex) continue;
-                    float s;
-                    const IT fx = (IT)fold_tap(b0, (long long)gx + u, g.d0[0], s);
-                    cp_async4(sm + si + e + u, grow + fx);
-                }
-            }
-        }
-        ry += sy_step;
-        rz += sz_step;
-        if (ry >= ey) {
-            ry -= ey;
-            ++rz;
-        }
-    }
-}
-
-// DST-II signs of a box loaded by ws_async_box (all consumer threads; the caller
-// synchronises them afterwards).
-__device__ __forceinline__ void ws_sign_box(const Box& box, const Geometry& g, int b0, int b1, int b2, float* sm,
-                                            int tid, int nthreads) {
-    const int ex = box.ext[0], ey = box.ext[1], rows = ey * box.ext[2];
-    const int lane16 = tid & 15;
-    for (int r = tid >> 4; r < rows; r += nthreads >> 4) {
-        const int rz = r / ey, ry = r - rz * ey;
-        float s1, s2;
-        (void)fold_tap(b1, (long long)box.lo[1] + ry, g.d0[1], s1);
-        (void)fold_tap(b2, (long long)box.lo[2] + rz, g.d0[2], s2);
-        float* row = sm + box.base + rz * box.Q + ry * box.P;
-        for (int e = lane16; e < ex; e += 16) {
-            float s0;
-            (void)fold_tap(b0, (long long)box.xo + e, g.d0[0], s0);
-            if (s0 * s1 * s2 < 0.f) row[e] = -row[e];
-        }
-    }
 }
 
 // A boundary box whose out-of-image margins all fold by a mirror (DCT-II or
@@ -632,22 +563,22 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
     };
     if (!publish_bounds(0, 3)) s_abort = 1;
     // load the rows of unit q's box (all consumers) and commit one group
-    auto load_rows = [&](int q) {
+    auto load_unit = [&](int q) {
         const int j = q / nc, c = q - j * nc;
         const Box& box = rec[q % kWsBufs];
         if (box.mode == 1) {
             const TileOrigin o = ws_origin(t, T0 + j * G);
             int b0, b1, b2;
             bnd_code(a, c, b0, b1, b2);
-            ws_async_box<IT>(box, g, b0, b1, b2, a.in + ((long long)o.b * nc + c) * g.n0, bufs + (q % kWsBufs) * kWsCap,
-                             ctid);
+            load_rows<kWsCons, IT>(box_rows(box), g, b0, b1, b2, a.in + ((long long)o.b * nc + c) * g.n0,
+                                   bufs + (q % kWsBufs) * kWsCap, ctid);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     if (ahead) {
         if (ntl > 1 && !publish_bounds(1, 2)) s_abort = 1;
         if (!mbar_wait(rec_full, 0u)) s_abort = 1;
-        if (!s_abort) load_rows(0);
+        if (!s_abort) load_unit(0);
     }
     const int nq = ntl * nc;
     for (int j = 0; j < ntl && !s_abort; ++j) {
@@ -664,7 +595,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
                 const int b1 = (q + 1) % kWsBufs;
                 if (!mbar_wait(rec_full + 8u * b1, (unsigned)(((q + 1) / kWsBufs) & 1))) s_abort = 1;
                 if (s_abort) break;
-                load_rows(q + 1);
+                load_unit(q + 1);
             }
             if (!mbar_wait(box_full + 8u * b, (unsigned)(k & 1))) s_abort = 1;
             if (s_abort) break;
@@ -677,7 +608,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
                     ws_mirror_fixup(box, g, b0, b1, b2, buf, ctid, kWsCons);
                 } else {
                     if (!ahead) {
-                        load_rows(q);
+                        load_unit(q);
                         wait_groups(0);
                     } else {
                         // this unit's rows; later: the deformation copied after the
@@ -686,7 +617,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
                     }
                     asm volatile("bar.sync 1, %0;" ::"n"(kWsCons) : "memory");
                     if (box.tma == 4) {
-                        ws_sign_box(box, g, b0, b1, b2, buf, ctid, kWsCons);
+                        sign_rows<kWsCons>(box_rows(box), g, b0, b1, b2, buf, ctid);
                         asm volatile("bar.sync 1, %0;" ::"n"(kWsCons) : "memory");
                     }
                 }
