@@ -43,14 +43,6 @@ __device__ __forceinline__ bool finitef(float v) { return fabsf(v) <= 3.40282346
 // Explicit shared-memory accesses through 32-bit shared-window addresses, so
 // box reads and reductions are always issued as shared-space instructions.
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ float lds_f32(unsigned a) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ void red_shared_s32(unsigned a, int v) {
-    asm volatile("red.shared.add.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
 __device__ __forceinline__ void red_shared_f32(unsigned a, float v) {
     asm volatile("red.shared.add.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }

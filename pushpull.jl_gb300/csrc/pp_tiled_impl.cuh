@@ -142,14 +142,6 @@ struct Box {
     int E;          // scale exponent of the fixed-point accumulator for S (see scale_exponent)
 };
 
-__device__ __forceinline__ int clamp_tap(long long o) {
-    return (int)(o < -kClamp ? -kClamp : (o > kClamp ? kClamp : o));
-}
-
-__device__ __forceinline__ int first_tap_i(float x, int DP) {
-    return clamp_tap((long long)ceilf(__fsub_rn(x, 0.5f * (float)DP)));
-}
-
 // Exponent E of the fixed-point accumulator scale for a bound S on the sum of
 // |contributions|: S < 2^E.  INT_MAX: nothing to accumulate (S == 0);
 // INT_MIN: S non-finite or outside the range the scale factors cover, so the
@@ -504,52 +496,6 @@ __device__ __forceinline__ void flush_box(const Box& box, const Geometry& g, int
     });
 }
 
-// Flush (and clear) a two-word fixed-point accumulator box into the image.
-// Rows of an x-interior box of an aligned image go as 16-byte groups: both
-// words of 4 elements in two 16-byte loads, cleared by two 16-byte stores, one
-// 4-wide global reduction (all-zero groups skipped).  Other boxes: the
-// element-wise walk.
-template <typename IT>
-__device__ __forceinline__ void flush_fixed(const Box& box, const Geometry& g, int b0, int b1, int b2, float* f0,
-                                            int* acc_hi, int* acc_lo, const FixedScale& fs) {
-    const bool vec = (box.interior & 1) && (g.d0[0] & 3) == 0 && (reinterpret_cast<uintptr_t>(f0) & 15) == 0 &&
-                     ((box.P | box.Q | box.size) & 3) == 0;
-    if (!vec) {
-        flush_box<IT>(box, g, b0, b1, b2, f0, [&](int si) {
-            const float v = fixed_value(acc_hi[si], acc_lo[si], fs);
-            acc_hi[si] = 0;
-            acc_lo[si] = 0;
-            return v;
-        });
-        return;
-    }
-    const int ey = box.ext[1], ez = box.ext[2];
-    const int n4 = (box.ext[0] + 3) >> 2;
-    RowWalk<> rw(n4, ey);
-    if (rw.e0 >= n4) return;   // lanes per row >= n4: at most one group of each row per thread
-    const IT sy = (IT)g.d0[0];
-    const IT sz = (IT)(g.d0[0] * g.d0[1]);
-    const int e = 4 * rw.e0;
-    for (; rw.rz < ez; rw.next()) {
-        const int rz = rw.rz, ry = rw.ry;
-        const int si = rz * box.Q + ry * box.P + e;
-        const int4 h = *reinterpret_cast<const int4*>(acc_hi + si);
-        const int4 l = *reinterpret_cast<const int4*>(acc_lo + si);
-        *reinterpret_cast<int4*>(acc_hi + si) = make_int4(0, 0, 0, 0);
-        *reinterpret_cast<int4*>(acc_lo + si) = make_int4(0, 0, 0, 0);
-        if ((h.x | h.y | h.z | h.w | l.x | l.y | l.z | l.w) == 0) continue;
-        float sgy = 1.f, sgz = 1.f;
-        const IT gy = (box.interior & 2) ? (IT)(box.lo[1] + ry)
-                                         : (IT)fold_tap(b1, (long long)box.lo[1] + ry, g.d0[1], sgy);
-        const IT gz = (box.interior & 4) ? (IT)(box.lo[2] + rz)
-                                         : (IT)fold_tap(b2, (long long)box.lo[2] + rz, g.d0[2], sgz);
-        const float sg = sgy * sgz;
-        const float4 v = make_float4(sg * fixed_value(h.x, l.x, fs), sg * fixed_value(h.y, l.y, fs),
-                                     sg * fixed_value(h.z, l.z, fs), sg * fixed_value(h.w, l.w, fs));
-        atomicAdd(reinterpret_cast<float4*>(f0 + (gz * sz + gy * sy + (IT)box.xo) + e), v);
-    }
-}
-
 // ---- tiles -----------------------------------------------------------------
 struct TileOrigin {
     int b;            // batch
@@ -612,7 +558,7 @@ __device__ __noinline__ void push_tile_fallback(const LaunchArgs& a, int b, long
     push_voxel_global<DP, OP, IT>(a, b, v, x0, x1, x2);
 }
 
-// ---- tile ring: per-tile deformation (and push values) several tiles ahead ----
+// ---- tile ring: per-tile deformation several tiles ahead ----
 //
 // Slot k of the ring holds one tile laid out as [component][z][y][x] -- exactly
 // the order of a 4-D TMA box (TX, TY, TZ, C) -- so the thread owning tile-local
@@ -670,14 +616,10 @@ struct Ring {
     unsigned bars;     // shared address of the first mbarrier
 };
 
-// Fill ring slot (j % kStages) with tile T: deformation components 0..2 and
-// NVAL value components of channel 0 of `vals` (layout (d1, NVAL, nc, nb); the
-// push input, or the fused step's target).  Called by every thread.  AFF (the
-// affine ops): the values only, the deformation part of the slot stays unused.
-template <int V, int NVAL, bool TMA, typename IT, bool AFF = false>
+// Fill ring slot (j % kStages) with the deformation of tile T.  Called by every thread.
+template <int V, bool TMA, typename IT>
 __device__ __forceinline__ void ring_fill(const Ring& r, int j, int T, const LaunchArgs& a, const TileGrid& t,
-                                          const ThreadVox<V>& tv, const CUtensorMap& phimap,
-                                          const CUtensorMap& valmap, const float* vals) {
+                                          const ThreadVox<V>& tv, const CUtensorMap& phimap) {
     constexpr int NV = kThreads * V;
     float* slot = r.base + (j % kStages) * r.slot_floats;
     const TileOrigin o = tile_origin(t, T);
@@ -685,25 +627,18 @@ __device__ __forceinline__ void ring_fill(const Ring& r, int j, int T, const Lau
         if (threadIdx.x == 0) {
             const unsigned bar = r.bars + 8u * (j % kStages);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_expect_tx(bar, (unsigned)(((AFF ? 0 : 3) + NVAL) * NV * sizeof(float)));
-            if constexpr (!AFF) tma_load_4d(smem_addr(slot), &phimap, bar, o.x0, o.y0, o.z0, 3 * o.b);
-            if constexpr (NVAL > 0)
-                tma_load_4d(smem_addr(slot + 3 * NV), &valmap, bar, o.x0, o.y0, o.z0, NVAL * a.g.nc * o.b);
+            mbar_expect_tx(bar, (unsigned)(3 * NV * sizeof(float)));
+            tma_load_4d(smem_addr(slot), &phimap, bar, o.x0, o.y0, o.z0, 3 * o.b);
         }
     } else {
         const long long n1 = a.g.n1;
-        const float* phi = AFF ? nullptr : a.phi + (long long)o.b * 3 * n1;
-        const float* val = vals + (long long)o.b * a.g.nc * NVAL * n1;
+        const float* phi = a.phi + (long long)o.b * 3 * n1;
 #pragma unroll
         for (int q = 0; q < V; ++q) {
             const int lin = threadIdx.x + q * kThreads;
             const IT v = tv.template index<IT>(o, q);
-            if constexpr (!AFF) {
 #pragma unroll
-                for (int k = 0; k < 3; ++k) slot[k * NV + lin] = v < 0 ? 0.f : __ldg(phi + v + k * n1);
-            }
-#pragma unroll
-            for (int k = 0; k < NVAL; ++k) slot[(3 + k) * NV + lin] = v < 0 ? 0.f : __ldg(val + v + k * n1);
+            for (int k = 0; k < 3; ++k) slot[k * NV + lin] = v < 0 ? 0.f : __ldg(phi + v + k * n1);
         }
     }
 }
@@ -714,32 +649,12 @@ __device__ __forceinline__ bool ring_wait(const Ring& r, int j) {
     return true;
 }
 
-// Sample positions of a tile's voxels: x = phi - 1 from the tile's ring slot,
-// or (AFF, the affine ops) A * (i, j, k, 1) from the voxel's grid coordinates;
-// either way with the validity test.
-template <int NV, bool AFF>
-struct TilePos {
-    const float* slot;
-    const AffineMap* A;
-    int lx, ly;
-    __device__ __forceinline__ bool operator()(const Geometry& g, const TileOrigin& o, int lin, float& x0, float& x1,
-                                               float& x2) const {
-        if constexpr (AFF) {
-            const int gx = o.x0 + (lin & ((1 << lx) - 1));
-            const int gy = o.y0 + ((lin >> lx) & ((1 << ly) - 1));
-            const int gz = o.z0 + (lin >> (lx + ly));
-            affine_position(*A, (float)gx, (float)gy, (float)gz, x0, x1, x2);
-            return position_valid(x0, x1, x2, g);
-        } else {
-            return load_valid(slot[lin], slot[NV + lin], slot[2 * NV + lin], g, x0, x1, x2);
-        }
-    }
-};
-
-// First-tap bounds of this thread's valid voxels of a tile.
-template <int DP, int V, typename IT, class POS>
-__device__ __forceinline__ void tile_bounds_pos(const Geometry& g, const TileOrigin& o, const ThreadVox<V>& tv,
-                                                const POS& pos, int (&mn)[3], int (&mx)[3]) {
+// First-tap bounds of this thread's valid voxels of the tile whose deformation is in
+// `slot`.
+template <int DP, int V, typename IT>
+__device__ __forceinline__ void tile_bounds(const Geometry& g, const TileOrigin& o, const ThreadVox<V>& tv,
+                                            const float* slot, int (&mn)[3], int (&mx)[3]) {
+    constexpr int NV = kThreads * V;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         mn[k] = INT_MAX;
@@ -750,7 +665,7 @@ __device__ __forceinline__ void tile_bounds_pos(const Geometry& g, const TileOri
         const int lin = threadIdx.x + q * kThreads;
         if (tv.template index<IT>(o, q) < 0) continue;
         float x[3];
-        if (!pos(g, o, lin, x[0], x[1], x[2])) continue;
+        if (!load_valid(slot[lin], slot[NV + lin], slot[2 * NV + lin], g, x[0], x[1], x[2])) continue;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const int f = first_tap32(x[k], DP);
@@ -759,13 +674,6 @@ __device__ __forceinline__ void tile_bounds_pos(const Geometry& g, const TileOri
             mx[k] = max(mx[k], c);
         }
     }
-}
-
-// ... of the tile whose deformation is in `slot`.
-template <int DP, int V, typename IT>
-__device__ __forceinline__ void tile_bounds(const Geometry& g, const TileOrigin& o, const ThreadVox<V>& tv,
-                                            const float* slot, int (&mn)[3], int (&mx)[3]) {
-    tile_bounds_pos<DP, V, IT>(g, o, tv, TilePos<kThreads * V, false>{slot, nullptr, 0, 0}, mn, mx);
 }
 
 // Planes in flight in the tiled kernels: two for pull up to four taps; the
@@ -989,7 +897,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pull_tiled(const __grid_constan
     }
     __syncthreads();
     for (int j = 0; j < kStages && j < ntl; ++j)
-        ring_fill<V, 0, TMA, IT>(ring, j, T0 + j * G, a, t, tv, phimap, phimap, a.in);
+        ring_fill<V, TMA, IT>(ring, j, T0 + j * G, a, t, tv, phimap);
     if (!TMA) __syncthreads();
 
     // one TMA copy of channel c's fixed image window into buffer `buf` (thread 0)
@@ -1047,7 +955,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pull_tiled(const __grid_constan
             pull_tile_global<DP, OP, V, IT>(a, o, tv, t, slot);
             __syncthreads();   // ring slot j is free
             if (j + kStages < ntl)
-                ring_fill<V, 0, TMA, IT>(ring, j + kStages, T0 + (j + kStages) * G, a, t, tv, phimap, phimap, a.in);
+                ring_fill<V, TMA, IT>(ring, j + kStages, T0 + (j + kStages) * G, a, t, tv, phimap);
             if (!TMA) __syncthreads();
             continue;
         }
@@ -1075,7 +983,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pull_tiled(const __grid_constan
         if (s_abort) break;
         __syncthreads();   // ring slot j and buffer j & 1 are free
         if (j + kStages < ntl)
-            ring_fill<V, 0, TMA, IT>(ring, j + kStages, T0 + (j + kStages) * G, a, t, tv, phimap, phimap, a.in);
+            ring_fill<V, TMA, IT>(ring, j + kStages, T0 + (j + kStages) * G, a, t, tv, phimap);
         if (!TMA) __syncthreads();
     }
 }
