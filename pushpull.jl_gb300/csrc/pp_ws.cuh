@@ -774,6 +774,30 @@ inline cudaError_t ws_image(const LaunchArgs& a, const TileGrid& t, CUtensorMap*
     return e;
 }
 
+// CTAs of a launch (CTA c takes tiles c, c + G, ...).  Where G and the tiles along x
+// share a factor, a CTA meets the same few x positions again and again, and the tiles
+// at the border of the image, whose boxes do not arrive by TMA alone, all fall on some
+// of the CTAs.  So a G without a common factor, unless it takes one more round of
+// tiles.  GB300, 152 SMs, cubic pull: 192^3 152 CTAs 152 us, 151 142; bounds (0, 1, 2)
+// 175 / 146; 160x192x160 quadratic, bounds (0, 1, 2) 87 / 78.  (The push kernels gain
+// too, 192^3 228 / 224 us, but a contracted 256^3 x 3 loses, 1584 / 1623: they keep
+// all their CTAs.)
+inline int ws_grid(const TileGrid& t) {
+    const int want = sm_count();
+    if (t.ntiles < 2 * want) return t.ntiles < want ? t.ntiles : want;
+    const int rounds = (t.ntiles + want - 1) / want;
+    for (int g = want; g > want - 8 && g > 1 && (t.ntiles + g - 1) / g == rounds; --g) {
+        int x = g, y = t.ntx;
+        while (y) {
+            const int r = x % y;
+            x = y;
+            y = r;
+        }
+        if (x == 1) return g;
+    }
+    return want;
+}
+
 template <int DP, int OP, typename IT, bool AFF>
 cudaError_t launch_ws_one(const LaunchArgs& a, const TileGrid& t, const CUtensorMap& phimap, const AffineMap& aff,
                           cudaStream_t s) {
@@ -787,8 +811,7 @@ cudaError_t launch_ws_one(const LaunchArgs& a, const TileGrid& t, const CUtensor
     e = ws_image(a, t, &imgmap, im, s);
     if (e == cudaSuccess) {
         tt.img_tma = im.tma ? 1 : 0;
-        const int grid = tt.ntiles < sm_count() ? tt.ntiles : sm_count();
-        kern<<<grid, kWsThreads, kWsSmem, s>>>(a, tt, phimap, imgmap, aff);
+        kern<<<ws_grid(tt), kWsThreads, kWsSmem, s>>>(a, tt, phimap, imgmap, aff);
         e = cudaGetLastError();
     }
     if (im.copy) {
