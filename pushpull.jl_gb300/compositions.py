@@ -43,10 +43,12 @@ def _fits(dim) -> bool:
 
 
 def Exp(v: torch.Tensor) -> torch.Tensor:  # noqa: N802 (the reference's name)
-    """Exponentiate a stationary velocity field ``v (d…, 3)`` (src/compositions.jl:42-50)."""
+    """Exponentiate a stationary velocity field ``v (d…, 3)`` (src/compositions.jl:42-50).
+
+    The result has no autograd history: the steps write through raw pointers."""
     assert v.dim() == 4 and v.shape[3] == 3, "`ϕ` must have three channels"
     _require_cuda(v)
-    u = L.colmajor(v / float(2 ** EXP_STEPS))
+    u = L.colmajor(v.detach() / float(2 ** EXP_STEPS))
     if not _fits(v.shape[:3]):
         Id = identity(v)
         for _ in range(EXP_STEPS):
