@@ -47,8 +47,8 @@ def Exp(v: torch.Tensor) -> torch.Tensor:  # noqa: N802 (the reference's name)
 
     The result has no autograd history: the steps write through raw pointers."""
     assert v.dim() == 4 and v.shape[3] == 3, "`ϕ` must have three channels"
-    _require_cuda(v)
-    u = L.colmajor(v.detach() / float(2 ** EXP_STEPS))
+    u = L.colmajor(v.detach() / float(2 ** EXP_STEPS))     # float32 of integer fields too
+    _require_cuda(u)
     if not _fits(v.shape[:3]):
         Id = identity(v)
         for _ in range(EXP_STEPS):

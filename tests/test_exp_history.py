@@ -8,6 +8,14 @@ import pytest
 import torch
 
 
+def _integer_input(pkg, device):
+    v = torch.arange(-6, 18, device=device).reshape(4, 2, 1, 3)
+    assert torch.equal(pkg.Exp(v), pkg.Exp(v.float()))
+    assert torch.equal(pkg.Exp(v.to(torch.int16)), pkg.Exp(v.float()))
+    with pytest.raises(TypeError):
+        pkg.Exp(v.double())
+
+
 def _velocity(pkg, device, rowmajor):
     g = torch.Generator().manual_seed(5)
     v = torch.rand((6, 5, 4, 3), generator=g) - 0.5
@@ -29,7 +37,11 @@ def _check(pkg, v):
 def torch_steps(pkg, monkeypatch):
     """The native step's contract on CPU tensors: writes ``out`` behind autograd's back."""
     import pushpull_gb300.compositions as comp
-    monkeypatch.setattr(comp, "_require_cuda", lambda *ts: None)
+
+    def require(*ts):
+        if any(t.dtype is not torch.float32 for t in ts):
+            raise TypeError("arrays must be Float32")
+    monkeypatch.setattr(comp, "_require_cuda", require)
 
     def step(u, out, last):
         with torch.no_grad():
@@ -40,6 +52,16 @@ def torch_steps(pkg, monkeypatch):
 @pytest.mark.parametrize("rowmajor", [False, True])
 def test_no_history(pkg, torch_steps, rowmajor):
     _check(pkg, _velocity(pkg, "cpu", rowmajor))
+
+
+def test_integer_velocities(pkg, torch_steps):
+    """v / 2^8 of an integer field is float32: such fields are taken as they always were."""
+    _integer_input(pkg, "cpu")
+
+
+@pytest.mark.gpu
+def test_integer_velocities_on_the_gpu(pkg):
+    _integer_input(pkg, "cuda")
 
 
 @pytest.mark.gpu
