@@ -227,28 +227,46 @@ int pp_batch_launch(pp_batch *plan, void *stream);
 void pp_batch_destroy(pp_batch *plan);
 
 /* ---- kernel selection ------------------------------------------------- */
-/* Ops for the tile registry. */
+/* Ops for the tile registry; the last two, which share the entries of pull_grad and
+ * pull_hess, for pp_get_route only. */
 enum pp_op { PP_OP_PULL = 0, PP_OP_PULL_GRAD = 1, PP_OP_PULL_HESS = 2, PP_OP_PUSH = 3, PP_OP_PUSH_GRAD = 4,
-             PP_OP_FUSED = 5 };
+             PP_OP_FUSED = 5, PP_OP_PULL_GRAD_DOT = 6, PP_OP_PULL_HESS_DOT = 7 };
 /* PP_PATH_AUTO: shared-memory tiled kernels where the degree is isotropic,
  * per-voxel global-memory kernels otherwise; PP_PATH_DIRECT: always the latter. */
 enum pp_path { PP_PATH_AUTO = 0, PP_PATH_DIRECT = 1 };
 
-/* Tile of sample voxels per CTA (2^lx x 2^ly x 2^lz, 32..512 voxels) and the
- * shared-memory budget of its image footprint box in floats, for one op
- * (-1: all ops) and one isotropic degree (-1: all degrees).  cap_floats == 0
- * selects the per-voxel kernels for that (op, degree); this is the default for
- * degree 0 and for the push family and the fused step at degree 1, where
- * gathering straight from L2 beats staging a box.  The code (lx, ly, lz) =
- * (3, 3, 4) selects, for pull, pull_grad and pull_hess (and through their
- * entries pull_grad_dot and pull_hess_dot), the
+/* Tile of sample voxels per CTA (2^lx x 2^ly x 2^lz, 32..512 voxels, push and
+ * push_grad ..1024) and the shared-memory budget of its image footprint box in
+ * floats (push and push_grad: accumulator words, two per element), for one op
+ * (-1: all ops) and one isotropic degree (-1: all degrees).  A tile set here is
+ * used as it is given, wherever its kernels take the launch.
+ * cap_floats == 0 selects the per-voxel kernels for that (op, degree).
+ * cap_floats == -1 returns to the library's own entry (the tile is ignored), under
+ * which the kernels are chosen per call by size, alignment and boundaries.  Until
+ * an entry is set it is the library's own, and pp_get_tile then reports its
+ * nominal tile; setting those values again makes them a choice like any other.
+ * The library's own entries: the per-voxel kernels at degree 0 and, for the push
+ * family and the fused step, at degree 1, where gathering straight from L2 beats
+ * staging a box; push and push_grad at degrees 2..4 a tile by the size of the
+ * sample grid; the pull family at degrees 1..4 the warp-specialised kernels or,
+ * on grids where those are slower, the per-voxel ones.
+ * The code (lx, ly, lz) = (3, 3, 4) selects, for pull, pull_grad and pull_hess
+ * (and through their entries pull_grad_dot and pull_hess_dot), the
  * warp-specialised kernels (one producer warp streams the deformation and
  * stages footprint boxes by TMA while fifteen consumer warps evaluate 8x16x15
- * tiles; their box budget is fixed); it is the default at degrees 1..4.  No
- * reference counterpart (the reference launches one thread per voxel with no
- * tiling, ext/pushpull_gpu.jl:386-391); used by the autotuner. */
+ * tiles; their box budget is fixed).  No reference counterpart (the reference
+ * launches one thread per voxel with no tiling, ext/pushpull_gpu.jl:386-391);
+ * used by the autotuner. */
 int pp_set_tile(int op, int deg, int lx, int ly, int lz, int cap_floats);
 int pp_get_tile(int op, int deg, int *lx, int *ly, int *lz, int *cap_floats);
+/* The kernels a call with these arguments would run on: route = {family, lx, ly,
+ * lz, cap_floats}, family 0 per-voxel kernels (the rest 0), 1 block-synchronous
+ * tiled kernels, 2 warp-specialised kernels.  A host function: nothing is
+ * launched, the pointers' alignment counts and their targets are not read.  No
+ * reference counterpart. */
+int pp_get_route(int op, const float *out, const float *phi, const float *in, const pp_usize d0[3],
+                 const pp_usize d1[3], int nc, int nb, const int *bnd, int nbnd, const int deg[3], int ext,
+                 int route[5]);
 /* Autotuner: times the per-voxel kernels and every candidate tile shape and
  * shared-memory budget for op (PP_OP_PULL .. PP_OP_PUSH_GRAD) on the caller's
  * own arguments (same meaning as the op's entry point; push ops run with

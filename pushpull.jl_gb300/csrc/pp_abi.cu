@@ -95,34 +95,30 @@ TileCfg g_tiles[6][5];   // ops: pull, pull_grad, pull_hess, push, push_grad, fu
 bool g_tiles_init = false;
 int g_path = PP_PATH_AUTO;
 
-bool is_push_default(const TileCfg& t) { return t.lx == 3 && t.ly == 3 && t.lz == 3 && t.cap == 16384; }
-
 // The tile code (lx, ly, lz) = (3, 3, 4) selects the warp-specialised pull
 // kernels (pp_ws.cuh, 8 x 16 x 15 tiles); every other shape the
 // block-synchronous ones.
 bool is_ws_tile(const TileCfg& t) { return t.lx == 3 && t.ly == 3 && t.lz == 4 && t.cap > 0; }
 
+// The library's own entry of (op, degree).  Its tile is what pp_get_tile reports; the
+// kernels of a call under it are chosen by size (pull_route, push_default_tile,
+// fused_grid).
+// Degrees 0 and 1 (one or two taps per axis) of the push family and the fused step:
+// the per-voxel kernels (cap 0), because with so few taps gathering through L2 is
+// faster than a block-synchronous staging of a footprint box (192^3, GB300: push 0.13
+// vs 0.24 ms, fused step 0.29 vs 0.40 ms at degree 1).
+// pull, pull_grad and pull_hess (with the dot ops, which share their entries) at
+// degrees 1..4: the warp-specialised kernels (192^3, GB300, against the
+// block-synchronous family: cubic pull 0.142 vs 0.254 ms, pull_grad 0.175 vs 0.262 ms).
+TileCfg default_tile(int op, int d) {
+    if (op < 3) return d == 0 ? TileCfg{3, 3, 3, 0, true} : TileCfg{3, 3, 4, 15360, true};
+    return TileCfg{3, 3, 3, d <= 1 ? 0 : (op < 5 ? 16384 : (d == 2 ? 2560 : 4096)), true};
+}
+
 void init_tiles_locked() {
     if (g_tiles_init) return;
-    // 8x8x8 tiles; the fused step's 2560-float budget at degree 2 leaves room for
-    // three CTAs per SM.  For push and push_grad at degrees 2..4 the entry stands
-    // for push_default_tile's choice by size.
-    // Degrees 0 and 1 (one or two taps per axis) default to the per-voxel
-    // kernels (cap 0; the pull family at degree 1 is set below): with so few
-    // taps, gathering through L2 is faster than a block-synchronous staging of
-    // a footprint box (192^3, GB300: pull 0.10 vs 0.16 ms, push 0.13 vs
-    // 0.24 ms, fused step 0.29 vs 0.40 ms at degree 1).
     for (int op = 0; op < 6; ++op)
-        for (int d = 0; d < 5; ++d)
-            g_tiles[op][d] = TileCfg{3, 3, 3, d <= 1 ? 0 : (op < 3 ? 8192 : (op < 5 ? 16384 : (d == 2 ? 2560 : 4096)))};
-    // pull, pull_grad and pull_hess (with the dot ops, which share their
-    // entries) at degrees 1..4: the warp-specialised kernels (192^3, GB300,
-    // against the next best family: cubic pull 0.179 vs 0.254 ms, pull_grad
-    // 0.198 vs 0.262 ms, pull_hess 0.222 vs 0.285 ms, pull_grad_dot 0.201 vs
-    // 0.271 ms, pull_hess_dot 0.236 vs 0.298 ms; linear pull 0.084 vs 0.095 ms,
-    // pull_grad 0.095 vs 0.144 ms, pull_hess 0.117 vs 0.177 ms)
-    for (int op = 0; op < 3; ++op)
-        for (int d = 1; d < 5; ++d) g_tiles[op][d] = TileCfg{3, 3, 4, 15360};
+        for (int d = 0; d < 5; ++d) g_tiles[op][d] = default_tile(op, d);
     g_tiles_init = true;
 }
 }  // namespace
@@ -135,7 +131,7 @@ TileCfg tile_for(int op_index, int deg) {
 
 TileCfg push_tile_for(int op, const LaunchArgs& a) {
     const TileCfg t = tile_for(3 + op, a.g.dp[0] - 1);
-    return is_push_default(t) ? push_default_tile(op, a) : t;
+    return t.automatic && t.cap > 0 ? push_default_tile(op, a) : t;
 }
 
 int current_path() {
@@ -245,6 +241,41 @@ static bool prefer_per_voxel(const LaunchArgs& a) {
     }
 }
 
+namespace {
+// What a call runs on.
+enum Family { kPerVoxel = 0, kBlockTiled = 1, kWarpSpecialised = 2 };
+struct Route {
+    Family family;
+    TileCfg t;
+};
+
+// Pull family: the registry's tile where its kernels take the launch, unless the
+// entry is the library's own and the per-voxel kernels are faster at this size.
+Route pull_route(int op, const LaunchArgs& a) {
+    TileCfg t = tile_for(op < 3 ? op : op - 2, a.g.dp[0] - 1);
+    if (current_path() == PP_PATH_DIRECT) return {kPerVoxel, t};
+    if (is_ws_tile(t)) {
+        if (t.automatic && prefer_per_voxel(a)) return {kPerVoxel, t};
+        if (ws_supported(a)) return {kWarpSpecialised, t};
+        // geometries the warp-specialised kernels do not take: the block-synchronous
+        // kernels, or the per-voxel ones at one or two taps per axis
+        t = TileCfg{3, 3, 3, a.g.dp[0] <= 2 ? 0 : 8192};
+    }
+    return {t.cap > 0 && tiled_supported(a, t) ? kBlockTiled : kPerVoxel, t};
+}
+
+Route push_route(int op, const LaunchArgs& a) {
+    const TileCfg t = push_tile_for(op, a);
+    return {current_path() != PP_PATH_DIRECT && push_supported(a, t) ? kBlockTiled : kPerVoxel, t};
+}
+
+Route fused_route(const LaunchArgs& a) {
+    const TileCfg t = tile_for(PP_OP_FUSED, a.g.dp[0] - 1);
+    if (current_path() == PP_PATH_DIRECT || !tiled_supported(a, t)) return {kPerVoxel, t};
+    return {kBlockTiled, t.automatic ? fused_own_tile(a) : t};
+}
+}  // namespace
+
 static int run_pull(int op, float* out, const float* phi, const float* f0, const pp_usize d0[3],
                     const pp_usize d1[3], int nc, int nb, const int* bnd, int nbnd, const int deg[3],
                     int ext, void* stream, const float* up = nullptr) {
@@ -256,25 +287,11 @@ static int run_pull(int op, float* out, const float* phi, const float* f0, const
         if (!aligned4(up)) return fail(PP_ERR_ALIGN, "float pointers must be 4-byte aligned");
         a.up = up;
     }
-    TileCfg t = tile_for(op < 3 ? op : op - 2, deg[0]);
-    cudaError_t e = cudaErrorNotSupported;
-    const bool auto_path = current_path() != PP_PATH_DIRECT;
-    if (auto_path && is_ws_tile(t)) {
-        if (prefer_per_voxel(a)) t.cap = 0;
-        else if (ws_supported(a)) e = launch_ws_pull(op, a, (cudaStream_t)stream);
-        if (e == cudaErrorNotSupported && t.cap > 0) {
-            (void)cudaGetLastError();
-            // ops or geometries the warp-specialised kernels do not take: the
-            // block-synchronous kernels, or the per-voxel ones at one or two taps per axis
-            t = TileCfg{3, 3, 3, deg[0] <= 1 ? 0 : 8192};
-        }
-    }
-    if (e == cudaErrorNotSupported) {
-        if (auto_path && t.cap > 0 && tiled_supported(a, t))
-            e = launch_pull_tiled(op, a, t, (cudaStream_t)stream);
-        else
-            e = launch_pull_direct(op, a, (cudaStream_t)stream);
-    }
+    const Route r = pull_route(op, a);
+    const cudaStream_t s = (cudaStream_t)stream;
+    const cudaError_t e = r.family == kWarpSpecialised ? launch_ws_pull(op, a, s)
+                          : r.family == kBlockTiled    ? launch_pull_tiled(op, a, r.t, s)
+                                                       : launch_pull_direct(op, a, s);
     if (e != cudaSuccess) return cuda_fail(e, "pull launch");
     return PP_OK;
 }
@@ -292,12 +309,9 @@ static int run_push(int op, float* out, const float* phi, const float* in, const
         if (e != cudaSuccess) return cuda_fail(e, "zero output");
     }
     if (g.n1 == 0) return PP_OK;
-    const TileCfg t = push_tile_for(op, a);
-    cudaError_t e;
-    if (current_path() != PP_PATH_DIRECT && push_supported(a, t))
-        e = launch_push_tiled(op, a, t, (cudaStream_t)stream);
-    else
-        e = launch_push_direct(op, a, (cudaStream_t)stream);
+    const Route r = push_route(op, a);
+    const cudaError_t e = r.family == kBlockTiled ? launch_push_tiled(op, a, r.t, (cudaStream_t)stream)
+                                                  : launch_push_direct(op, a, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "push launch");
     return PP_OK;
 }
@@ -324,8 +338,9 @@ static int run_fused(double* loss, float* df, float* dphi, const float* f0, cons
     if (!aligned4(g) || !aligned4(dphi)) return fail(PP_ERR_ALIGN, "float pointers must be 4-byte aligned");
     a.up = g;
     a.out2 = dphi;
-    const TileCfg t = tile_for(PP_OP_FUSED, deg[0]);
-    const bool tiled = current_path() != PP_PATH_DIRECT && tiled_supported(a, t);
+    const Route r = fused_route(a);
+    const TileCfg& t = r.t;
+    const bool tiled = r.family == kBlockTiled;
     long long slots;
     int grid = 0;
     if (tiled) {
@@ -427,19 +442,26 @@ int pp_set_tile(int op, int deg, int lx, int ly, int lz, int cap_floats) {
     if (op < -1 || op > 5) return pp::fail(PP_ERR_UNSUPPORTED, "op %d outside -1..5", op);
     if (deg < -1 || deg > 4) return pp::fail(PP_ERR_DEGREE, "deg %d outside -1..4", deg);
     const bool ws = lx == 3 && ly == 3 && lz == 4;   // the warp-specialised pull tile
-    if (!ws && (lx < 0 || ly < 0 || lz < 0 || lx + ly + lz < 5 || lx + ly + lz > 9))
-        return pp::fail(PP_ERR_UNSUPPORTED, "tile 2^%d x 2^%d x 2^%d must hold 32..512 voxels (or be the code 3,3,4)", lx,
-                        ly, lz);
-    if (ws && cap_floats != 0 && (op < 0 || op > 2))
-        return pp::fail(PP_ERR_UNSUPPORTED, "the tile code 3,3,4 (warp-specialised kernels) serves pull and pull_grad only");
-    if (cap_floats != 0 && (cap_floats < 64 || (cap_floats & 3) || cap_floats > (227 * 1024) / 4))
-        return pp::fail(PP_ERR_UNSUPPORTED, "cap %d floats must be 0 or a multiple of 4 in [64, 58112]",
-                        cap_floats);
+    const bool defaults = cap_floats == -1;
+    const int most = op == 3 || op == 4 ? 10 : 9;    // the push kernels take 1024 voxels as well
+    if (!defaults) {
+        if (!ws && (lx < 0 || ly < 0 || lz < 0 || lx + ly + lz < 5 || lx + ly + lz > most))
+            return pp::fail(PP_ERR_UNSUPPORTED,
+                            "tile 2^%d x 2^%d x 2^%d must hold 32..%d voxels (or be the code 3,3,4)", lx, ly, lz,
+                            1 << most);
+        if (ws && cap_floats != 0 && (op < 0 || op > 2))
+            return pp::fail(PP_ERR_UNSUPPORTED,
+                            "the tile code 3,3,4 (warp-specialised kernels) serves pull and pull_grad only");
+        if (cap_floats != 0 && (cap_floats < 64 || (cap_floats & 3) || cap_floats > (227 * 1024) / 4))
+            return pp::fail(PP_ERR_UNSUPPORTED, "cap %d floats must be 0, a multiple of 4 in [64, 58112] or -1",
+                            cap_floats);
+    }
     std::lock_guard<std::mutex> lk(pp::g_cfg_mu);
     pp::init_tiles_locked();
     for (int o = 0; o < 6; ++o)
         for (int d = 0; d < 5; ++d)
-            if ((op < 0 || o == op) && (deg < 0 || d == deg)) pp::g_tiles[o][d] = pp::TileCfg{lx, ly, lz, cap_floats};
+            if ((op < 0 || o == op) && (deg < 0 || d == deg))
+                pp::g_tiles[o][d] = defaults ? pp::default_tile(o, d) : pp::TileCfg{lx, ly, lz, cap_floats};
     return PP_OK;
 }
 
@@ -451,6 +473,24 @@ int pp_get_tile(int op, int deg, int* lx, int* ly, int* lz, int* cap_floats) {
     *ly = t.ly;
     *lz = t.lz;
     *cap_floats = t.cap;
+    return PP_OK;
+}
+
+int pp_get_route(int op, const float* out, const float* phi, const float* in, const pp_usize d0[3],
+                 const pp_usize d1[3], int nc, int nb, const int* bnd, int nbnd, const int deg[3], int ext,
+                 int route[5]) {
+    using namespace pp;
+    if (op < 0 || op > PP_OP_PULL_HESS_DOT) return fail(PP_ERR_UNSUPPORTED, "op %d outside 0..7", op);
+    if (!route) return fail(PP_ERR_NULL, "route must not be NULL");
+    LaunchArgs a{};
+    int rc = prepare(a, const_cast<float*>(out), phi, in, d0, d1, nc, nb, bnd, nbnd, deg, ext);
+    if (rc != PP_OK) return rc;
+    const Route r = op == PP_OP_FUSED                            ? fused_route(a)
+                    : op == PP_OP_PUSH || op == PP_OP_PUSH_GRAD  ? push_route(op - PP_OP_PUSH, a)
+                                                                 : pull_route(op < 3 ? op : op - 3, a);
+    const TileCfg t = r.family == kPerVoxel ? TileCfg{0, 0, 0, 0} : r.t;
+    const int v[5] = {r.family, t.lx, t.ly, t.lz, t.cap};
+    for (int k = 0; k < 5; ++k) route[k] = v[k];
     return PP_OK;
 }
 
@@ -482,7 +522,8 @@ int pp_autotune(int op, float* out, const float* phi, const float* in, const pp_
             default: return pp_push_grad(out, phi, in, d0, d1, nc, nb, bnd, nbnd, deg, ext, 0, stream);
         }
     };
-    const int tiles[][3] = {{3, 3, 3}, {4, 3, 2}, {4, 2, 3}, {5, 2, 2}, {3, 4, 2}, {3, 3, 2}, {4, 2, 2}, {3, 3, 4}};
+    const int tiles[][3] = {{3, 3, 3}, {4, 3, 2}, {4, 2, 3}, {5, 2, 2}, {3, 4, 2},
+                            {3, 3, 2}, {4, 2, 2}, {4, 3, 3}, {3, 3, 4}};
     const int caps_pull[] = {6144, 8192, 12288};
     const int caps_push[] = {7936, 9984, 16384};
     const TileCfg saved = tile_for(op, deg[0]);
@@ -521,6 +562,7 @@ int pp_autotune(int op, float* out, const float* phi, const float* in, const pp_
     for (const auto& t : tiles) {
         const bool ws = t[0] == 3 && t[1] == 3 && t[2] == 4;
         if (ws && is_push) continue;
+        if (t[0] + t[1] + t[2] > 9 && !is_push && !ws) continue;
         for (int ci = 0; ci < (ws ? 1 : 3) && rc == PP_OK; ++ci) {
             const int cap = ws ? 15360 : (is_push ? caps_push[ci] : caps_pull[ci]);
             if (pp_set_tile(op, deg[0], t[0], t[1], t[2], cap) != PP_OK) continue;
@@ -540,7 +582,8 @@ int pp_autotune(int op, float* out, const float* phi, const float* in, const pp_
     cudaEventDestroy(e1);
     pp_set_path(saved_path);
     if (rc != PP_OK) {
-        pp_set_tile(op, deg[0], saved.lx, saved.ly, saved.lz, saved.cap);
+        std::lock_guard<std::mutex> lk(g_cfg_mu);
+        g_tiles[op][deg[0]] = saved;
         return rc;
     }
     // install the winner: a tile configuration, or cap 0 for the per-voxel kernels

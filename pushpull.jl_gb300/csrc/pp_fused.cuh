@@ -247,15 +247,10 @@ __global__ void __launch_bounds__(kPushThreads, kFusedCtas<DP>) k_fused_tiled(co
     }
 }
 
-// Tile grid, shared memory and CTAs of a fused launch.  The registry's default
-// entries (8x8x8 voxels, 2560 floats at degree 2, 4096 above) stand for the tile and
-// budget (floats of the image box, words of the accumulator) measured best:
-// 160x192x160 quadratic, us: 16x8x4 229, 8x8x8 241, 16x4x8 237, 8x16x4 250, 32x4x4
-// 248; with five CTAs per SM and a larger budget 237, with four 231.
+// Tile grid, shared memory and CTAs of a fused launch.
 TileGrid fused_grid(const LaunchArgs& a, TileCfg c, size_t& smem, int& ctas) {
     const int dp = a.g.dp[0];
-    if (c.lx == 3 && c.ly == 3 && c.lz == 3 && c.cap == (dp == 3 ? 2560 : 4096))
-        c = TileCfg{4, 3, 2, dp <= 3 ? 3072 : 4864};
+    if (c.automatic) c = fused_own_tile(a);
     TileGrid t = make_grid(a, c);
     t.pmod = (1 << c.lx) & 31;
     const int most = dp <= 3 ? kFusedCtas<3> : kFusedCtas<4>;

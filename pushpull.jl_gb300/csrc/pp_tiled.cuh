@@ -10,12 +10,14 @@ namespace pp {
 struct TileCfg {
     int lx, ly, lz;
     int cap;
+    bool automatic = false;   // the library's own entry: kernel and tile are chosen by the call's size;
+                              // otherwise they are the caller's choice
 };
 
 bool tiled_supported(const LaunchArgs& a, const TileCfg& t);
 // the same for the push family, whose tiles hold up to 2048 voxels
 bool push_supported(const LaunchArgs& a, const TileCfg& t);
-// the push tile for a launch when the registry holds its default entry (16x8x8)
+// the push tile for a launch whose registry entry is the library's own
 TileCfg push_default_tile(int op, const LaunchArgs& a);
 // warp-specialised pull family (8 x 16 x 15 tiles, pp_ws.cuh): geometry test and
 // launch (cudaErrorNotSupported for ops or layouts it does not take)
@@ -44,6 +46,8 @@ struct TileGrid {
     int nv, stages;     // push: voxels per tile, ring slots
 };
 
+// The fused step's tile for a launch whose registry entry is the library's own.
+TileCfg fused_own_tile(const LaunchArgs& a);
 // Fused forward + adjoint step over tiles: grid size for a launch, and the
 // launch itself (one loss partial per CTA into a.partial[0 .. grid)).
 int fused_tiled_grid(const LaunchArgs& a, const TileCfg& t);

@@ -4,6 +4,11 @@
 
 namespace pp {
 
+// The tile and budget (floats of the image box, words of the accumulator) measured
+// best: 160x192x160 quadratic, us: 16x8x4 229, 8x8x8 241, 16x4x8 237, 8x16x4 250,
+// 32x4x4 248; with five CTAs per SM and a larger budget 237, with four 231.
+TileCfg fused_own_tile(const LaunchArgs& a) { return TileCfg{4, 3, 2, a.g.dp[0] <= 3 ? 3072 : 4864}; }
+
 int fused_tiled_grid(const LaunchArgs& a, const TileCfg& c) {
     size_t smem;
     int ctas;

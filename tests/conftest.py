@@ -37,6 +37,17 @@ def pkg():
     return entry.package()
 
 
+@pytest.fixture(autouse=True)
+def _own_tiles(request):
+    """Every test that uses the package starts from the library's own tile registry
+    entries (a test that reads the tiles, sets others and sets the old values again
+    leaves them as explicit choices)."""
+    if "pkg" in request.fixturenames:
+        lib = request.getfixturevalue("pkg").native_library()
+        assert lib.pp_set_tile(-1, -1, 0, 0, 0, -1) == 0
+    yield
+
+
 @pytest.fixture(scope="session")
 def O():
     from oracle import oracle

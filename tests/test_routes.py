@@ -1,0 +1,75 @@
+"""Which kernels a call runs on (pp_get_route; host logic, no GPU): a tile that was set
+is used as it is given, the library's own entry chooses by the call."""
+from __future__ import annotations
+
+import ctypes as C
+
+import pytest
+
+PULL, GRAD, HESS, PUSH, PUSHG, FUSED, GDOT, HDOT = range(8)
+PER_VOXEL, BLOCK, WS = range(3)
+
+
+@pytest.fixture
+def lib(pkg):
+    lib = pkg.native_library()
+    yield lib
+    assert lib.pp_set_tile(-1, -1, 0, 0, 0, -1) == 0 and lib.pp_set_path(0) == 0
+
+
+def route(lib, op, deg, d1, d0=None, bnd=(1, 1, 1), nc=1, nb=1, ext=1, ptrs=(256, 256, 256)):
+    out = (C.c_int * 5)()
+    u = C.c_ulonglong * 3
+    rc = lib.pp_get_route(op, *ptrs, u(*(d0 or d1)), u(*d1), nc, nb, C.cast((C.c_int * 3)(*bnd), C.c_void_p), 1,
+                          (C.c_int * 3)(*((deg,) * 3 if isinstance(deg, int) else deg)), ext, out)
+    assert rc == 0, lib.pp_last_error()
+    return tuple(out)
+
+
+@pytest.mark.parametrize("op", [PULL, GRAD, HESS, GDOT, HDOT])
+@pytest.mark.parametrize("deg", [1, 2, 3, 4])
+@pytest.mark.parametrize("bnd", [(1, 1, 1), (0, 1, 2)])
+@pytest.mark.parametrize("d1", [(40, 36, 44), (41, 35, 43), (192, 192, 39)])
+def test_the_warp_specialised_code_is_honoured(lib, op, deg, bnd, d1):
+    entry = {GDOT: GRAD, HDOT: HESS}.get(op, op)
+    assert lib.pp_set_tile(entry, deg, 3, 3, 4, 15360) == 0
+    assert route(lib, op, deg, d1, d0=(96, 96, 97), bnd=bnd) == (WS, 3, 3, 4, 15360)
+    assert lib.pp_set_path(1) == 0
+    assert route(lib, op, deg, d1, bnd=bnd)[0] == PER_VOXEL
+
+
+@pytest.mark.parametrize("op,tile", [(PULL, (3, 3, 3, 8192)), (HESS, (4, 3, 2, 6144)), (PUSH, (3, 3, 3, 16384)),
+                                     (PUSH, (4, 3, 3, 19968)), (PUSHG, (3, 3, 3, 16384)), (PUSHG, (3, 3, 2, 9984)),
+                                     (FUSED, (3, 3, 3, 2560)), (FUSED, (3, 3, 3, 4096))])
+@pytest.mark.parametrize("d1", [(40, 36, 44), (192, 192, 192)])
+def test_a_set_tile_is_honoured(lib, op, tile, d1):
+    for deg in (2, 3, 4):
+        assert lib.pp_set_tile(op, deg, *tile) == 0
+        assert route(lib, op, deg, d1) == (BLOCK,) + tile
+    assert lib.pp_set_tile(op, 3, *tile[:3], 0) == 0
+    assert route(lib, op, 3, d1)[0] == PER_VOXEL
+
+
+def test_back_to_the_own_entry(lib):
+    """Read and set again is a choice; cap -1 is the way back."""
+    def tile(op, deg):
+        v = [C.c_int() for _ in range(4)]
+        assert lib.pp_get_tile(op, deg, *[C.byref(x) for x in v]) == 0
+        return tuple(x.value for x in v)
+
+    small = (40, 36, 44)
+    own = {(op, deg): route(lib, op, deg, small) for op in range(8) for deg in range(5)}
+    assert own[PULL, 3][0] == PER_VOXEL and own[FUSED, 2] == (BLOCK, 4, 3, 2, 3072)
+    seen = {(op, deg): tile(op, deg) for op in range(6) for deg in range(5)}
+    for (op, deg), t in seen.items():
+        assert lib.pp_set_tile(op, deg, *t) == 0 and tile(op, deg) == t
+    assert route(lib, PULL, 3, small)[0] == WS and route(lib, PUSH, 3, small) == (BLOCK, 3, 3, 3, 16384)
+    assert lib.pp_set_tile(-1, -1, 0, 0, 0, -1) == 0
+    assert {k: route(lib, *k, small) for k in own} == own
+    assert {k: tile(*k) for k in seen} == seen
+
+
+def test_refused(lib):
+    for op, t in [(PULL, (4, 3, 3, 8192)), (-1, (4, 3, 3, 8192)), (FUSED, (4, 3, 3, 2560)), (PUSH, (4, 4, 3, 8192)),
+                  (PUSH, (3, 3, 4, 8192)), (PULL, (3, 3, 3, -2)), (PULL, (3, 3, 3, 66)), (6, (3, 3, 3, 0))]:
+        assert lib.pp_set_tile(op, 3, *t) != 0 and lib.pp_last_error()
