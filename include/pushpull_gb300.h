@@ -261,7 +261,8 @@ int pp_set_tile(int op, int deg, int lx, int ly, int lz, int cap_floats);
 int pp_get_tile(int op, int deg, int *lx, int *ly, int *lz, int *cap_floats);
 /* The kernels a call with these arguments would run on: route = {family, lx, ly,
  * lz, cap_floats}, family 0 per-voxel kernels (the rest 0), 1 block-synchronous
- * tiled kernels, 2 warp-specialised kernels.  A host function: nothing is
+ * tiled kernels, 2 warp-specialised kernels, 3 family 2 or, where a sample of the
+ * deformation shows footprints that it has no room for, family 0.  A host function: nothing is
  * launched, the pointers' alignment counts and their targets are not read.  No
  * reference counterpart. */
 int pp_get_route(int op, const float *out, const float *phi, const float *in, const pp_usize d0[3],

@@ -207,6 +207,20 @@ int prepare_args(LaunchArgs& a, float* out, const float* phi, const float* in, c
     return prepare(a, out, phi, in, d0, d1, nc, nb, bnd, nbnd, deg, ext);
 }
 
+// Sample grids so much coarser than the image that an 8 x 16 x 15 tile's footprint may
+// not fit its buffer of 640 rows of 24 floats, and the per-voxel kernels are faster
+// where it does not.  160^3 samples over the whole of a finer image, per-voxel /
+// warp-specialised, us, GB300: over 220^3 pull quadratic 93 / 109, cubic 167 / 161,
+// quartic 290 / 252, cubic pull_hess 202 / 186; over 320^3 102 / 156, 174 / 276,
+// 299 / 458, 218 / 276.  A 96^3 block out of the middle of 192^3 has the same ratio of
+// extents as the latter and spacing one: cubic pull 34 / 24, quartic 60 / 36.  So the
+// extents only say where to look at the deformation itself: both kernels are launched
+// and a sample of it decides in each which one runs.  Small quadratic grids, where that
+// costs more than it gives (the block 15 / 17), go per voxel.
+static bool coarse_grid(int op, const LaunchArgs& a) {
+    return grid_zoom(a) >= (op == kPull && a.g.dp[0] == 3 ? 1.25 : 1.5);
+}
+
 // Sample grids on which the per-voxel kernels beat the warp-specialised ones:
 // small ones, because those take 1920 voxels per CTA at a time, and larger ones
 // where their boxes do not arrive by TMA alone (odd x extents, circulant margins).
@@ -217,17 +231,9 @@ int prepare_args(LaunchArgs& a, float* out, const float* phi, const float* in, c
 // 181x217x181 76 / 133; quadratic 121x145x121 46 / 57, 181x217x181 138 / 151; cubic
 // 91x109x91 40 / 43, 121x145x121 (two channels) 121 / 118; quartic 61x73x61 27 /
 // 32, 91x109x91 66 / 63.  Circulant: quadratic 128^3 54 / 58, cubic 76 / 74.
-static bool prefer_per_voxel(const LaunchArgs& a) {
+static bool prefer_per_voxel(int op, const LaunchArgs& a) {
     const Geometry& g = a.g;
     if (g.dp[0] != g.dp[1] || g.dp[1] != g.dp[2] || g.n0 >= (1LL << 31) - 1) return false;
-    // a sample grid that spans a finer image: an 8 x 16 x 15 tile's footprint does not
-    // fit its buffer of 640 rows of 24 (160^3, per-voxel / warp-specialised, pull: into
-    // 192^3 quadratic 87 / 76, cubic 156 / 138, quartic 278 / 230; into 205^3 91 / 122,
-    // 171 / 182, 304 / 304; quartic pull_grad into 220^3 314 / 498)
-    const double ry = g.d1[1] > 1 ? (double)(g.d0[1] - 1) / (double)(g.d1[1] - 1) : 1.0;
-    const double rz = g.d1[2] > 1 ? (double)(g.d0[2] - 1) / (double)(g.d1[2] - 1) : 1.0;
-    const double most = g.dp[0] == 5 ? 650.0 : (g.dp[0] == 4 ? 600.0 : 575.0);
-    if ((15.0 * ry + g.dp[1] + 2.5) * (14.0 * rz + g.dp[2] + 2.5) > most) return true;
     const long long n = g.n1 * g.nb;
     const bool odd = (g.d1[0] & 3) || (reinterpret_cast<uintptr_t>(a.phi) & 15);
     bool rough = odd || (g.d0[0] & 3) || (reinterpret_cast<uintptr_t>(a.in) & 15);
@@ -235,7 +241,7 @@ static bool prefer_per_voxel(const LaunchArgs& a) {
         rough = rough || !a.bnd.code[c][0] || !a.bnd.code[c][1] || !a.bnd.code[c][2];
     switch (g.dp[0]) {
         case 2: return rough || n <= (1LL << 21);
-        case 3: return odd || n <= (rough ? 1LL << 21 : 1LL << 19);
+        case 3: return odd || n <= (rough ? 1LL << 21 : 1LL << 19) || (n < (1LL << 21) && coarse_grid(op, a));
         case 4: return n <= (rough ? 1LL << 21 : 1LL << 19);
         default: return n <= (rough ? 1LL << 20 : 1LL << 18);
     }
@@ -243,11 +249,19 @@ static bool prefer_per_voxel(const LaunchArgs& a) {
 
 namespace {
 // What a call runs on.
-enum Family { kPerVoxel = 0, kBlockTiled = 1, kWarpSpecialised = 2 };
+enum Family { kPerVoxel = 0, kBlockTiled = 1, kWarpSpecialised = 2, kSampled = 3 };
 struct Route {
     Family family;
     TileCfg t;
 };
+
+// Do the launch's outputs overlap its deformation?  (Of two launches, the second must
+// find the deformation as the first did.)
+bool writes_phi(int op, const LaunchArgs& a) {
+    const long long comps = op == kPull ? a.g.nc : (op == kPullGrad ? 3LL * a.g.nc : (op == kPullHess ? 9LL * a.g.nc : 3));
+    const float* out = a.out;
+    return out < a.phi + 3 * a.g.n1 * a.g.nb && a.phi < out + comps * a.g.n1 * a.g.nb;
+}
 
 // Pull family: the registry's tile where its kernels take the launch, unless the
 // entry is the library's own and the per-voxel kernels are faster at this size.
@@ -255,8 +269,11 @@ Route pull_route(int op, const LaunchArgs& a) {
     TileCfg t = tile_for(op < 3 ? op : op - 2, a.g.dp[0] - 1);
     if (current_path() == PP_PATH_DIRECT) return {kPerVoxel, t};
     if (is_ws_tile(t)) {
-        if (t.automatic && prefer_per_voxel(a)) return {kPerVoxel, t};
-        if (ws_supported(a)) return {kWarpSpecialised, t};
+        if (t.automatic && prefer_per_voxel(op, a)) return {kPerVoxel, t};
+        if (ws_supported(a)) {
+            const bool look = t.automatic && coarse_grid(op, a) && !writes_phi(op, a);
+            return {look ? kSampled : kWarpSpecialised, t};
+        }
         // geometries the warp-specialised kernels do not take: the block-synchronous
         // kernels, or the per-voxel ones at one or two taps per axis
         t = TileCfg{3, 3, 3, a.g.dp[0] <= 2 ? 0 : 8192};
@@ -289,9 +306,14 @@ static int run_pull(int op, float* out, const float* phi, const float* f0, const
     }
     const Route r = pull_route(op, a);
     const cudaStream_t s = (cudaStream_t)stream;
-    const cudaError_t e = r.family == kWarpSpecialised ? launch_ws_pull(op, a, s)
-                          : r.family == kBlockTiled    ? launch_pull_tiled(op, a, r.t, s)
-                                                       : launch_pull_direct(op, a, s);
+    cudaError_t e = cudaSuccess;
+    if (r.family == kWarpSpecialised || r.family == kSampled) {
+        a.sample = r.family == kSampled ? kIfBoxesFit : 0;
+        e = launch_ws_pull(op, a, s);
+        a.sample = kIfBoxesOverflow;
+    }
+    if (e == cudaSuccess && (r.family == kPerVoxel || r.family == kSampled)) e = launch_pull_direct(op, a, s);
+    if (r.family == kBlockTiled) e = launch_pull_tiled(op, a, r.t, s);
     if (e != cudaSuccess) return cuda_fail(e, "pull launch");
     return PP_OK;
 }

@@ -14,8 +14,22 @@
 namespace pp {
 namespace {
 
+// Is a launch that runs only where the sampled boxes overflow (a.sample) to run?  All
+// threads of the block.
+template <int DP, int OP>
+__device__ __forceinline__ bool sampled_in(const LaunchArgs& a) {
+    __shared__ int s_run;
+    if (threadIdx.x < 32) {
+        const bool over = sampled_overflow<DP, OP>(a);
+        if (threadIdx.x == 0) s_run = over;
+    }
+    __syncthreads();
+    return s_run;
+}
+
 template <int DP, int OP, typename IT>
 __global__ void __launch_bounds__(256, DP >= 4 ? 2 : 0) k_pull_direct(LaunchArgs a) {
+    if (DP > 0 && a.sample && !sampled_in<DP, OP>(a)) return;
     const Geometry& g = a.g;
     const long long n1 = g.n1;
     const int b = blockIdx.y;
@@ -63,6 +77,7 @@ template <int DP, int OP_, int V>
 __global__ void __launch_bounds__(256, DP == 3 && op_order(OP_) <= 1 && !pull_is_dot<OP_>() ? 3 : 0) k_pull_lean(const __grid_constant__ LaunchArgs a) {
     constexpr int OP = pull_base_op<OP_>();
     constexpr int ORD = op_order(OP);
+    if (a.sample && !sampled_in<DP, OP_>(a)) return;
     const Geometry& g = a.g;
     const long long n1 = g.n1;
     const int b = blockIdx.y;
@@ -182,16 +197,19 @@ cudaError_t dispatch_dp(const LaunchArgs& a, dim3 grid, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-dim3 direct_grid(const LaunchArgs& a) {
+dim3 direct_grid(int op, const LaunchArgs& a) {
     const long long blocks_needed = (a.g.n1 + 255) / 256;
-    const long long cap = (long long)sm_count() * 8;
+    long long cap = (long long)sm_count() * 8;
+    // only where the sample says so: no more blocks than fit at once, which look at it
+    // once each (eight per SM take three rounds: 6 us more)
+    if (a.sample) cap = ((long long)sm_count() * (a.g.dp[0] > 3 ? 2 : (op <= kPullGrad ? 3 : 6)) + a.g.nb - 1) / a.g.nb;
     return dim3((unsigned)(blocks_needed < cap ? blocks_needed : cap), (unsigned)a.g.nb);
 }
 
 }  // namespace
 
 cudaError_t launch_pull_direct(int op, const LaunchArgs& a, cudaStream_t s) {
-    const dim3 grid = direct_grid(a);
+    const dim3 grid = direct_grid(op, a);
     const bool small = a.g.n0 < (1LL << 31) - 1;
     switch (op) {
         case kPull: return small ? dispatch_dp<kPull, int, false>(a, grid, s)
@@ -208,7 +226,7 @@ cudaError_t launch_pull_direct(int op, const LaunchArgs& a, cudaStream_t s) {
 }
 
 cudaError_t launch_push_direct(int op, const LaunchArgs& a, cudaStream_t s) {
-    const dim3 grid = direct_grid(a);
+    const dim3 grid = direct_grid(op, a);
     const bool small = a.g.n0 < (1LL << 31) - 1;
     if (op == kPush)
         return small ? dispatch_dp<kPush, int, true>(a, grid, s) : dispatch_dp<kPush, long long, true>(a, grid, s);

@@ -19,6 +19,13 @@ __host__ __device__ constexpr int op_order(int op) {
     return op == kPull ? 0 : (op == kPullHess || op == kPullHessDot ? 2 : 1);
 }
 enum PushOp { kPush = 0, kPushGrad = 1 };
+enum Sample { kIfBoxesFit = 1, kIfBoxesOverflow = 2 };
+
+// Sample tile of the warp-specialised pull kernels (8 x 16 x 15 voxels) and the floats
+// of its footprint box's buffer.
+constexpr int kWsLy = 4, kWsTy = 1 << kWsLy, kWsTz = 15;
+constexpr int kWsWinX = 24, kWsRows = 640;
+constexpr int kWsCap = kWsWinX * kWsRows;
 
 // Arguments of one pull-family or push-family launch.  Pointers address the
 // first (channel 0, batch 0) element; channel c / batch b slices follow the
@@ -31,9 +38,24 @@ struct LaunchArgs {
                         // fused step: the target g, (d1, nc, nb)
     float* out2;        // fused step: deformation cotangent (d1, 3, nb); push: count image or NULL
     double* partial;    // fused step: one loss partial per CTA
+    int sample;         // pull family: 0 always run; kIfBoxesFit, kIfBoxesOverflow: only where a sample of
+                        // the deformation says so (sampled_overflow)
     Geometry g;
     BndTable bnd;
 };
+
+// Image voxels per sample voxel along the axis where they are fewest.  A sample grid
+// that spans the image has about this spacing; a slab or a block of a larger grid,
+// which spans a part of the image along some axes only, has it too.
+inline double grid_zoom(const LaunchArgs& a) {
+    double z = 1e30;
+    for (int k = 0; k < 3; ++k)
+        if (a.g.d1[k] > 1) {
+            const double r = (double)(a.g.d0[k] - 1) / (double)(a.g.d1[k] - 1);
+            z = r < z ? r : z;
+        }
+    return z < 1e30 ? z : 1.0;
+}
 
 // pull family: direct gather (one thread per sample voxel, all channels per thread)
 cudaError_t launch_pull_direct(int op, const LaunchArgs& a, cudaStream_t s);

@@ -40,6 +40,49 @@ __device__ __forceinline__ float* pull_out(const LaunchArgs& a, int b, int c, lo
     return a.out + ((long long)b * a.g.nc + c) * NCOMP * a.g.n1 + v;
 }
 
+// Do most of 32 sample tiles, spread over the grid, have a footprint that the
+// warp-specialised kernels' buffer does not hold?  By the positions of each tile's
+// eight corners; the answer is the same in every lane of every warp of both kernels
+// that ask (one runs if it is yes, the other if it is no).  One warp.
+template <int DP, int OP>
+__device__ __forceinline__ bool sampled_overflow(const LaunchArgs& a) {
+    const Geometry& g = a.g;
+    const int ntx = (int)((g.d1[0] + 7) >> 3), nty = (int)((g.d1[1] + kWsTy - 1) >> kWsLy);
+    const int ntz = (int)((g.d1[2] + kWsTz - 1) / kWsTz);
+    const long long per = (long long)ntx * nty * ntz;
+    long long T = (2 * (long long)(threadIdx.x & 31) + 1) * per * g.nb >> 6;
+    const float* phi = a.phi + T / per * 3 * g.n1;
+    T %= per;
+    const long long x0 = T % ntx * 8, y0 = T / ntx % nty * kWsTy, z0 = T / ((long long)ntx * nty) * kWsTz;
+    float lo[3], hi[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = 3.0e38f;
+        hi[k] = -3.0e38f;
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const long long x = min(x0 + (c & 1 ? 7 : 0), g.d1[0] - 1), y = min(y0 + (c & 2 ? kWsTy - 1 : 0), g.d1[1] - 1);
+        const long long z = min(z0 + (c & 4 ? kWsTz - 1 : 0), g.d1[2] - 1);
+        const long long v = x + g.d1[0] * (y + g.d1[1] * z);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float p = __ldg(phi + v + k * g.n1);
+            if (finitef(p)) {
+                lo[k] = fminf(lo[k], p);
+                hi[k] = fmaxf(hi[k], p);
+            }
+        }
+    }
+    // taps of the corners' span; rows carry three words of alignment, and the quadratic
+    // pull gains only where a box of 24-word rows fits
+    float e[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) e[k] = fmaxf(hi[k] - lo[k], 0.f) + (float)(DP + 1);
+    const float row = OP == kPull && DP == 3 ? fmaxf(e[0] + 3.f, (float)kWsWinX) : e[0] + 3.f;
+    return __popc(__ballot_sync(0xffffffffu, row * e[1] * e[2] > (float)kWsCap)) > 16;
+}
+
 // Write every output component of voxel v as NaN (invalid sample).
 template <int OP>
 __device__ __forceinline__ void pull_voxel_nan(const LaunchArgs& a, int b, long long v) {

@@ -57,14 +57,13 @@ constexpr int kWsV = 4;                        // sample voxels per consumer thr
 // still fits the window and few samples of the last tiles are lost (192^3 cubic
 // pull 156 -> 154 us, pull_grad 179 -> 175, 181x217x181 200 -> 191 against 8 x 8 x
 // 30; affine pulls with rotations up to 10 degrees 191 -> 167).
-constexpr int kWsLy = 4, kWsTy = 1 << kWsLy, kWsTz = 15;   // tile: 8 x 16 x 15 sample voxels
+// (kWsLy, kWsTy and kWsTz are shared with the per-voxel kernels: pp_kernels.cuh.)
 constexpr int kWsNV = kWsCons * kWsV;          // 1920 voxels per tile
 constexpr int kWsStages = 4;                   // deformation ring slots
 constexpr int kWsBufs = 2;                     // box buffers
-// TMA image window: row pitch 24 (an undeformed 8 x 4 warp tile reads 32 distinct
-// banks), t.winy rows and t.winz planes chosen per launch (ws_window)
-constexpr int kWsWinX = 24, kWsRows = 640;
-constexpr int kWsCap = kWsWinX * kWsRows;      // floats per box buffer
+// TMA image window: row pitch kWsWinX = 24 (an undeformed 8 x 4 warp tile reads 32
+// distinct banks), t.winy rows and t.winz planes, kWsRows rows at most, chosen per
+// launch (ws_window); kWsCap floats per box buffer
 constexpr size_t kWsSmem = (size_t)(kWsStages * 3 * kWsNV + kWsBufs * kWsCap) * sizeof(float);
 
 __device__ __forceinline__ void mbar_arrive(unsigned bar) {
@@ -420,6 +419,14 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_pull_ws(const __grid_constant
     // unit ahead, and publish their bounds two tiles ahead
     const bool ahead = t.img_tma == 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (!AFF && a.sample) {
+        if (warp == 0) {
+            const bool over = sampled_overflow<DP, OP>(a);
+            if (lane == 0) s_abort = over;
+        }
+        __syncthreads();
+        if (s_abort) return;
+    }
     if (threadIdx.x == 0) {
         s_abort = 0;
         for (int k = 0; k < kWsStages; ++k) mbar_init(phi_full + 8u * k, 1);
@@ -675,10 +682,12 @@ TileGrid ws_make_grid(const LaunchArgs& a) {
     t.nv = kWsNV;
     t.stages = kWsStages;
     // the sample grid usually spans the image: a tile's footprint scales with their
-    // ratio, plus the taps and some displacement
+    // ratio, plus the taps and some displacement.  A ratio above the smallest of the
+    // three (and above one) is a slab's, which spans a part of the image there.
+    const double most = std::fmax(1.0, grid_zoom(a));
     const double ry = a.g.d1[1] > 1 ? (double)(a.g.d0[1] - 1) / (double)(a.g.d1[1] - 1) : 1.0;
     const double rz = a.g.d1[2] > 1 ? (double)(a.g.d0[2] - 1) / (double)(a.g.d1[2] - 1) : 1.0;
-    ws_window(t, (kWsTy - 1) * ry + a.g.dp[0] + 3.5, (kWsTz - 1) * rz + a.g.dp[0] + 3.5);
+    ws_window(t, (kWsTy - 1) * std::fmin(ry, most) + a.g.dp[0] + 3.5, (kWsTz - 1) * std::fmin(rz, most) + a.g.dp[0] + 3.5);
     return t;
 }
 

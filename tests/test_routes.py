@@ -7,7 +7,7 @@ import ctypes as C
 import pytest
 
 PULL, GRAD, HESS, PUSH, PUSHG, FUSED, GDOT, HDOT = range(8)
-PER_VOXEL, BLOCK, WS = range(3)
+PER_VOXEL, BLOCK, WS, SAMPLED = range(4)
 
 
 @pytest.fixture
@@ -73,3 +73,26 @@ def test_refused(lib):
     for op, t in [(PULL, (4, 3, 3, 8192)), (-1, (4, 3, 3, 8192)), (FUSED, (4, 3, 3, 2560)), (PUSH, (4, 4, 3, 8192)),
                   (PUSH, (3, 3, 4, 8192)), (PULL, (3, 3, 3, -2)), (PULL, (3, 3, 3, 66)), (6, (3, 3, 3, 0))]:
         assert lib.pp_set_tile(op, 3, *t) != 0 and lib.pp_last_error()
+
+
+@pytest.mark.parametrize("op", [PULL, GRAD, HESS, GDOT, HDOT])
+@pytest.mark.parametrize("deg", [2, 3, 4])
+@pytest.mark.parametrize("d1", [(192, 192, 39), (192, 192, 96), (192, 60, 192), (60, 192, 192), (192, 60, 100)])
+def test_a_slab_goes_where_the_whole_grid_goes(lib, op, deg, d1):
+    """A slab of a sample grid spans a part of the image: along that axis the ratio of the
+    extents says nothing about the spacing of the samples."""
+    d0 = (192, 192, 192)
+    assert route(lib, op, deg, d0)[0] == WS
+    assert route(lib, op, deg, d1, d0=d0, ptrs=(1 << 34, 256, 1 << 33))[0] == WS
+
+
+def test_the_deformation_decides_between_a_block_and_a_coarse_grid(lib):
+    """n^3 samples over (2n)^3 are every other voxel or a block: by their extents alone
+    the same.  Outputs that overlap the deformation leave it to one kernel."""
+    far = (1 << 34, 256, 1 << 33)
+    for op in (PULL, GRAD, HESS, GDOT, HDOT):
+        for deg, n in ((2, 136), (3, 96), (4, 96)):
+            d1, d0 = (n, n, n), (2 * n, 2 * n, 2 * n)
+            assert route(lib, op, deg, d1, d0=d0, ptrs=far)[0] == SAMPLED
+            assert route(lib, op, deg, d1, d0=(n + 20,) * 3, ptrs=far)[0] == WS
+            assert route(lib, op, deg, d1, d0=d0, ptrs=(256, 256, 1 << 33))[0] == WS
