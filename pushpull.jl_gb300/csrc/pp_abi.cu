@@ -221,30 +221,46 @@ static bool coarse_grid(int op, const LaunchArgs& a) {
     return grid_zoom(a) >= (op == kPull && a.g.dp[0] == 3 ? 1.25 : 1.5);
 }
 
-// Sample grids on which the per-voxel kernels beat the warp-specialised ones:
-// small ones, because those take 1920 voxels per CTA at a time, and larger ones
-// where their boxes do not arrive by TMA alone (odd x extents, circulant margins).
-// Device us per-voxel / warp-specialised, one channel, pull, GB300.  Clean: linear
-// 128^3 29 / 33, 192^3 78 / 80 (pull_grad 111 / 95); quadratic 64^3 15 / 15,
-// 92x108x92 25 / 25, 128^3 56 / 42; cubic 48^3 11 / 15, 64^3 17 / 19, 92x108x92
-// 38 / 33; quartic 64^3 23 / 23, 92x108x92 62 / 50.  Odd extents: linear
-// 181x217x181 76 / 133; quadratic 121x145x121 46 / 57, 181x217x181 138 / 151; cubic
-// 91x109x91 40 / 43, 121x145x121 (two channels) 121 / 118; quartic 61x73x61 27 /
-// 32, 91x109x91 66 / 63.  Circulant: quadratic 128^3 54 / 58, cubic 76 / 74.
+// Sample grids on which the per-voxel kernels beat the warp-specialised ones: small
+// ones, because those take 1920 voxels per CTA at a time, and larger ones where their
+// boxes do not arrive by TMA alone (circulant margins, rows that are not multiples of
+// 16 bytes in the image, the deformation or both).  More channels move the line up:
+// each costs the warp-specialised kernels a box of its own.
+// Device us per-voxel / warp-specialised, GB300, pull, pull_grad, pull_hess,
+// pull_grad_dot, pull_hess_dot; one channel:
+//   linear     128^3 27/27 33/31 48/39 37/35 46/41; 160^3 38/47 66/54 80/68 79/78 88/89
+//   quadratic  72^3 14/15 17/16 19/18 18/17 19/19;  80^3 17/15 19/16 23/19 21/17 23/19
+//     circ     104^3 26/33 32/35 37/41 34/37 39/43; 128^3 50/41 60/48 90/58 70/52 85/59
+//     odd      181x217x181 124/143 158/167 194/210 181/200 204/224
+//   cubic      64^3 15/18 15/19 15/19 15/19 16/21;  80^3 25/19 25/21 26/23 25/21 25/24
+//     circ     80^3 25/23 25/25 27/27 25/25 26/29;  112^3 55/44 60/48 65/57 60/51 62/58
+//     odd      97^3 37/42 39/46 43/54 39/48 43/54;  129^3 78/72 82/80 99/101 86/84 95/99
+//   quartic    64^3 23/22 23/23 27/30 25/26 29/29;  80^3 39/28 37/28 45/36 40/31 45/37
+//     circ     64^3 23/28 22/28 27/35 24/30 29/34;  80^3 39/33 37/33 45/43 39/37 46/43
+//     odd      81^3 39/41 39/42 45/57 41/50 47/58;  113^3 94/75 96/82 115/114 101/95 119/116
+// and with two channels, cubic 72^3 29/30 29/32 31/38 29/35 30/40, 88^3 46/39 47/43
+// 52/51 48/47 51/54.
 static bool prefer_per_voxel(int op, const LaunchArgs& a) {
     const Geometry& g = a.g;
     if (g.dp[0] != g.dp[1] || g.dp[1] != g.dp[2] || g.n0 >= (1LL << 31) - 1) return false;
     const long long n = g.n1 * g.nb;
-    const bool odd = (g.d1[0] & 3) || (reinterpret_cast<uintptr_t>(a.phi) & 15);
-    bool rough = odd || (g.d0[0] & 3) || (reinterpret_cast<uintptr_t>(a.in) & 15);
+    const bool phi_odd = (g.d1[0] & 3) || (reinterpret_cast<uintptr_t>(a.phi) & 15);
+    const bool img_odd = (g.d0[0] & 3) || (reinterpret_cast<uintptr_t>(a.in) & 15);
+    bool circ = false;
     for (int c = 0; c < g.nbnd; ++c)
-        rough = rough || !a.bnd.code[c][0] || !a.bnd.code[c][1] || !a.bnd.code[c][2];
-    switch (g.dp[0]) {
-        case 2: return rough || n <= (1LL << 21);
-        case 3: return odd || n <= (rough ? 1LL << 21 : 1LL << 19) || (n < (1LL << 21) && coarse_grid(op, a));
-        case 4: return n <= (rough ? 1LL << 21 : 1LL << 19);
-        default: return n <= (rough ? 1LL << 20 : 1LL << 18);
+        circ = circ || !a.bnd.code[c][0] || !a.bnd.code[c][1] || !a.bnd.code[c][2];
+    const bool dot = op == kPullGradDot || op == kPullHessDot;
+    if (g.dp[0] == 2) {
+        if (phi_odd || img_odd) return true;
+        if (circ) return op == kPull || dot || n <= (1LL << 22);
+        return n <= (op == kPull ? 1LL << 22 : 3LL << 19);
     }
+    if (g.dp[0] == 3 && phi_odd) return true;
+    const int kind = phi_odd ? (img_odd ? 3 : 2) : (img_odd || circ ? 1 : 0);
+    static const int units[3][4] = {{3, 12, 0, 0}, {3, 6, 8, 16}, {2, 3, 4, 8}};   // of 2^17 voxels; degrees 2..4
+    long long most = (long long)units[g.dp[0] - 3][kind] << 17;
+    if (g.nc > 1) most = dot && g.dp[0] < 5 ? 3 * most : 3 * most / 2;
+    return n <= most || (g.dp[0] == 3 && n < (1LL << 21) && coarse_grid(op, a));
 }
 
 namespace {

@@ -96,3 +96,24 @@ def test_the_deformation_decides_between_a_block_and_a_coarse_grid(lib):
             assert route(lib, op, deg, d1, d0=d0, ptrs=far)[0] == SAMPLED
             assert route(lib, op, deg, d1, d0=(n + 20,) * 3, ptrs=far)[0] == WS
             assert route(lib, op, deg, d1, d0=d0, ptrs=(256, 256, 1 << 33))[0] == WS
+
+
+@pytest.mark.parametrize("op,deg,n,kind,nc,family", [
+    (PULL, 2, 64, "clean", 1, PER_VOXEL), (PULL, 2, 80, "clean", 1, WS), (HESS, 3, 80, "clean", 1, WS),
+    (GDOT, 3, 72, "clean", 1, PER_VOXEL), (PULL, 4, 64, "clean", 1, PER_VOXEL), (HDOT, 4, 80, "clean", 1, WS),
+    (PULL, 1, 160, "clean", 1, PER_VOXEL), (HESS, 1, 128, "clean", 1, WS), (GRAD, 1, 96, "clean", 1, PER_VOXEL),
+    (PULL, 2, 128, "circ", 1, WS), (HESS, 3, 128, "circ", 1, WS), (GRAD, 2, 104, "circ", 1, PER_VOXEL),
+    (PULL, 4, 96, "circ", 1, WS), (HDOT, 1, 192, "circ", 1, PER_VOXEL),
+    (PULL, 2, 181, "odd", 1, PER_VOXEL), (PULL, 3, 97, "odd", 1, PER_VOXEL), (GRAD, 3, 161, "odd", 1, WS),
+    (HESS, 4, 97, "odd", 1, PER_VOXEL), (GDOT, 4, 129, "odd", 1, WS), (PULL, 3, 128, "image", 1, WS),
+    (HESS, 3, 80, "image", 1, PER_VOXEL), (PULL, 3, 129, "grid", 1, WS), (GRAD, 3, 97, "grid", 1, PER_VOXEL),
+    (HESS, 3, 80, "clean", 2, PER_VOXEL), (PULL, 3, 104, "clean", 3, WS), (HDOT, 3, 104, "clean", 3, PER_VOXEL),
+    (GDOT, 3, 128, "clean", 3, WS)])
+def test_families_by_size_boundary_and_alignment(lib, op, deg, n, kind, nc, family):
+    """The families as they measured on both sides of the line (the table in pp_abi.cu):
+    clean, circulant margins, rows that are no multiples of 16 bytes in image and grid,
+    in the image only, in the grid only."""
+    d1 = (n, n, n) if kind in ("clean", "circ", "image") else (n, n + 1, n)
+    d0 = {"image": (n + 1, n, n), "grid": (n + 3, n + 1, n)}.get(kind, d1)
+    bnd = (1, 0, 1) if kind == "circ" else (1, 1, 2)
+    assert route(lib, op, deg, d1, d0=d0, bnd=bnd, nc=nc, ptrs=(1 << 34, 256, 1 << 33))[0] == family
