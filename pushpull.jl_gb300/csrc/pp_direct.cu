@@ -167,13 +167,19 @@ void launch_one(const LaunchArgs& a, dim3 grid, cudaStream_t s) {
     if constexpr (PUSH) {
         k_push_direct<DP, OP, IT><<<grid, 256, 0, s>>>(a);
     } else if constexpr (DP > 0 && DP <= 3 && sizeof(IT) == 4) {
-        // four voxels per thread only at one tap per axis, and only when that still
-        // fills the chip (121^3, degree 0: 17 us against 19 with one; 181x217x181:
-        // 38 against 66; 64^3: 11 against 9)
-        if (DP == 1 && a.g.n1 * a.g.nb >= (1LL << 20)) {
-            constexpr int V = DP == 1 ? 4 : 1;
-            const long long blocks = (a.g.n1 + 256 * V - 1) / (256 * V), cap = (long long)sm_count() * 8;
-            k_pull_lean<DP, OP, V><<<dim3((unsigned)(blocks < cap ? blocks : cap), grid.y), 256, 0, s>>>(a);
+        // Small volumes: a warp of 32 voxels along x nearly always holds some at the
+        // border and takes both of k_pull_lean's paths, so that folding every voxel is
+        // faster (64^3, k_pull_lean / here, us: linear pull 8.4 / 6.5, three channels
+        // 12.4 / 10.4, quadratic pull_hess 16.5 / 12.6; from 80^3 on within a tenth, and
+        // a block that stays inside a larger image gains by k_pull_lean: 96^3 out of 192^3
+        // quadratic pull 14.5 / 22.8).  Four voxels per thread only at one tap per axis
+        // and only when that still fills the chip (degree 0, one / four: 121^3 19 / 17,
+        // 181x217x181 66 / 38, 64^3 9 / 11; 64^3 here 6).
+        if (a.g.n1 * a.g.nb < (DP == 1 ? 1LL << 20 : 3LL << 17)) {
+            k_pull_direct<DP, OP, IT><<<grid, 256, 0, s>>>(a);
+        } else if constexpr (DP == 1) {
+            const long long blocks = (a.g.n1 + 1023) / 1024, cap = (long long)sm_count() * 8;
+            k_pull_lean<DP, OP, 4><<<dim3((unsigned)(blocks < cap ? blocks : cap), grid.y), 256, 0, s>>>(a);
         } else {
             k_pull_lean<DP, OP, 1><<<grid, 256, 0, s>>>(a);
         }
