@@ -290,8 +290,12 @@ Route pull_route(int op, const LaunchArgs& a) {
             const bool look = t.automatic && coarse_grid(op, a) && !writes_phi(op, a);
             return {look ? kSampled : kWarpSpecialised, t};
         }
-        // geometries the warp-specialised kernels do not take: the block-synchronous
-        // kernels, or the per-voxel ones at one or two taps per axis
+        // grids thinner than half their tile: per voxel.  Where the caller asked for the
+        // warp-specialised kernels, the block-synchronous ones, or the per-voxel ones at
+        // one or two taps per axis.  (300x6x300, per-voxel / block-synchronous, us: pull
+        // quadratic 18 / 31, cubic 27 / 39, quartic 43 / 47; pull_grad 21 / 31, 29 / 41,
+        // 43 / 49)
+        if (t.automatic) return {kPerVoxel, t};
         t = TileCfg{3, 3, 3, a.g.dp[0] <= 2 ? 0 : 8192};
     }
     return {t.cap > 0 && tiled_supported(a, t) ? kBlockTiled : kPerVoxel, t};

@@ -117,3 +117,15 @@ def test_families_by_size_boundary_and_alignment(lib, op, deg, n, kind, nc, fami
     d0 = {"image": (n + 1, n, n), "grid": (n + 3, n + 1, n)}.get(kind, d1)
     bnd = (1, 0, 1) if kind == "circ" else (1, 1, 2)
     assert route(lib, op, deg, d1, d0=d0, bnd=bnd, nc=nc, ptrs=(1 << 34, 256, 1 << 33))[0] == family
+
+
+@pytest.mark.parametrize("op", [PULL, GRAD, HESS, GDOT, HDOT])
+@pytest.mark.parametrize("deg", [2, 3, 4])
+@pytest.mark.parametrize("d1", [(300, 6, 300), (300, 300, 6), (400, 7, 400), (3, 600, 600)])
+def test_grids_thinner_than_a_tile(lib, op, deg, d1):
+    """Half a tile of the warp-specialised kernels thin: per voxel, and on a tile that was
+    set as it was set."""
+    assert route(lib, op, deg, d1)[0] == PER_VOXEL
+    if d1[0] > 3 and d1[2] > 6:
+        assert lib.pp_set_tile({GDOT: GRAD, HDOT: HESS}.get(op, op), deg, 4, 2, 3, 8192) == 0
+        assert route(lib, op, deg, d1) == (BLOCK, 4, 2, 3, 8192)
