@@ -3,18 +3,19 @@
 // loss = sum_{b,c,v} (pull(f_c, phi)[v] - g_c[v])^2, df = push(2 r), and
 // dphi[v] = sum_c 2 r_c grad pull(f_c)[v]: the forward pull, the pull rrule's
 // two cotangents (src/pushpull_pb.jl:11-18) and the loss of the differentiable
+// step, in one pass over phi, f and g.
 //
 // A CTA takes a tile: the deformation and the target stream in like the push
 // kernels' (pp_push.cuh); the image box is loaded row by row into shared memory
 // and serves the value and the gradient of every voxel; the residuals replace the
 // targets in the tile's ring words and are then scattered through push_channel,
-// one fixed-point word per element, into an accumulator with the box's pitches.
+// two fixed-point words per element, into an accumulator with the box's pitches.
 // Taking the scatter after all residuals of the tile are known lets their actual
 // size set the scale: the pass over the image for max|f| that a scale in advance
-// needs is gone, and so are the second words (the step's df is as accurate as
-// push's).  Six CTAs of 128 threads per SM (four from degree 3 on) cover each
-// other's phases.  160x192x160, bounds (0, 1, 2), GB300, before -> here: quadratic
-// 276 -> 235 us, cubic 471 -> 320, quartic 730 -> 450.
+// needs is gone.  Four CTAs of 128 threads per SM cover each other's phases (the
+// registers of six made the quadratic kernel spill, and three words per element leave
+// room for four).  160x192x160, GB300, with that pass and 256-thread CTAs / here:
+// quadratic 282 / 240 us, cubic 483 / 382; quartic 128^3 409 / 295.
 #pragma once
 
 #include "pp_push.cuh"
@@ -79,18 +80,16 @@ __device__ __forceinline__ float fused_voxel_global(const LaunchArgs& a, int b, 
     return res;
 }
 
-template <int DP>
-constexpr int kFusedCtas = DP <= 3 ? 6 : 4;
+constexpr int kFusedCtas = 4;
 
 template <int DP, typename IT, bool TMA>
-__global__ void __launch_bounds__(kPushThreads, kFusedCtas<DP>) k_fused_tiled(const __grid_constant__ LaunchArgs a,
+__global__ void __launch_bounds__(kPushThreads, kFusedCtas) k_fused_tiled(const __grid_constant__ LaunchArgs a,
                                                                              const __grid_constant__ TileGrid t,
                                                                              const __grid_constant__ CUtensorMap phimap,
                                                                              const __grid_constant__ CUtensorMap gmap) {
     extern __shared__ __align__(128) float4 smem4[];
     constexpr int NW = kPushThreads / 32;
     __shared__ int wrec[NW][8];
-    __shared__ unsigned wmax[NW];
     __shared__ double dred[NW];
     __shared__ __align__(8) unsigned long long bars8[4];
     __shared__ int s_abort;
@@ -106,7 +105,7 @@ __global__ void __launch_bounds__(kPushThreads, kFusedCtas<DP>) k_fused_tiled(co
     float* img = ring + t.stages * slot_floats;      // image box
     float* accf = img + t.cap;                       // adjoint accumulator
     const unsigned bars = smem_addr(bars8);
-    for (int i = threadIdx.x; i < (t.cap >> 2); i += kPushThreads)
+    for (int i = threadIdx.x; i < (t.cap >> 1); i += kPushThreads)
         reinterpret_cast<float4*>(accf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (threadIdx.x == 0) {
         s_abort = 0;
@@ -226,7 +225,7 @@ __global__ void __launch_bounds__(kPushThreads, kFusedCtas<DP>) k_fused_tiled(co
             if (box.mode == 1) {
                 tile_combine(wrec, false, mn, mx, ssum, smax);
                 push_channel<DP, kPush, IT>(g, t, pt, pos, vslot, box, b0, b1, b2,
-                                            a.out + ((long long)o.b * g.nc + c) * g.n0, accf, ssum, smax, wmax);
+                                            a.out + ((long long)o.b * g.nc + c) * g.n0, accf, ssum, smax);
             }
         }
         if (TMA) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // residuals, then the next copy
@@ -249,12 +248,14 @@ __global__ void __launch_bounds__(kPushThreads, kFusedCtas<DP>) k_fused_tiled(co
 
 // Tile grid, shared memory and CTAs of a fused launch.
 TileGrid fused_grid(const LaunchArgs& a, TileCfg c, size_t& smem, int& ctas) {
-    const int dp = a.g.dp[0];
     if (c.automatic) c = fused_own_tile(a);
+    // a budget set by the caller: three words per element and one ring slot in 227 KB
+    const int room = (int)((225 * 1024 - ((size_t)16 << (c.lx + c.ly + c.lz))) / 12) & ~3;
+    if (c.cap > room) c.cap = room;
     TileGrid t = make_grid(a, c);
     t.pmod = (1 << c.lx) & 31;
-    const int most = dp <= 3 ? kFusedCtas<3> : kFusedCtas<4>;
-    const size_t slot = (size_t)4 * t.nv * 4, boxes = (size_t)2 * c.cap * 4;
+    const int most = kFusedCtas;
+    const size_t slot = (size_t)4 * t.nv * 4, boxes = (size_t)3 * c.cap * 4;
     t.stages = 4;
     while (t.stages > 1 && t.stages * slot + boxes > (226 / most - 1) * 1024) --t.stages;
     smem = t.stages * slot + boxes;

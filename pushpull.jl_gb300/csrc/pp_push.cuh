@@ -6,25 +6,17 @@
 // its weighted taps into a shared-memory accumulator that covers the tile's
 // footprint box in the image and flushes the box with 4-wide global reductions.
 //
-// Accumulator: ONE 32-bit fixed-point word per element.  Shared-memory integer
-// reductions run at one wavefront per clock on this part and are what bounds
-// the scatter, so the word count per tap is the first-order cost (cubic push of
-// 192^3: two words 0.406 ms, one 0.226 ms).  A first pass
-// over the tile sums |value| * (its x weights) per (element, first-tap row) with
-// the same reductions (DP per voxel) and takes the maximum h; no element of the
-// box can then receive more than
-//     B = h * (sum of the y weights' maxima) * (sum of the z weights' maxima)
-// in absolute value, so with the quantum q = 2^(E-31), B < 2^E, no sum can leave
-// the word.  Contributions are formed in fixed point as well: the row factor
-// value * wy * wz / q and the x weight as 32-bit integers, their product's upper
-// half (rounded) in one mad.wide, which issues at the rate of the reductions
-// (a float product converted by F2I issues at half of it).  The word is used
-// when B <= kOneWordRatio * mean|value|, which bounds the rounding noise of an
-// element (about 2.3 q for 64 contributions) by 7e-8 of the tile's mean value;
-// it is 1e-8 for image-like values and 3e-8 for noise, below the rounding of the
-// float32 weights.  Other tiles (a few values among zeros, large dynamic range)
-// scatter in two passes: the upper and the lower word of a 42-bit fixed point,
-// each flushed by itself.
+// Accumulator: two 32-bit fixed-point words per element, filled by shared-memory
+// integer reductions, which run at one wavefront per clock on this part and are what
+// bounds the scatter.  A contribution is formed in float32 and split: its upper part
+// in quanta of 2^(E - 22), the rest in quanta of 2^(E - 43).  The scale follows the
+// largest value of the tile and the sum of all, whichever needs more (push_exponent), so
+// that the quantum is at most 2^-41 of the largest value.
+// (One word per element, bounded by a first pass over the tile, takes 226 us at 192^3
+// cubic where two take 323; but 31 bits below the largest sum of a tile leave the
+// elements of its dark parts, of the sample grid's edge and of contracted tiles with
+// errors an order of magnitude above float32's, and push_grad of noise with 1.45e-7
+// against 1.1e-7 in the l2 norm.  It was taken back.)
 //
 // Lanes: a warp covers 2^lx voxels in x and 32 / 2^lx rows.  The row pitch is an odd
 // multiple of 2^lx and the plane pitch a multiple of 32, so that a first tap one
@@ -41,30 +33,13 @@
 namespace pp {
 namespace {
 
-// Four CTAs of 128 threads per SM rather than two of 256: the phases of a tile
-// (bounds, sums, scatter, flush) are separated by barriers, and more CTAs in
-// different phases keep the shared-memory pipe busy (192^3 cubic 0.264 -> 0.227 ms).
+// Four CTAs of 128 threads per SM rather than two of 256: the phases of a tile (bounds,
+// scatter, flush) are separated by barriers, and more CTAs in different phases keep the
+// shared-memory pipe busy (cubic 192^3, best tile of each, us: 335 against 345; three of
+// 128 388, five 334; push_grad 181x217x181 394 against 457, 418, 397).
 constexpr int kPushThreads = 128;
 constexpr int kPushCtas = 4;
-constexpr float kOneWordRatio = 32.0f;
 constexpr int kFarTap = 1 << 22;    // first taps beyond this leave float32 weights inexact: per-voxel path
-
-// Sum over one axis' taps of the largest weight a tap can take (push_grad: of
-// the larger of weight and derivative weight), rounded up.
-template <int DP, int OP>
-__device__ __forceinline__ constexpr float peak_sum() {
-    constexpr float w[5] = {1.f, 2.f, 1.75f, 1.667f, 1.601f};
-    constexpr float d[5] = {1.f, 2.f, 3.f, 2.334f, 2.03f};
-    return OP == kPushGrad ? d[DP - 1] : w[DP - 1];
-}
-
-// Fixed-point formats: an accumulator word holds sums below 2^kWordBits quanta,
-// x weights are scaled by 2^kWeightBits.  At one or two taps a weight can be 1,
-// which needs one bit less of weight and two of sum.
-template <int DP>
-constexpr int kWordBits = DP >= 3 ? 31 : 29;
-template <int DP>
-constexpr int kWeightBits = DP >= 3 ? 31 : 30;
 
 // Voxel `lin` of a tile (x fastest) -> its sample index within the batch.
 // full: the whole tile lies inside the sample grid.
@@ -309,88 +284,17 @@ __device__ __forceinline__ void push_flush(const PushBox& box, const Geometry& g
     else push_flush_rows<false, IT>(box, g, b0, b1, b2, f0, base0, ld4, ld1);
 }
 
-// One voxel into the one-word accumulator.  cv: the values times 2^(bits) / q
-// such that (row factor * x weight) >> 32 is the contribution in quanta.
-template <int DP, int OP, class WT>
-__device__ __forceinline__ void scatter_one(const WT& wx, const WT& wy, const WT& wz, float v0, float v1, float v2,
-                                            unsigned base, unsigned P4, unsigned Q4) {
-    int X[DP], D[OP == kPushGrad ? DP : 1];
-    const float ws = (float)(1ll << kWeightBits<DP>);
-#pragma unroll
-    for (int i = 0; i < DP; ++i) {
-        X[i] = __float2int_rn(wx.w[i] * ws);
-        if constexpr (OP == kPushGrad) D[i] = __float2int_rn(wx.dw[i] * ws);
-    }
-#pragma unroll
-    for (int k = 0; k < DP; ++k) {
-#pragma unroll
-        for (int j = 0; j < DP; ++j) {
-            const unsigned row = base + k * Q4 + j * P4;
-            int y[DP];
-            if constexpr (OP == kPushGrad) {
-                const float wyz = wy.w[j] * wz.w[k];
-                const int A = __float2int_rn(v0 * wyz);
-                const int B = __float2int_rn(v1 * (wy.dw[j] * wz.w[k]) + v2 * (wy.w[j] * wz.dw[k]));
-#pragma unroll
-                for (int i = 0; i < DP; ++i)
-                    y[i] = (int)(((long long)A * D[i] + ((long long)B * X[i] + 0x80000000ll)) >> 32);
-            } else {
-                const int B = __float2int_rn(v0 * (wy.w[j] * wz.w[k]));
-#pragma unroll
-                for (int i = 0; i < DP; ++i) y[i] = (int)(((long long)B * X[i] + 0x80000000ll) >> 32);
-            }
-#pragma unroll
-            for (int i = 0; i < DP; ++i) asm volatile("red.shared.add.s32 [%0], %1;" ::"r"(row + 4u * i), "r"(y[i]));
-        }
-    }
-}
-
-// One voxel, one word (PART 0 upper, 1 lower) of the two-word fixed point, or
-// (PART 2) float.  Values pre-scaled to units of the upper quantum (PART 2: as
-// they are).
-template <int DP, int OP, int PART, class WT>
-__device__ __forceinline__ void scatter_part(const WT& wx, const WT& wy, const WT& wz, float v0, float v1, float v2,
-                                             unsigned base, unsigned P4, unsigned Q4) {
-#pragma unroll 1
-    for (int k = 0; k < DP; ++k) {
-        // runtime z tap without indexing registers
-        float wk = wz.w[0], dk = OP == kPushGrad ? wz.dw[0] : 0.f;
-#pragma unroll
-        for (int i = 1; i < DP; ++i) {
-            if (k == i) {
-                wk = wz.w[i];
-                if constexpr (OP == kPushGrad) dk = wz.dw[i];
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < DP; ++j) {
-            float ca = 0.f, cb;
-            if constexpr (OP == kPushGrad) {
-                ca = v0 * (wy.w[j] * wk);
-                cb = v1 * (wy.dw[j] * wk) + v2 * (wy.w[j] * dk);
-            } else {
-                cb = v0 * (wy.w[j] * wk);
-            }
-            const unsigned row = base + k * Q4 + j * P4;
-#pragma unroll
-            for (int i = 0; i < DP; ++i) {
-                float y;
-                if constexpr (OP == kPushGrad) y = fmaf(ca, wx.dw[i], cb * wx.w[i]);
-                else y = cb * wx.w[i];
-                if constexpr (PART == 2) {
-                    red_f32_nb(row + 4u * i, y);
-                } else {
-                    const float t1 = __fadd_rn(y, kMagic);
-                    if constexpr (PART == 0) {
-                        red_s32_nb(row + 4u * i, __float_as_int(t1) - kMagicBits);
-                    } else {
-                        const float r = __fsub_rn(y, __fsub_rn(t1, kMagic));
-                        red_s32_nb(row + 4u * i, __float_as_int(__fmaf_rn(r, kLoScale, kMagic)) - kMagicBits);
-                    }
-                }
-            }
-        }
-    }
+// Exponent E of the accumulator's scale for a tile whose contributions are at most M
+// each and S in sum (absolute values): the upper quantum is 2^(E - 22), the lower
+// 2^(E - 43).  An upper part is at most 2^22 quanta (E >= log2 M) and an element's
+// sum of them at most 2^30 (E >= log2 S - 8); a lower part is at most 2^20 quanta
+// and an element receives one per voxel, of which a tile has at most 2^10.  INT_MIN:
+// S outside the range the scale factors cover, the tile accumulates in float.
+__device__ __forceinline__ int push_exponent(float S, float M) {
+    const int es = scale_exponent(S);
+    if (es == INT_MIN || es == INT_MAX) return INT_MIN;
+    const int em = scale_exponent(M);      // (INT_MIN below 2^-80)
+    return max(max(em, es - 8), -80);
 }
 
 // Wait until at most n (0..3) of this thread's latest cp.async groups are in flight.
@@ -451,139 +355,65 @@ __device__ __forceinline__ void push_ring_fill(float* base, int slot_floats, int
 template <int DP, int OP, typename IT, class POS>
 __device__ __forceinline__ void push_channel(const Geometry& g, const TileGrid& t, const PushTile& pt, const POS& pos,
                                              const float* vslot, const PushBox& box, int b0, int b1, int b2, float* f0,
-                                             float* accf, float ssum, float smax, unsigned* wmax) {
+                                             float* accf, float ssum, float smax) {
     constexpr int ORD = OP == kPushGrad ? 1 : 0;
     constexpr int NCOMP = OP == kPushGrad ? 3 : 1;
-    constexpr int NW = kPushThreads / 32;
     if (smax == 0.f) return;   // every value of this channel is zero or skipped
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nv = t.nv;
+    const int nv = t.nv, half = box.size;
     int* acc = reinterpret_cast<int*>(accf);
     const int bxo = box.lo[0], by0 = box.lo[1], bz0 = box.lo[2];
     const unsigned P4 = 4u * box.P, Q4 = 4u * box.Q;
     const int base0 = box_base(box, g, f0);
     const unsigned cbase = smem_addr(accf) + 4u * base0;
-    auto values = [&](int lin, float (&val)[3]) -> bool {
-        bool fin = true;
-        val[1] = val[2] = 0.f;
-#pragma unroll
-        for (int p = 0; p < NCOMP; ++p) {
-            val[p] = vslot[p * nv + lin];
-            fin = fin & finitef(val[p]);
-        }
-        return fin;
-    };
-    // every valid voxel of this thread with finite values: fn(values, weights, element address)
-    auto each = [&](auto fn) {
+    const int E = push_exponent(NCOMP == 3 ? 2.f * ssum : ssum, NCOMP == 3 ? 2.f * smax : smax);
+    auto scatter = [&](float sc, auto fixed) {
 #pragma unroll 1
         for (int lin = threadIdx.x; lin < nv; lin += kPushThreads) {
-            float x0, x1, x2, val[3];
-            if (!pt.inside(lin) || !pos(g, pt, lin, x0, x1, x2) || !values(lin, val)) continue;
+            float x0, x1, x2, val[3] = {0.f, 0.f, 0.f};
+            if (!pt.inside(lin) || !pos(g, pt, lin, x0, x1, x2)) continue;
+            bool fin = true;
+#pragma unroll
+            for (int p = 0; p < NCOMP; ++p) {
+                val[p] = vslot[p * nv + lin];
+                fin = fin & finitef(val[p]);
+            }
+            if (!fin) continue;
             W3<DP, ORD> wx, wy, wz;
             const int ox = spline_taps32<DP, ORD>(x0, wx.w, wx.dw, wx.hw) - bxo;
             const int oy = spline_taps32<DP, ORD>(x1, wy.w, wy.dw, wy.hw) - by0;
             const int oz = spline_taps32<DP, ORD>(x2, wz.w, wz.dw, wz.hw) - bz0;
-            fn(val, wx, wy, wz, cbase + 4u * (unsigned)(oz * box.Q + oy * box.P + ox));
+            push_scatter<DP, OP, decltype(fixed)::value>(wx, wy, wz, val[0] * sc, val[1] * sc, val[2] * sc,
+                                                         cbase + 4u * (unsigned)(oz * box.Q + oy * box.P + ox), P4, Q4,
+                                                         4u * half);
         }
+        __syncthreads();
     };
-    const float S = NCOMP == 3 ? 2.f * ssum : ssum;   // bound on the sum of |contributions|
-    int E = scale_exponent(S);
-    bool one = false;
     if (E != INT_MIN) {
-        // ---- bound on any element's sum --------------------------
-        int em;
-        frexpf(smax, &em);                               // smax < 2^em
-        const float hs = pow2f(20 - em);                 // |value| * weight -> at most 2^20 units
-        // branch free like the first pass: skipped voxels add 0 to the box's first words
-#pragma unroll 2
-        for (int lin = threadIdx.x; lin < nv; lin += kPushThreads) {
-            float x0, x1, x2, val[3];
-            const bool ok = pos(g, pt, lin, x0, x1, x2) & values(lin, val) & pt.inside(lin);
-            W3<DP, ORD> wx;
-            const int ox = spline_taps32<DP, ORD>(x0, wx.w, wx.dw, wx.hw) - bxo;
-            const int oy = first_tap32(x1, DP) - by0, oz = first_tap32(x2, DP) - bz0;
-            const unsigned p = ok ? cbase + 4u * (unsigned)(oz * box.Q + oy * box.P + ox) : cbase;
-            const float s0 = fabsf(val[0]) * hs, s12 = (fabsf(val[1]) + fabsf(val[2])) * hs;
-#pragma unroll
-            for (int i = 0; i < DP; ++i) {
-                float h;
-                if constexpr (OP == kPushGrad) h = fmaf(s0, fabsf(wx.dw[i]), s12 * wx.w[i]);
-                else h = s0 * wx.w[i];
-                red_s32_nb(p + 4u * i, ok ? (int)__float2uint_ru(h) : 0);
-            }
-        }
-        __syncthreads();
-        unsigned hm = 0;
-        for (int i = threadIdx.x; i < (box.size >> 2); i += kPushThreads) {
-            uint4 v = reinterpret_cast<uint4*>(accf)[i];
-            reinterpret_cast<uint4*>(accf)[i] = make_uint4(0u, 0u, 0u, 0u);
-            hm = max(max(hm, max(v.x, v.y)), max(v.z, v.w));
-        }
-        hm = __reduce_max_sync(0xffffffffu, hm);
-        if (lane == 0) wmax[warp] = hm;
-        __syncthreads();
-        hm = __reduce_max_sync(0xffffffffu, wmax[lane & (NW - 1)]);
-        constexpr float pk = peak_sum<DP, OP>();
-        const float B = __uint2float_ru(hm) * (pk * pk) * pow2f(em - 20);
-        // mean |value| per voxel, and voxels per element where the tile is denser than the grid
-        const float cnt = (float)pt.count(t);
-        const float rho = 2.f * cnt / ((float)(box.e[0] - DP + 1) * (float)(box.e[1] - DP + 1) *
-                                       (float)(box.e[2] - DP + 1));
-        if (B * cnt <= kOneWordRatio * ssum * sqrtf(fmaxf(rho, 1.f))) {
-            const int EB = scale_exponent(B);
-            if (EB != INT_MIN && EB != INT_MAX) {
-                one = true;
-                E = EB;
-            }
-        }
-    }
-    auto ld1f = [&](int w) {
-        const float v = accf[w];
-        accf[w] = 0.f;
-        return v;
-    };
-    auto ld4f = [&](int w) {
-        const float4 v = *reinterpret_cast<const float4*>(accf + w);
-        *reinterpret_cast<float4*>(accf + w) = make_float4(0.f, 0.f, 0.f, 0.f);
-        return v;
-    };
-    auto flush_words = [&](float q) {
+        scatter(pow2f(22 - E), std::true_type{});
+        const float q1 = pow2f(E - 22), q2 = pow2f(E - 43);
+        auto val = [&](int h, int l) { return fmaf((float)h, q1, (float)l * q2); };
         push_flush<IT>(box, g, b0, b1, b2, f0, base0, [&](int w) {
-            const int4 h = *reinterpret_cast<const int4*>(acc + w);
-            *reinterpret_cast<int4*>(acc + w) = make_int4(0, 0, 0, 0);
-            return make_float4(__int2float_rn(h.x) * q, __int2float_rn(h.y) * q, __int2float_rn(h.z) * q,
-                               __int2float_rn(h.w) * q);
+            int4* hp = reinterpret_cast<int4*>(acc + w);
+            int4* lp = reinterpret_cast<int4*>(acc + half + w);
+            const int4 h = *hp, l = *lp;
+            *hp = *lp = make_int4(0, 0, 0, 0);
+            return make_float4(val(h.x, l.x), val(h.y, l.y), val(h.z, l.z), val(h.w, l.w));
         }, [&](int w) {
-            const int h = acc[w];
-            acc[w] = 0;
-            return __int2float_rn(h) * q;
+            const int h = acc[w], l = acc[half + w];
+            acc[w] = acc[half + w] = 0;
+            return val(h, l);
         });
-    };
-    if (one) {
-        const float sc = pow2f(32 - kWeightBits<DP> + kWordBits<DP> - E);
-        each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
-            scatter_one<DP, OP>(wx, wy, wz, val[0] * sc, val[1] * sc, val[2] * sc, p, P4, Q4);
-        });
-        __syncthreads();
-        flush_words(pow2f(E - kWordBits<DP>));
-    } else if (E != INT_MIN) {
-        const float sc = pow2f(22 - E);
-        each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
-            scatter_part<DP, OP, 0>(wx, wy, wz, val[0] * sc, val[1] * sc, val[2] * sc, p, P4, Q4);
-        });
-        __syncthreads();
-        flush_words(pow2f(E - 22));
-        __syncthreads();
-        each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
-            scatter_part<DP, OP, 1>(wx, wy, wz, val[0] * sc, val[1] * sc, val[2] * sc, p, P4, Q4);
-        });
-        __syncthreads();
-        flush_words(pow2f(E - 22) * (1.f / kLoScale));
     } else {
-        each([&](float (&val)[3], auto& wx, auto& wy, auto& wz, unsigned p) {
-            scatter_part<DP, OP, 2>(wx, wy, wz, val[0], val[1], val[2], p, P4, Q4);
+        scatter(1.f, std::false_type{});
+        push_flush<IT>(box, g, b0, b1, b2, f0, base0, [&](int w) {
+            const float4 v = *reinterpret_cast<const float4*>(accf + w);
+            *reinterpret_cast<float4*>(accf + w) = make_float4(0.f, 0.f, 0.f, 0.f);
+            return v;
+        }, [&](int w) {
+            const float v = accf[w];
+            accf[w] = 0.f;
+            return v;
         });
-        __syncthreads();
-        push_flush<IT>(box, g, b0, b1, b2, f0, base0, ld4f, ld1f);
     }
 }
 
@@ -592,67 +422,66 @@ __device__ __forceinline__ void push_channel(const Geometry& g, const TileGrid& 
 // A tile with several samples per first-tap cell (a contracting deformation) is
 // scattered cell by cell.  The voxels of a batch are counting-sorted by cell;
 // then a warp takes a cell, one tap (or two) per lane, sums the cell's voxels in
-// registers for up to three channels at once and adds each tap's sum to the
-// two-word accumulator once.  A voxel costs the warp its position within the
+// registers for up to three channels at once, a few voxels at a time, and adds each
+// tap's sums to the two-word accumulator.  A voxel costs the warp its position within the
 // cell and its values (16-byte broadcast loads of two voxels) and packed f32x2
 // arithmetic: the lane's weights are polynomials in that position whose
-// coefficients the lane holds.  256^3 x 3 channels, 0.25x contraction, GB300:
-// 3.90 ms with one voxel per warp instruction and channel, 1.43 ms cell by cell.
-// Under six samples per cell the per-thread scatter is the faster one (192^3,
-// 0.5x, one channel: 0.51 ms cell by cell, 0.28 ms per thread; 0.35x: 0.42 and
-// 0.50 ms).
+// coefficients the lane holds.
+// A cell's sums are float32: 32 voxels (two halves of 16) between fixed-point additions
+// keep their rounding near that of the terms themselves (cubic, contracted 0.25x, l2
+// error against 64 bits of push of noise / push_grad of noise, 1e-7: halves of 8 1.29 /
+// 1.35, of 16 1.36 / 1.42, of any length 1.45 / 1.52; every voxel into fixed point by
+// itself 1.67 / 1.47; us, 192^3: 489, 471, 462, 618).
+// From three samples per cell on (cubic push; push_grad four, quadratic six) this is the
+// faster scatter.  192^3, one channel, us, cell by cell / per voxel: 0.35x 441 / 614,
+// 0.5x 480 / 560, 0.6x 544 / 454; quadratic 0.4x 367 / 332; push_grad 160^3 0.4x 349 / 417,
+// 0.5x 402 / 340.
 constexpr int kCellBatch = 512;       // voxels sorted at a time
-constexpr int kCellMin = 6;           // samples per cell from which a tile counts as contracted
+constexpr int kCellRun = 16;          // pairs of voxels a lane sums before they go into fixed point
+template <int DP, int OP>             // samples per cell from which a tile counts as contracted
+constexpr int kCellMin = DP == 3 ? 6 : (OP == kPush ? 3 : 4);
 constexpr int kCellChannels = 3;      // channels summed at once (push)
-
-// Power-basis coefficients of weight `i` of degree DP - 1 (and of its derivative)
-// in the position s of spline_weights; constants chosen so the weights sum to one.
-template <int DP>
-__device__ __forceinline__ void weight_poly(int i, float (&w)[4], float (&d)[3]) {
-    if constexpr (DP == 3) {          // (1/2 - s)^2 / 2, 3/4 - s^2, (1/2 + s)^2 / 2
-        w[0] = i == 1 ? 0.75f : 0.125f;
-        w[1] = i == 0 ? -0.5f : (i == 1 ? 0.f : 0.5f);
-        w[2] = i == 1 ? -1.f : 0.5f;
-        w[3] = 0.f;
-    } else {                          // (1 - s)^3 / 6, 2/3 - s^2 + s^3 / 2, ..., s^3 / 6
-        constexpr float c6 = 1.0f / 6.0f, c23 = 2.0f / 3.0f;
-        w[0] = i == 0 ? c6 : (i == 1 ? c23 : (i == 2 ? (1.0f - c23) - c6 : 0.f));
-        w[1] = i == 0 ? -0.5f : (i == 2 ? 0.5f : 0.f);
-        w[2] = i == 1 ? -1.f : (i == 3 ? 0.f : 0.5f);
-        w[3] = i == 0 ? -c6 : (i == 1 ? 0.5f : (i == 2 ? -0.5f : c6));
-    }
-    d[0] = w[1];
-    d[1] = 2.f * w[2];
-    d[2] = 3.f * w[3];
-}
 
 __device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
 
-// A weight (and derivative) polynomial, for two voxels at once.
+// One lane's weight (and derivative) along an axis, for two voxels at once, in the
+// factored form of spline_weights (a power basis in s cancels where a weight is
+// small).  u is the position from the end of the spline's piece that makes the piece
+// one of two shapes: degree 3 u^3 / 6 and c - u^2 + u^3 / 2 with u = s or 1 - s,
+// degree 2 u^2 / 2 with u = 1/2 + s or 1/2 - s and 3/4 - s^2.
 template <int DP, int ORD>
 struct LanePoly {
-    float2 w[DP], d[ORD >= 1 ? DP - 1 : 1];
+    float2 sg, off, k3, k2, c, cl, m2, m1;
     __device__ __forceinline__ void set(int i) {
-        float c[4], e[3];
-        weight_poly<DP>(i, c, e);
-#pragma unroll
-        for (int k = 0; k < DP; ++k) w[k] = dup(c[k]);
-        if constexpr (ORD >= 1) {
-#pragma unroll
-            for (int k = 0; k + 1 < DP; ++k) d[k] = dup(e[k]);
+        if constexpr (DP == 4) {
+            const bool mirror = i == 0 || i == 2, outer = i == 0 || i == 3;
+            const float s1 = mirror ? -1.f : 1.f;
+            constexpr float c6 = 1.0f / 6.0f, c23 = 2.0f / 3.0f;
+            sg = dup(s1);
+            off = dup(mirror ? 1.f : 0.f);
+            k3 = dup(outer ? c6 : 0.5f);
+            k2 = dup(outer ? 0.f : -1.f);
+            // 2/3 in two words: rounded to one it is off by 2e-8, in one direction for every sample
+            c = dup(outer ? 0.f : c23);
+            cl = dup(outer ? 0.f : (float)(2.0 / 3.0 - (double)c23));
+            m2 = dup(s1 * (outer ? 0.5f : 1.5f));
+            m1 = dup(outer ? 0.f : -2.f * s1);
+        } else {
+            sg = dup(i == 0 ? -1.f : 1.f);
+            off = dup(i == 1 ? 0.f : 0.5f);
+            k2 = dup(i == 1 ? -1.f : 0.5f);
+            c = dup(i == 1 ? 0.75f : 0.f);
+            m1 = dup(i == 0 ? -1.f : (i == 1 ? -2.f : 1.f));
         }
     }
-    __device__ __forceinline__ float2 val(float2 s) const {
-        float2 r = w[DP - 1];
-#pragma unroll
-        for (int k = DP - 2; k >= 0; --k) r = __ffma2_rn(r, s, w[k]);
-        return r;
+    __device__ __forceinline__ float2 at(float2 s) const { return __ffma2_rn(s, sg, off); }
+    __device__ __forceinline__ float2 val(float2 u) const {
+        if constexpr (DP == 4) return __fadd2_rn(c, __ffma2_rn(__fmul2_rn(u, u), __ffma2_rn(u, k3, k2), cl));
+        else return __ffma2_rn(__fmul2_rn(u, k2), u, c);
     }
-    __device__ __forceinline__ float2 der(float2 s) const {
-        float2 r = d[DP - 2];
-#pragma unroll
-        for (int k = DP - 3; k >= 0; --k) r = __ffma2_rn(r, s, d[k]);
-        return r;
+    __device__ __forceinline__ float2 der(float2 u) const {
+        if constexpr (DP == 4) return __fmul2_rn(u, __ffma2_rn(u, m2, m1));
+        else return __fmul2_rn(u, m1);
     }
 };
 
@@ -690,61 +519,64 @@ __device__ __forceinline__ void cell_scatter(const CellArrays& ca, int ncells, i
     const int off = ti + P * tj + Q * tk;
     const bool live = DP == 4 || lane < DP * DP * DP;
     for (int cell = warp; cell < ncells; cell += kPushThreads / 32) {
-        const int b = ca.start[cell], e = ca.start[cell + 1];
-        if (b == e) continue;
-        float2 acc2[PASSES][NOUT];
-#pragma unroll
-        for (int p = 0; p < PASSES; ++p)
-#pragma unroll
-            for (int c = 0; c < NOUT; ++c) acc2[p][c] = make_float2(0.f, 0.f);
-#pragma unroll 2
-        for (int t = b >> 1; t < e >> 1; ++t) {
-            const float4 a4 = ca.A[t], b4 = ca.B[t];
-            const float2 sx = make_float2(a4.x, a4.y), sy = make_float2(a4.z, a4.w), sz = make_float2(b4.x, b4.y);
-            float2 v[3];
-            v[0] = make_float2(b4.z, b4.w);
-            if constexpr (NVAL > 1) {
-                const float4 c4 = ca.C[t];
-                v[1] = make_float2(c4.x, c4.y);
-                v[2] = make_float2(c4.z, c4.w);
-            }
-            const float2 wx = px.val(sx), wy = py.val(sy);
-            if constexpr (OP == kPushGrad) {
-                // v0 dwx wy wz + v1 wx dwy wz + v2 wx wy dwz
-                const float2 f = __ffma2_rn(wy, __fmul2_rn(v[0], px.der(sx)),
-                                            __fmul2_rn(py.der(sy), __fmul2_rn(v[1], wx)));
-                const float2 h = __fmul2_rn(wy, __fmul2_rn(v[2], wx));
-#pragma unroll
-                for (int p = 0; p < PASSES; ++p) {
-                    acc2[p][0] = __ffma2_rn(pz[p].val(sz), f, acc2[p][0]);
-                    acc2[p][0] = __ffma2_rn(pz[p].der(sz), h, acc2[p][0]);
-                }
-            } else {
-                const float2 wxy = __fmul2_rn(wx, wy);
-#pragma unroll
-                for (int p = 0; p < PASSES; ++p) {
-                    const float2 w = __fmul2_rn(wxy, pz[p].val(sz));
-#pragma unroll
-                    for (int c = 0; c < NOUT; ++c) acc2[p][c] = __ffma2_rn(w, v[c], acc2[p][c]);
-                }
-            }
-        }
+        const int b = ca.start[cell] >> 1, e = ca.start[cell + 1] >> 1;
         // cell -> box element of its first tap
         const int cz = cell / c01, cr = cell - cz * c01, cy = cr / c0, cx = cr - cy * c0;
         const unsigned base = acc + 4u * (unsigned)(cx + P * cy + Q * cz + off);
-        if (live) {
+        for (int t0 = b; t0 < e; t0 += kCellRun) {
+            const int t1 = min(t0 + kCellRun, e);
+            float2 acc2[PASSES][NOUT];
 #pragma unroll
             for (int p = 0; p < PASSES; ++p)
 #pragma unroll
-                for (int c = 0; c < NOUT; ++c) {
-                    // y in units of the upper quantum, |y| <= 2^22: hi = round(y), lo = round((y - hi) * 2^20)
-                    const float y = (acc2[p][c].x + acc2[p][c].y) * inv[c];
-                    const float t1 = __fadd_rn(y, kMagic);
-                    const float r = __fsub_rn(y, __fsub_rn(t1, kMagic));
-                    const unsigned ad = base + 4u * (unsigned)(2 * p * Q + c * 2 * half + base0[c]);
-                    red_s32_nb(ad, __float_as_int(t1) - kMagicBits);
-                    red_s32_nb(ad + 4u * half, __float_as_int(__fmaf_rn(r, kLoScale, kMagic)) - kMagicBits);
+                for (int c = 0; c < NOUT; ++c) acc2[p][c] = make_float2(0.f, 0.f);
+#pragma unroll 2
+            for (int t = t0; t < t1; ++t) {
+                const float4 a4 = ca.A[t], b4 = ca.B[t];
+                const float2 ux = px.at(make_float2(a4.x, a4.y)), uy = py.at(make_float2(a4.z, a4.w));
+                const float2 sz = make_float2(b4.x, b4.y);
+                float2 v[3];
+                v[0] = make_float2(b4.z, b4.w);
+                if constexpr (NVAL > 1) {
+                    const float4 c4 = ca.C[t];
+                    v[1] = make_float2(c4.x, c4.y);
+                    v[2] = make_float2(c4.z, c4.w);
                 }
+                const float2 wx = px.val(ux), wy = py.val(uy);
+                if constexpr (OP == kPushGrad) {
+                    // v0 dwx wy wz + v1 wx dwy wz + v2 wx wy dwz
+                    const float2 f = __ffma2_rn(wy, __fmul2_rn(v[0], px.der(ux)),
+                                                __fmul2_rn(py.der(uy), __fmul2_rn(v[1], wx)));
+                    const float2 h = __fmul2_rn(wy, __fmul2_rn(v[2], wx));
+#pragma unroll
+                    for (int p = 0; p < PASSES; ++p) {
+                        const float2 uz = pz[p].at(sz);
+                        acc2[p][0] = __fadd2_rn(acc2[p][0], __ffma2_rn(pz[p].val(uz), f, __fmul2_rn(pz[p].der(uz), h)));
+                    }
+                } else {
+                    const float2 wxy = __fmul2_rn(wx, wy);
+#pragma unroll
+                    for (int p = 0; p < PASSES; ++p) {
+                        const float2 w = __fmul2_rn(wxy, pz[p].val(pz[p].at(sz)));
+#pragma unroll
+                        for (int c = 0; c < NOUT; ++c) acc2[p][c] = __ffma2_rn(w, v[c], acc2[p][c]);
+                    }
+                }
+            }
+            if (live) {
+#pragma unroll
+                for (int p = 0; p < PASSES; ++p)
+#pragma unroll
+                    for (int c = 0; c < NOUT; ++c) {
+                        // y in units of the upper quantum, |y| <= 2^22: hi = round(y), lo = round((y - hi) * 2^21)
+                        const float y = (acc2[p][c].x + acc2[p][c].y) * inv[c];
+                        const float t1f = __fadd_rn(y, kMagic);
+                        const float r = __fsub_rn(y, __fsub_rn(t1f, kMagic));
+                        const unsigned ad = base + 4u * (unsigned)(2 * p * Q + c * 2 * half + base0[c]);
+                        red_s32_nb(ad, __float_as_int(t1f) - kMagicBits);
+                        red_s32_nb(ad + 4u * half, __float_as_int(__fmaf_rn(r, kLoScale, kMagic)) - kMagicBits);
+                    }
+            }
         }
     }
 }
@@ -764,7 +596,6 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
     constexpr int NW = kPushThreads / 32;
     constexpr bool CELLS = DP == 3 || DP == 4;   // degrees whose taps fill one or two warp instructions
     __shared__ int wrec[NW][8];
-    __shared__ unsigned wmax[NW];
     __shared__ int wscan[NW];
     __shared__ __align__(8) unsigned long long bars8[4];
     __shared__ int s_abort;
@@ -851,7 +682,7 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
                 // contracted: the two-word accumulators of a channel group, the
                 // sorted voxels, their tags and the cell starts fit the budget
                 const long long nce = (long long)(box.e[0] - DP + 1) * (box.e[1] - DP + 1) * (box.e[2] - DP + 1);
-                if (nce * kCellMin <= pt.count(t) && nce < 1024) {
+                if (nce * kCellMin<DP, OP> <= pt.count(t) && nce < 1024) {
                     long long P = box.e[0] + 3;
                     P += (4 - P) & 7;                 // odd multiples of 4, and planes 16 banks apart:
                     long long Q = P * box.e[1];       // a cell's taps fall in distinct banks
@@ -872,7 +703,7 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
                     }
                 }
             }
-            if (!box.cells) box_pitches(t, t.cap, g, box);
+            if (!box.cells) box_pitches(t, (t.cap >> 1) & ~3, g, box);
         }
         if (box.mode == 2) {
             for (int lin = threadIdx.x; lin < nv; lin += kPushThreads) {
@@ -1042,7 +873,7 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
                         int b0, b1, b2;
                         bnd_code(a, cg + q, b0, b1, b2);
                         FixedScale fs;
-                        fs.set(Es[q], 42);
+                        fs.set(Es[q], 43);
                         int* hi = acc + 2 * q * half;
                         push_flush<IT>(box, g, b0, b1, b2, a.out + ((long long)o.b * g.nc + cg + q) * g.n0, base0[q],
                                        [&](int w) {
@@ -1107,7 +938,7 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
                     combine(false);
                 }
                 push_channel<DP, OP, IT>(g, t, pt, pos, vslot, box, b0, b1, b2,
-                                         a.out + ((long long)o.b * g.nc + c) * g.n0, accf, ssum, smax, wmax);
+                                         a.out + ((long long)o.b * g.nc + c) * g.n0, accf, ssum, smax);
             }
         }
         if (TMA && g.nc > 1) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1118,8 +949,8 @@ __global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push_tiled(const __
     if constexpr (!TMA) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
-// Tile grid of a push launch: ring depth for the shared memory
-// that two resident CTAs per SM leave (or one, for budgets too large for two).
+// Tile grid of a push launch: ring depth for the shared memory that kPushCtas resident
+// CTAs per SM leave; one slot, and fewer CTAs, for budgets too large for that.
 TileGrid push_grid(const LaunchArgs& a, const TileCfg& c, int comps, size_t& smem) {
     TileGrid t = make_grid(a, c);
     t.nv = 1 << (c.lx + c.ly + c.lz);

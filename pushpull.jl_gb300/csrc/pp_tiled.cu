@@ -44,21 +44,25 @@ bool grid_supported(const LaunchArgs& a, const TileCfg& t, int max_vox) {
 }  // namespace
 
 bool tiled_supported(const LaunchArgs& a, const TileCfg& t) { return grid_supported(a, t, 2 * kThreads); }
-bool push_supported(const LaunchArgs& a, const TileCfg& t) { return grid_supported(a, t, 8 * kThreads); }
+bool push_supported(const LaunchArgs& a, const TileCfg& t) { return grid_supported(a, t, 4 * kThreads); }
 
-// The default push tiles are the largest of 16x8x8, 16x8x4 and 8x8x4 voxels that
-// still give every SM a few tiles: with fewer than about three 16x8x8 tiles (two
-// 16x8x4 tiles) per SM the smaller ones win because more CTAs take part.  Cubic
-// push, GB300, device us with 16x8x8 / 16x8x4 / 8x8x4 tiles: 32^3 22 / 18 / 15,
-// 48^3 22 / 20 / 18, 64^3 27 / 22 / 25, 80^3 31 / 33 / 35, 128^3 80 / 92 / 107;
-// at 192^3 16x8x8 takes 226, 8x8x8 255, 16x8x4 263, 32x4x8 244, 32x8x4 242.
+// Push tiles: 8x8x8 voxels where they give every SM a few, else 8x8x4, so that more CTAs
+// take part; budgets (accumulator words, two per element) that leave room for four CTAs
+// per SM with one ring slot (push_grad at degrees 2 and 3: the ring holds three values).
+// GB300, us, 8x8x8 / 8x8x4: cubic 32^3 20 / 18, 48^3 22 / 19, 64^3 29 / 28, 72^3 33 / 31,
+// 80^3 37 / 37; quartic 64^3 43 / 35; quadratic 64^3 18 / 20; push_grad cubic 56^3 25 / 23,
+// 72^3 33 / 32.  192^3 cubic, with the best budget of each: 8x8x8 335, 16x8x4 349, 8x16x4
+// 352, 16x8x8 378.  Budgets: quadratic 192^3 9472 words 202, 11008 209; quartic 160^3
+// 9472 397, 11008 344; cubic contracted 256^3 x 3 9472 1997, 11008 1751; push_grad
+// 181x217x181 cubic 8448 394, 9472 427, quartic 128^3 8448 182, 9472 167.
+// Grids under 8 voxels in x fill half a tile: at degree 2 the per-voxel kernels
+// (6x300x300 32 / 49 us).
 TileCfg push_default_tile(int op, const LaunchArgs& a) {
-    const int cap = op == kPush ? 9984 : 7936;   // words: four CTAs per SM with one ring slot
-    const long long y = (a.g.d1[1] + 7) >> 3, b = a.g.nb;
-    const long long x16 = (a.g.d1[0] + 15) >> 4;
-    if (x16 * y * ((a.g.d1[2] + 7) >> 3) * b >= 3LL * sm_count()) return TileCfg{4, 3, 3, cap};
-    if (x16 * y * ((a.g.d1[2] + 3) >> 2) * b >= 2LL * sm_count()) return TileCfg{4, 3, 2, cap};
-    return TileCfg{3, 3, 2, cap};
+    const int dp = a.g.dp[0];
+    if (dp == 3 && a.g.d1[0] < 8) return TileCfg{3, 3, 3, 0};
+    const int cap = op == kPush ? (dp <= 3 ? 9472 : 11008) : (dp <= 4 ? 8448 : 9472);
+    const long long tiles = ((a.g.d1[0] + 7) >> 3) * ((a.g.d1[1] + 7) >> 3) * ((a.g.d1[2] + 7) >> 3) * a.g.nb;
+    return TileCfg{3, 3, tiles >= (dp <= 3 ? 3LL : 5LL) * sm_count() ? 3 : 2, cap};
 }
 
 cudaError_t launch_pull_tiled(int op, const LaunchArgs& a, const TileCfg& t, cudaStream_t s) {

@@ -4,10 +4,14 @@
 
 namespace pp {
 
-// The tile and budget (floats of the image box, words of the accumulator) measured
-// best: 160x192x160 quadratic, us: 16x8x4 229, 8x8x8 241, 16x4x8 237, 8x16x4 250,
-// 32x4x4 248; with five CTAs per SM and a larger budget 237, with four 231.
-TileCfg fused_own_tile(const LaunchArgs& a) { return TileCfg{4, 3, 2, a.g.dp[0] <= 3 ? 3072 : 4864}; }
+// The tile and budget (floats of the image box; the accumulator has two words for each)
+// measured best.  160x192x160, us, with the best budget of each shape: quadratic 16x8x4
+// 240, 8x8x8 241, 16x4x8 244; cubic 382, 385, 390; quartic 128^3 8x8x8 295, 8x16x4 321,
+// 16x8x4 326.
+TileCfg fused_own_tile(const LaunchArgs& a) {
+    const int dp = a.g.dp[0];
+    return dp == 5 ? TileCfg{3, 3, 3, 4864} : TileCfg{4, 3, 2, dp <= 3 ? 3328 : 3840};
+}
 
 int fused_tiled_grid(const LaunchArgs& a, const TileCfg& c) {
     size_t smem;

@@ -440,7 +440,7 @@ __device__ __forceinline__ void sign_rows(const RowBox& box, const Geometry& g, 
 // is out of range (S = 0, non-finite, or extreme) the tile uses float atomics.
 constexpr float kMagic = 12582912.0f;     // 1.5 * 2^23: float -> nearest int for |y| <= 2^22
 constexpr int kMagicBits = 0x4B400000;
-constexpr float kLoScale = 1048576.0f;    // push tiles of up to 2048 voxels: 2^20 lower quanta per upper one
+constexpr float kLoScale = 2097152.0f;    // 2^21 lower quanta per upper one (tiles of up to 1024 voxels)
 
 __device__ __forceinline__ float pow2f(int k) { return __int_as_float((127 + k) << 23); }   // -126 <= k <= 127
 
@@ -1022,7 +1022,7 @@ __device__ __forceinline__ void push_scatter(const WT& wx, const WT& wy, const W
                     const float2 t1 = __fadd2_rn(y2, make_float2(kMagic, kMagic));
                     const float2 u = __fadd2_rn(t1, make_float2(-kMagic, -kMagic));
                     const float2 r = __ffma2_rn(u, make_float2(-1.f, -1.f), y2);
-                    const float2 l2 = __ffma2_rn(r, make_float2(2097152.0f, 2097152.0f), make_float2(kMagic, kMagic));
+                    const float2 l2 = __ffma2_rn(r, make_float2(kLoScale, kLoScale), make_float2(kMagic, kMagic));
                     h[i] = __float_as_int(t1.x) - kMagicBits;
                     h[i + 1] = __float_as_int(t1.y) - kMagicBits;
                     l[i] = __float_as_int(l2.x) - kMagicBits;
@@ -1037,7 +1037,7 @@ __device__ __forceinline__ void push_scatter(const WT& wx, const WT& wy, const W
                     const float t1 = __fadd_rn(y, kMagic);
                     const float r = __fsub_rn(y, __fsub_rn(t1, kMagic));
                     h[i] = __float_as_int(t1) - kMagicBits;
-                    l[i] = __float_as_int(__fmaf_rn(r, 2097152.0f, kMagic)) - kMagicBits;
+                    l[i] = __float_as_int(__fmaf_rn(r, kLoScale, kMagic)) - kMagicBits;
                 }
                 red_row_s32<DP>(row, h);
                 red_row_s32<DP>(row + lo_off, l);
