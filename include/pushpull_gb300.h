@@ -28,6 +28,15 @@
  * (nbnd == 1: one triple for every channel, nbnd == nc: one per channel);
  * ext 0/1 (src/pushpull_general.jl:15-60).
  *
+ * Device memory: native calls take stream-ordered scratch from a memory pool that
+ * this library owns per device, outside the caller's allocator: the fused step one
+ * double per thread block, and pull-family calls on an image whose rows are not
+ * multiples of 16 bytes a copy of it with padded rows (up to 256 MiB; larger
+ * images, calls under stream capture and calls that find no memory do without,
+ * with the same results).  The pool keeps up to 64 MiB between calls, returns the
+ * rest at the next synchronisation, and returns what is free on
+ * pp_release_scratch.
+ *
  * Thread safety: native calls keep no state besides the thread-local error
  * string and are safe from any thread on any stream.  Compatibility calls use
  * a per-thread device workspace and stream.
@@ -142,9 +151,8 @@ int pp_push_count(float *f0, float *c0, const float *phi, const float *f1,
  * pull_grad) and two broadcasts.  g has the layout of a pull output, (d1, nc, nb).
  * Invalid voxels make the loss NaN and their dphi NaN; non-finite residuals are
  * not pushed.  accumulate applies to df only.  The loss is reduced in a fixed
- * order and is reproducible from run to run.  Uses stream-ordered scratch (one
- * double per CTA, one float per image volume) from a memory pool this library
- * owns per device. */
+ * order and is reproducible from run to run.  Uses stream-ordered scratch, one
+ * double per thread block. */
 int pp_fused_step(double *loss, float *df, float *dphi, const float *f0, const float *phi, const float *g,
                   const pp_usize d0[3], const pp_usize d1[3], int nc, int nb,
                   const int *bnd, int nbnd, const int deg[3], int ext, int accumulate, void *stream);
@@ -281,6 +289,11 @@ int pp_autotune(int op, float *out, const float *phi, const float *in, const pp_
                 int *best, float *best_ms);
 /* Kernel family choice for all later calls in the process (PP_PATH_*). */
 int pp_set_path(int path);
+
+/* Give the unused scratch memory of the current device back to the system (see
+ * "Device memory" above; scratch of calls still running stays until it is freed).
+ * Safe at any time; later calls take scratch again. */
+int pp_release_scratch(void);
 
 /* Message of the last failing call on this thread ("" when none). */
 const char *pp_last_error(void);

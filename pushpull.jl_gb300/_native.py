@@ -68,6 +68,7 @@ _SIGS = {
     "pp_autotune": (C.c_int, [C.c_int, _vp, _vp, _vp, _u64x3, _u64x3, C.c_int, C.c_int, _vp, C.c_int, _i32x3,
                               C.c_int, C.c_int, _vp, C.POINTER(C.c_int), C.POINTER(C.c_float)]),
     "pp_last_error": (C.c_char_p, []),
+    "pp_release_scratch": (C.c_int, []),
     "pp_get_route": (C.c_int, [C.c_int, _vp, _vp, _vp, _u64x3, _u64x3, C.c_int, C.c_int, _vp, C.c_int, _i32x3, C.c_int,
                                C.c_int * 5]),
     "pp_set_tile": (C.c_int, [C.c_int] * 6),

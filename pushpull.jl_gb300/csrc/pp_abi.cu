@@ -58,15 +58,16 @@ void set_error_message(const char* msg) { g_err = msg ? msg : ""; }
 // device, that keeps its memory (up to kScratchKeep) between calls: the device's
 // default pool returns memory to the system at every synchronisation, which would
 // re-map it per call.
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pools[64] = {};
+
 static cudaError_t scratch_pool(cudaMemPool_t* out) {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lk(mu);
-    if (!pools[dev]) {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (!g_pools[dev]) {
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -75,9 +76,9 @@ static cudaError_t scratch_pool(cudaMemPool_t* out) {
         if ((e = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return e;
         unsigned long long keep = kScratchKeep;
         if ((e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) return e;
-        pools[dev] = p;
+        g_pools[dev] = p;
     }
-    *out = pools[dev];
+    *out = g_pools[dev];
     return cudaSuccess;
 }
 
@@ -475,6 +476,17 @@ int pp_fused_step(double* loss, float* df, float* dphi, const float* f0, const f
                   const pp_usize d0[3], const pp_usize d1[3], int nc, int nb, const int* bnd, int nbnd,
                   const int deg[3], int ext, int accumulate, void* stream) {
     return run_fused(loss, df, dphi, f0, phi, g, d0, d1, nc, nb, bnd, nbnd, deg, ext, accumulate, stream);
+}
+
+int pp_release_scratch(void) {
+    pp::g_err.clear();
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return pp::cuda_fail(e, "cudaGetDevice");
+    std::lock_guard<std::mutex> lk(pp::g_pool_mu);
+    if (dev < 0 || dev >= 64 || !pp::g_pools[dev]) return PP_OK;   // nothing was ever taken
+    e = cudaMemPoolTrimTo(pp::g_pools[dev], 0);
+    return e == cudaSuccess ? PP_OK : pp::cuda_fail(e, "release scratch");
 }
 
 const char* pp_last_error(void) { return pp::g_err.c_str(); }

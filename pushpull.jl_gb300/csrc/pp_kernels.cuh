@@ -67,10 +67,14 @@ cudaError_t launch_push_direct(int op, const LaunchArgs& a, cudaStream_t s);
 dim3 fused_direct_grid(const LaunchArgs& a);
 cudaError_t launch_fused_direct(const LaunchArgs& a, cudaStream_t s);
 cudaError_t launch_sum_partials(const double* partial, int n, double* out, cudaStream_t s);
-// Stream-ordered scratch from a pool owned by this library (one per device),
-// which keeps up to kScratchKeep bytes between calls and gives back the rest;
-// freed with cudaFreeAsync.
-constexpr size_t kScratchKeep = 512u << 20;
+// Stream-ordered scratch from a pool owned by this library (one per device), freed
+// with cudaFreeAsync.  The pool keeps up to kScratchKeep bytes between calls, gives the
+// rest back when the stream is next synchronised, and all that is free when the
+// caller asks (pp_release_scratch).  Nothing larger than kScratchMost is asked for.
+// (A cubic pull of an odd volume copied through the pool, waited for after each call, us:
+// 181x217x181, 27 MiB, kept 192, remapped in every call 353, without the copy 273;
+// 257^3 x 2, 130 MiB, kept 697, remapped 976, without the copy 1114.)
+constexpr size_t kScratchKeep = 64u << 20, kScratchMost = 256u << 20;
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
 
 // number of SMs of the current device (cached per device)

@@ -750,8 +750,7 @@ __global__ void __launch_bounds__(256) k_pad_rows(const float* __restrict__ in, 
 // 8 bytes per image voxel and channel (28 MB of image: about 10 us) and saves the
 // consumers loading every box themselves (181x217x181 cubic pull, GB300: 186 us
 // with it, 279 us without).  It is not made for images much larger than the
-// sample grid, above the scratch the library keeps, or while the stream is being
-// captured into a graph.
+// sample grid, above kScratchMost, or while the stream is being captured into a graph.
 struct WsImage {
     float* copy = nullptr;
     bool tma = false;
@@ -764,7 +763,7 @@ inline cudaError_t ws_image(const LaunchArgs& a, const TileGrid& t, CUtensorMap*
     if (im.tma) return cudaSuccess;
     const long long pitch = (g.d0[0] + 3) & ~3LL, rows = g.d0[1] * g.d0[2] * planes;
     const long long bytes = pitch * rows * 4;
-    if (g.n0 > 4 * g.n1 || bytes > (long long)kScratchKeep / 2 || rows > 0x7fffffffLL) return cudaSuccess;
+    if (g.n0 > 4 * g.n1 || bytes > (long long)kScratchMost || rows > 0x7fffffffLL) return cudaSuccess;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
         (void)cudaGetLastError();
