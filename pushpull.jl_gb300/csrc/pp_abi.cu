@@ -579,7 +579,7 @@ int pp_autotune(int op, float* out, const float* phi, const float* in, const pp_
     const int tiles[][3] = {{3, 3, 3}, {4, 3, 2}, {4, 2, 3}, {5, 2, 2}, {3, 4, 2},
                             {3, 3, 2}, {4, 2, 2}, {4, 3, 3}, {3, 3, 4}};
     const int caps_pull[] = {6144, 8192, 12288};
-    const int caps_push[] = {7936, 9984, 16384};
+    const int caps_push[] = {8448, 11008, 16384};
     const TileCfg saved = tile_for(op, deg[0]);
     const int saved_path = current_path();
     cudaEvent_t e0, e1;

@@ -108,11 +108,8 @@ int pp_batch_create(pp_batch** plan, const pp_batch_item* items, int n, int zero
         const bool iso = deg[0] == deg[1] && deg[1] == deg[2];
         const pp::TileCfg tc = batch_tile_for(it.d1, deg[0]);
         bi.t = pp::tile_grid(bi.pull, tc);
-        // the push registry entry of the degree sets the box budget (two words per
-        // element there, three here), within the kernel's fixed budget
-        const pp::TileCfg pc = pp::tile_for(PP_OP_PUSH, deg[0]);
-        const long long want = pc.cap > 0 ? (3LL * pc.cap / 2) & ~3LL : p->cap;
-        bi.t.cap = (int)(want < 64 ? 64 : (want > p->cap ? p->cap : want));
+        // the launch has the whole budget whatever an item uses of it
+        bi.t.cap = p->cap;
         // anisotropic degrees: the per-voxel path of the batched kernel (dp 0)
         bi.dp = iso ? deg[0] + 1 : 0;
         total += (long long)bi.t.ntiles;
