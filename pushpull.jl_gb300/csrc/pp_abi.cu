@@ -309,7 +309,7 @@ Route push_route(int op, const LaunchArgs& a) {
 
 Route fused_route(const LaunchArgs& a) {
     const TileCfg t = tile_for(PP_OP_FUSED, a.g.dp[0] - 1);
-    if (current_path() == PP_PATH_DIRECT || !tiled_supported(a, t)) return {kPerVoxel, t};
+    if (current_path() == PP_PATH_DIRECT || !fused_supported(a, t)) return {kPerVoxel, t};
     return {kBlockTiled, t.automatic ? fused_own_tile(a) : t};
 }
 }  // namespace

@@ -112,7 +112,7 @@ extern "C" int pp_fused_step_noalloc(double* loss, float* df, float* dphi, const
             return fail_status(PP_ERR_ALIGN, "float pointers must be 4-byte aligned");
         a.up = g;
         a.out2 = dphi;
-        tiled = current_path() != PP_PATH_DIRECT && tiled_supported(a, t);
+        tiled = current_path() != PP_PATH_DIRECT && fused_supported(a, t);
         if (tiled) {
             grid = fused_tiled_grid(a, t);
             slots = grid;

@@ -46,6 +46,14 @@ bool grid_supported(const LaunchArgs& a, const TileCfg& t, int max_vox) {
 bool tiled_supported(const LaunchArgs& a, const TileCfg& t) { return grid_supported(a, t, 2 * kThreads); }
 bool push_supported(const LaunchArgs& a, const TileCfg& t) { return grid_supported(a, t, 4 * kThreads); }
 
+// The own tile is 16 voxels wide.  On narrow grids the per-voxel kernels are faster
+// (us, per-voxel / tiled: 6x300x300 quadratic 45 / 106, cubic 82 / 152, quartic 154 / 190;
+// 12x300x300 73 / 105, 149 / 152, 279 / 225).
+bool fused_supported(const LaunchArgs& a, const TileCfg& t) {
+    const long long x = a.g.d1[0];
+    return tiled_supported(a, t) && !(t.automatic && (x <= 8 || (x < 16 && a.g.dp[0] == 3)));
+}
+
 // Push tiles: 8x8x8 voxels where they give every SM a few, else 8x8x4, so that more CTAs
 // take part; budgets (accumulator words, two per element) that leave room for four CTAs
 // per SM with one ring slot (push_grad at degrees 2 and 3: the ring holds three values).

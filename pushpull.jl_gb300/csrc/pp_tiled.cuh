@@ -5,7 +5,7 @@
 
 namespace pp {
 
-// Tile of sample voxels handled by one CTA: 2^lx x 2^ly x 2^lz (32..512 voxels, push up to 2048),
+// Tile of sample voxels handled by one CTA: 2^lx x 2^ly x 2^lz (32..512 voxels, push up to 1024),
 // and the shared-memory budget of its footprint box, in floats (multiple of 4).
 struct TileCfg {
     int lx, ly, lz;
@@ -15,8 +15,10 @@ struct TileCfg {
 };
 
 bool tiled_supported(const LaunchArgs& a, const TileCfg& t);
-// the same for the push family, whose tiles hold up to 2048 voxels
+// the same for the push family, whose tiles hold up to 1024 voxels
 bool push_supported(const LaunchArgs& a, const TileCfg& t);
+// and for the fused step, whose own tile leaves out narrow grids
+bool fused_supported(const LaunchArgs& a, const TileCfg& t);
 // the push tile for a launch whose registry entry is the library's own
 TileCfg push_default_tile(int op, const LaunchArgs& a);
 // warp-specialised pull family (8 x 16 x 15 tiles, pp_ws.cuh): geometry test and

@@ -129,3 +129,15 @@ def test_grids_thinner_than_a_tile(lib, op, deg, d1):
     if d1[0] > 3 and d1[2] > 6:
         assert lib.pp_set_tile({GDOT: GRAD, HDOT: HESS}.get(op, op), deg, 4, 2, 3, 8192) == 0
         assert route(lib, op, deg, d1) == (BLOCK, 4, 2, 3, 8192)
+
+
+@pytest.mark.parametrize("d1,deg,family", [((6, 300, 300), 2, PER_VOXEL), ((8, 256, 256), 3, PER_VOXEL),
+                                           ((4, 256, 256), 4, PER_VOXEL), ((12, 300, 300), 2, PER_VOXEL),
+                                           ((12, 300, 300), 3, BLOCK), ((20, 20, 400), 3, BLOCK),
+                                           ((300, 6, 300), 3, BLOCK), ((300, 300, 6), 4, BLOCK)])
+def test_fused_step_on_narrow_grids(lib, d1, deg, family):
+    """Tiles 16 voxels wide on a grid of less than half that: per voxel, unless a tile was set."""
+    assert route(lib, FUSED, deg, d1)[0] == family
+    if d1[0] > 3:
+        assert lib.pp_set_tile(FUSED, deg, 3, 3, 3, 2560) == 0
+        assert route(lib, FUSED, deg, d1)[0] == (BLOCK if min(d1) >= 4 else PER_VOXEL)
