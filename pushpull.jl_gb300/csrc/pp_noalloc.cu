@@ -112,14 +112,13 @@ extern "C" int pp_fused_step_noalloc(double* loss, float* df, float* dphi, const
             return fail_status(PP_ERR_ALIGN, "float pointers must be 4-byte aligned");
         a.up = g;
         a.out2 = dphi;
-        tiled = current_path() != PP_PATH_DIRECT && fused_supported(a, t);
-        if (tiled) {
-            grid = fused_tiled_grid(a, t);
-            slots = grid;
-        } else {
-            const dim3 gd = fused_direct_grid(a);
-            slots = (long long)gd.x * gd.y;
-        }
+        // the per-voxel kernels need a partial per block and volume, the tiled ones a few
+        // per SM: those where the others' do not fit
+        const bool may = current_path() != PP_PATH_DIRECT;
+        const dim3 gd = fused_direct_grid(a);
+        slots = (long long)gd.x * gd.y;
+        tiled = may && (fused_supported(a, t) || (slots > PP_NOALLOC_MAX_PARTIALS && tiled_supported(a, t)));
+        if (tiled) slots = grid = fused_tiled_grid(a, t);
         const long long planes = (long long)a.g.nc * a.g.nb;
         if (slots > PP_NOALLOC_MAX_PARTIALS)
             return fail_status(PP_ERR_TOO_LARGE,
