@@ -78,7 +78,7 @@ def _oracle_threads():
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of each kernel on this
 # workload, from one ncu capture each (profiles/k_pull_ws_192cubic.md, k_push_tiled_192cubic.md,
 # k_pull_ws_affine_192cubic.md, k_push_tiled_affine_192cubic.md)
-TRAFFIC = {"pull": 125_219_072, "push": 153_690_624, "affine_pull": 28_572_160, "affine_push": 56_656_128}
+TRAFFIC = {"pull": 125_219_072, "push": 154_402_560, "affine_pull": 28_572_160, "affine_push": 56_674_560}
 
 
 class Clocks:

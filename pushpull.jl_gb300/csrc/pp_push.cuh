@@ -13,7 +13,7 @@
 // largest value of the tile and the sum of all, whichever needs more (push_exponent), so
 // that the quantum is at most 2^-41 of the largest value.
 // (One word per element, bounded by a first pass over the tile, takes 226 us at 192^3
-// cubic where two take 323; but 31 bits below the largest sum of a tile leave the
+// cubic where two take 331; but 31 bits below the largest sum of a tile leave the
 // elements of its dark parts, of the sample grid's edge and of contracted tiles with
 // errors an order of magnitude above float32's, and push_grad of noise with 1.45e-7
 // against 1.1e-7 in the l2 norm.  It was taken back.)
